@@ -189,6 +189,58 @@ __host__ __device__ __forceinline__ void decode3(int64_t id, int ny, int nz, int
   x = (int)r;
 }
 
+// -------------------------------------------------------------------------------
+// Layout of the arrays the MIC(0) sweeps stream (sc_sweep.cuh).
+//
+// The grid is cut into tiles of 16 (x) by 8 (y) columns spanning z, and a tile
+// into 2 x 2 warp tiles of 8 (x) by 4 (y) columns.  Lane (ty * 8 + tx) of the warp
+// that owns a warp tile walks its column at step sigma = z + tx + ty, so the x and
+// y neighbours of the values a step computes were computed by the adjacent lanes
+// one step before.  A warp tile stores, step after step, what its 32 lanes touch:
+// four steps form a chunk of 128 consecutive elements, in which every lane's
+// values are 16-byte vectors (float: 4 steps; double: 2 x 2 steps), so that a
+// warp's accesses are whole 512-byte lines.  nc chunks hold the nz + 10 steps; the
+// entries of steps at which a lane has no cell (and of columns outside the grid)
+// are padding and hold zeros.  Several arrays can be interleaved chunk by chunk
+// (a stream of `arrays` arrays).
+struct SweepLayout {
+  static constexpr int TX = 16, TY = 8, kWarps = 4;
+  int nx, ny, nz;
+  int ntx, nty;        // tiles
+  int nc;              // chunks of a warp tile
+  int64_t total;       // elements of one array
+
+  static SweepLayout make(int nx, int ny, int nz) {
+    SweepLayout g;
+    g.nx = nx;
+    g.ny = ny;
+    g.nz = nz;
+    g.ntx = (nx + TX - 1) / TX;
+    g.nty = (ny + TY - 1) / TY;
+    g.nc = (nz + 10 + 3) / 4;
+    g.total = (int64_t)g.ntx * g.nty * kWarps * g.nc * 128;
+    return g;
+  }
+  __host__ __device__ __forceinline__ int ntiles() const { return ntx * nty; }
+  // first chunk of a warp tile
+  __host__ __device__ __forceinline__ int64_t chunk0(int X, int Y, int warp) const {
+    return (int64_t)((Y * ntx + X) * kWarps + warp) * nc;
+  }
+  // element of lane `lane` at step sigma, within a warp tile of one array
+  template <class T>
+  __host__ __device__ __forceinline__ static int within(int sigma, int lane) {
+    constexpr int VE = 16 / (int)sizeof(T);
+    return (sigma / VE * 32 + lane) * VE + sigma % VE;
+  }
+  // element of a cell in array `a` of a stream of `arrays` arrays
+  template <class T>
+  __host__ __device__ __forceinline__ int64_t off(int x, int y, int z, int arrays = 1, int a = 0) const {
+    const int tx = x & 7, ty = y & 3, sigma = z + tx + ty;
+    const int64_t c = chunk0(x >> 4, y >> 3, ((y >> 2) & 1) * 2 + ((x >> 3) & 1)) + (sigma >> 2);
+    return (c * arrays + a) * 128 + within<T>(sigma & 3, ty * 8 + tx);
+  }
+};
+
 // Reference-layout index helpers.
 __host__ __device__ __forceinline__ int64_t lin(int i, int j, int k, int sy, int sz) {
   return (int64_t)k + (int64_t)j * sz + (int64_t)i * sy * sz;

@@ -11,11 +11,16 @@
 // memory, so a chunk of iterations is captured once as a CUDA graph):
 //   k_spmv   Az = A s, partial s.Az          -> alpha      (project-solver.cc:328-331)
 //   k_axpy   p += alpha s, r -= alpha Az     -> residual   (:332-335)
-//   k_wave   forward sweep  q = K^-1 r                     (:276-288)
-//   k_wave   backward sweep z = K^-T q, z.r -> beta        (:293-305, :338-341)
+//   k_sweep  forward sweep  q = K^-1 r                     (:276-288)
+//   k_sweep  backward sweep z = K^-T q, z.r -> beta        (:293-305, :338-341)
 //   k_sa     s = z + beta s                  -> iter++     (:342, util.cc:404-410)
 // The MIC(0) pivots E = 1/sqrt(e) are computed once per solve by a wavefront
 // kernel; the reference recomputes them on every call with identical values.
+//
+// Two layouts.  The system as its producers write it (matrix, right-hand side,
+// active flags, the pressure handed back, and the mixed solve's FP64 residual) is
+// in the Tiled layout; everything an iteration touches is in the SweepLayout, in
+// which the sweeps (sc_sweep.cuh) stream whole chunks.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -27,46 +32,16 @@
 #include <mutex>
 #include <string>
 
-#include <cooperative_groups.h>
-
-#include "sc_pcg.cuh"
+#include "sc_sweep.cuh"
 
 namespace sc {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kRing = 32;     // boundary ring entries per wavefront CTA
-// Nanoseconds a waiting warp of a sweep (the control warp, the mailbox
-// loaders) sleeps between two polls that found nothing (0: back to back).
-// 16 took ~1.5% off the 128^3 mixed solve (A/B of two builds, two runs each:
-// 40.4 -> 39.8 ms); the spinning warps were taking issue slots from the row
-// warps of the same SM.
-#ifndef SC_WAVE_CTL_NS
-#define SC_WAVE_CTL_NS 16
-#endif
 // 1: the iterations sweep only the tiles holding an active cell; 0: every tile
 #ifndef SC_SKIP_EMPTY_TILES
 #define SC_SKIP_EMPTY_TILES 1
 #endif
-#ifndef SC_WAVE_STAGE_MAX
-#define SC_WAVE_STAGE_MAX 8
-#endif
-// Bytes per cp.async chunk of the staged sweep input (4, 8 or 16); 8 measured
-// best for both precisions at 128^3 and 512^3 (16 costs FP64 sweeps ~4%).
-#ifndef SC_WAVE_CHUNK64
-#define SC_WAVE_CHUNK64 8
-#endif
-#ifndef SC_WAVE_CHUNK32
-#define SC_WAVE_CHUNK32 8
-#endif
-// Ring slots of staged sweep input (steps in flight per compute warp): as many
-// as fit in ~180 KB of shared memory, at most SC_WAVE_STAGE_MAX.
-template <class T, int NV>
-constexpr int wave_stages() {
-  constexpr int fit = (int)(180 * 1024 / ((size_t)Tiled::TY * NV * 32 * sizeof(T)));
-  return fit < SC_WAVE_STAGE_MAX ? fit : SC_WAVE_STAGE_MAX;
-}
-constexpr int kSpinLimit = 1 << 22;  // default bound of the waits: ~0.1-1 s, far above any legitimate wait
 
 enum { FIN_NONE = 0, FIN_INIT, FIN_SPMV, FIN_AXPY, FIN_BWD, FIN_SA, FIN_NORMS, FIN_EINIT, FIN_EAXPY, FIN_EREPLACE };
 
@@ -272,12 +247,6 @@ __global__ void __launch_bounds__(kThreads) k_from_tiled(Tiled g, const Ts* __re
     if (c.inside) dst[lin(c.x, c.y, c.z, g.ny, g.nz)] = (Td)src[c.e];
   }
 }
-template <class Ts, class Td>
-__global__ void k_convert(int64_t n, const Ts* __restrict__ src, Td* __restrict__ dst) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride)
-    dst[e] = (Td)src[e];
-}
 template <class T>
 __global__ void k_fill(int64_t n, T* __restrict__ dst, T v) {
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -305,250 +274,289 @@ __global__ void k_symmetry(int nx, int ny, int nz, const double* const* an,
 }
 
 // ---------------------------------------------------------------------------------
-// Elementwise PCG kernels (tiled layout).
+// Elementwise kernels over a SweepLayout.  A thread owns the four consecutive
+// elements at 4 * i (a 16- or 32-byte vector).
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_init(Tiled g, const double* __restrict__ src,
+struct __align__(16) Vec4 {
+  T e[4];
+};
+template <class T>
+__device__ __forceinline__ Vec4<T> vload(const T* p) {
+  return *reinterpret_cast<const Vec4<T>*>(p);
+}
+template <class T>
+__device__ __forceinline__ void vstore(T* p, const Vec4<T>& v) {
+  *reinterpret_cast<Vec4<T>*>(p) = v;
+}
+
+// Position of a lane's chunk in the grid: (x, y) of its column and z of its step
+// 4 * chunk; `inside`: the column lies in the grid.  A chunk's four steps are four
+// consecutive z, those outside [0, nz) padding.
+struct ChunkPos {
+  int tile, lane, x, y, z0;
+  bool inside;
+  int64_t chunk;  // over the grid
+  int64_t e;      // element of the first step in one array (chunk_load, chunk_store)
+  // and in array `a` of a stream of `arrays`
+  template <class T>
+  __device__ __forceinline__ int64_t in_stream(int arrays, int a) const {
+    return (chunk * arrays + a) * 128 + lane * (16 / (int)sizeof(T));
+  }
+};
+template <class T>
+__device__ __forceinline__ ChunkPos chunk_pos(const SweepLayout& g, int64_t i) {  // i: chunk * 32 + lane over the grid
+  const int lane = (int)(i & 31);
+  const unsigned c = (unsigned)(i >> 5), w = c / (unsigned)g.nc, ch = c - w * (unsigned)g.nc;
+  const int tile = (int)(w >> 2), ww = (int)(w & 3);
+  const int Y = tile / g.ntx, X = tile - Y * g.ntx, tx = lane & 7, ty = lane >> 3;
+  ChunkPos p;
+  p.tile = tile;
+  p.chunk = c;
+  p.lane = lane;
+  p.x = X * 16 + (ww & 1) * 8 + tx;
+  p.y = Y * 8 + (ww >> 1) * 4 + ty;
+  p.z0 = (int)ch * 4 - tx - ty;
+  p.inside = p.x < g.nx && p.y < g.ny;
+  p.e = (int64_t)c * 128 + lane * (16 / (int)sizeof(T));
+  return p;
+}
+#define SC_CHUNK_LOOP(i, g) \
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (g).total / 4; i += (int64_t)gridDim.x * blockDim.x)
+
+// r = scale * src on active cells (src in the Tiled layout, r in the SweepLayout), p = 0.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_init(Tiled tg, SweepLayout g, const double* __restrict__ src,
                                                    double scale, const uint8_t* __restrict__ act,
                                                    T* __restrict__ r, T* __restrict__ p,
                                                    double* partials, PcgScalars* sc,
                                                    int fin = FIN_INIT) {
   double s2 = 0.0, mx = 0.0;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < g.total; e += stride) {
-    T v = act[e] ? (T)(src[e] * scale) : T(0);
-    r[e] = v;
-    p[e] = T(0);
-    double dv = (double)v;
-    s2 += dv * dv;
-    mx = fmax(mx, fabs(dv));
+  SC_CHUNK_LOOP(i, g) {
+    const ChunkPos c = chunk_pos<T>(g, i);
+    T v[4], zero[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int z = c.z0 + j;
+      v[j] = T(0);
+      if (c.inside && z >= 0 && z < g.nz) {
+        const int64_t o = tg.off(c.x, c.y, z);
+        if (act[o]) v[j] = (T)(src[o] * scale);
+      }
+      const double dv = (double)v[j];
+      s2 += dv * dv;
+      mx = fmax(mx, fabs(dv));
+    }
+    chunk_store(r + c.e, v);
+    chunk_store(p + c.e, zero);
   }
   reduce_finalize(s2, mx, partials, sc, fin);
+}
+// Norms of src on active cells, and (out given) its masked copy; Tiled layout.
+__global__ void __launch_bounds__(kThreads) k_norms(int64_t n, const double* __restrict__ src,
+                                                    const uint8_t* __restrict__ act, double* __restrict__ out,
+                                                    double* partials, PcgScalars* sc) {
+  double s2 = 0.0, mx = 0.0;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    const double v = act[e] ? src[e] : 0.0;
+    if (out) out[e] = v;
+    s2 += v * v;
+    mx = fmax(mx, fabs(v));
+  }
+  reduce_finalize(s2, mx, partials, sc, FIN_NORMS);
+}
+// SweepLayout -> Tiled (the pressure handed back) and Tiled -> SweepLayout.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_sweep_to_tiled(SweepLayout g, Tiled tg, const T* __restrict__ src,
+                                                             double* __restrict__ dst) {
+  SC_ROWBLOCK_LOOP(tg) {
+    Cell c;
+    c.init(tg, rb, threadIdx.x);
+    dst[c.e] = c.inside ? (double)src[g.off<T>(c.x, c.y, c.z)] : 0.0;
+  }
+}
+// Reference layout <-> SweepLayout.
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_ref_to_sweep(SweepLayout g, const double* __restrict__ src, T* __restrict__ dst) {
+  SC_CHUNK_LOOP(i, g) {
+    const ChunkPos c = chunk_pos<T>(g, i);
+    T v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int z = c.z0 + j;
+      v[j] = c.inside && z >= 0 && z < g.nz ? (T)src[lin(c.x, c.y, z, g.ny, g.nz)] : T(0);
+    }
+    chunk_store(dst + c.e, v);
+  }
+}
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_sweep_to_ref(SweepLayout g, const T* __restrict__ src, double* __restrict__ dst) {
+  SC_CHUNK_LOOP(i, g) {
+    const ChunkPos c = chunk_pos<T>(g, i);
+    const Quad<T> v = chunk_load(src + c.e);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int z = c.z0 + j;
+      if (c.inside && z >= 0 && z < g.nz) dst[lin(c.x, c.y, z, g.ny, g.nz)] = (double)v.e[j];
+    }
+  }
 }
 
 // The iteration kernels below visit only the tiles of a sweep order list
 // (tiles[-1].x entries; the tiles holding an active cell): the vectors they
-// update are zero on every other tile and stay so.  Work unit: one slot of a
-// tile, its TY x 32 = 256 consecutive elements, one per thread of the block.
-static_assert(Tiled::TY * 32 == kThreads, "a tile slot is one element per thread");
-__device__ __forceinline__ int slot_count(const Tiled& g, const int2* __restrict__ tiles) {
-  return tiles[-1].x * g.nz;
+// update are zero on every other tile and stay so.  Work unit: nc-th part of a
+// tile, 512 consecutive elements, four per thread of half a block.
+__device__ __forceinline__ int unit_count(const SweepLayout& g, const int2* __restrict__ tiles) {
+  return tiles[-1].x * g.nc;
 }
-__device__ __forceinline__ int64_t slot_elem(const Tiled& g, const int2* __restrict__ tiles, int c) {
-  const int t = c / g.nz, sl = c - t * g.nz;
+constexpr int kUnits = kThreads / 128;  // units a block visits at once
+__device__ __forceinline__ int first_unit() { return blockIdx.x * kUnits + (threadIdx.x >> 7); }
+__device__ __forceinline__ int64_t unit_elem(const SweepLayout& g, const int2* __restrict__ tiles, int c) {
+  const int t = c / g.nc, u = c - t * g.nc;
   const int2 XY = tiles[t];
-  return ((int64_t)(XY.y * g.ntx + (XY.x & 0xffff)) * g.nz + sl) * kThreads + threadIdx.x;
+  return ((int64_t)(XY.y * g.ntx + XY.x) * g.nc + u) * 512 + 4 * (threadIdx.x & 127);
 }
 
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_copy(Tiled g, const int2* __restrict__ tiles, const T* __restrict__ a,
+__global__ void __launch_bounds__(kThreads) k_copy(SweepLayout g, const int2* __restrict__ tiles, const T* __restrict__ a,
                                                    T* __restrict__ b, const PcgScalars* sc) {
   if (sc->done != DONE_RUNNING) return;
-  const int nch = slot_count(g, tiles);
-  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
-    const int64_t e = slot_elem(g, tiles, c);
-    b[e] = a[e];
+  const int nch = unit_count(g, tiles);
+  for (int c = first_unit(); c < nch; c += kUnits * gridDim.x) {
+    const int64_t e = unit_elem(g, tiles, c);
+    vstore(b + e, vload(a + e));
   }
 }
 
 // applyCompressedMatrix (project-solver.cc:16-39) on the tiled layout.  The
 // upper couplings come from the neighbours' lower ones (A symmetric,
 // checkSystemSymmetry, :41-57).
-template <class T, class X>
-__device__ __forceinline__ T apply_row(const Tiled& g, const Cell& c, const T* __restrict__ adiag,
-                                       const T* __restrict__ al, const T* __restrict__ ad,
-                                       const T* __restrict__ ab, const uint8_t* __restrict__ act,
-                                       const X* __restrict__ x) {
+// x(dx, dy, dz) is the vector's value at the cell's neighbour.
+template <class X>
+__device__ __forceinline__ double apply_row(const Tiled& g, const Cell& c, const double* __restrict__ adiag,
+                                            const double* __restrict__ al, const double* __restrict__ ad,
+                                            const double* __restrict__ ab, const uint8_t* __restrict__ act, X x) {
   const int64_t e = c.e;
-  T t = adiag[e] * (T)x[e];
+  double t = adiag[e] * x(0, 0, 0);
   if (c.x > 0) {
     int64_t o = c.xm(g);
-    if (act[o]) t += al[e] * (T)x[o];
+    if (act[o]) t += al[e] * x(-1, 0, 0);
   }
   if (c.y > 0) {
     int64_t o = c.ym(g);
-    if (act[o]) t += ad[e] * (T)x[o];
+    if (act[o]) t += ad[e] * x(0, -1, 0);
   }
   if (c.z > 0) {
     int64_t o = c.zm(g);
-    if (act[o]) t += ab[e] * (T)x[o];
+    if (act[o]) t += ab[e] * x(0, 0, -1);
   }
   if (c.x < g.nx - 1) {
     int64_t o = c.xp(g);
-    if (act[o]) t += al[o] * (T)x[o];
+    if (act[o]) t += al[o] * x(1, 0, 0);
   }
   if (c.y < g.ny - 1) {
     int64_t o = c.yp(g);
-    if (act[o]) t += ad[o] * (T)x[o];
+    if (act[o]) t += ad[o] * x(0, 1, 0);
   }
   if (c.z < g.nz - 1) {
     int64_t o = c.zp(g);
-    if (act[o]) t += ab[o] * (T)x[o];
+    if (act[o]) t += ab[o] * x(0, 0, 1);
   }
   return t;
 }
 
-// The PCG's own SpMV.  The PCG vectors are zero on inactive cells and the
-// couplings are finite (k_mask_system), so the neighbour activity tests of
-// apply_row drop out: every load is unconditional and independent, and the
-// result equals applyCompressedMatrix.
-template <class T>
-__device__ __forceinline__ T apply_row_pcg(const Tiled& g, const Cell& c, const T* __restrict__ adiag,
-                                           const T* __restrict__ al, const T* __restrict__ ad,
-                                           const T* __restrict__ ab, const T* __restrict__ x) {
-  const int64_t e = c.e;
-  const bool hx = c.x > 0, hy = c.y > 0, hz = c.z > 0;
-  const bool px = c.x < g.nx - 1, py = c.y < g.ny - 1, pz = c.z < g.nz - 1;
-  const int64_t oxm = hx ? c.xm(g) : e, oym = hy ? c.ym(g) : e, ozm = hz ? c.zm(g) : e;
-  const int64_t oxp = px ? c.xp(g) : e, oyp = py ? c.yp(g) : e, ozp = pz ? c.zp(g) : e;
-  const T cxm = hx ? al[e] : T(0), cym = hy ? ad[e] : T(0), czm = hz ? ab[e] : T(0);
-  const T cxp = px ? al[oxp] : T(0), cyp = py ? ad[oyp] : T(0), czp = pz ? ab[ozp] : T(0);
-  T t = adiag[e] * x[e];
-  t += cxm * x[oxm];
-  t += cym * x[oym];
-  t += czm * x[ozm];
-  t += cxp * x[oxp];
-  t += cyp * x[oyp];
-  t += czp * x[ozp];
-  return t;
-}
-
-// Each block walks a contiguous range of row blocks (consecutive slots of a
-// tile), so the neighbour rows it reads (x and z neighbours, the upper
-// couplings) were just loaded by the same block; two row blocks per pass.
-// (Measured against two alternatives at 128^3-512^3: per-warp row streaming
-// with register windows, and a multistage cp.async slab pipeline; both were
-// slower.)
-template <class T>
-__global__ void __launch_bounds__(kThreads)
-    k_spmv(Tiled g, const T* __restrict__ adiag, const T* __restrict__ al,
-           const T* __restrict__ ad, const T* __restrict__ ab, const uint8_t* __restrict__ act,
-           const T* __restrict__ x, T* __restrict__ y, double* partials, PcgScalars* sc,
-           int use_skip) {
-  if (use_skip && sc->done != DONE_RUNNING) return;
-  double acc = 0.0;
-  const int nrb = g.ntiles() * g.nz;
-  const int chunk = (nrb + gridDim.x - 1) / gridDim.x;
-  const int rb_end = min(nrb, (int)(blockIdx.x + 1) * chunk);
-  for (int rb0 = blockIdx.x * chunk; rb0 < rb_end; rb0 += 2) {
-    const int rb1 = rb0 + 1;
-    Cell c0, c1;
-    c0.init(g, rb0, threadIdx.x);
-    c1.init(g, rb1 < rb_end ? rb1 : rb0, threadIdx.x);
-    const T t0 = apply_row_pcg(g, c0, adiag, al, ad, ab, x);
-    const T t1 = apply_row_pcg(g, c1, adiag, al, ad, ab, x);
-    const bool a0 = c0.inside && act[c0.e], a1 = rb1 < rb_end && c1.inside && act[c1.e];
-    const T o0 = a0 ? t0 : T(0), o1 = a1 ? t1 : T(0);
-    acc += (double)x[c0.e] * (double)o0;
-    y[c0.e] = o0;
-    if (rb1 < rb_end) {
-      acc += (double)x[c1.e] * (double)o1;
-      y[c1.e] = o1;
-    }
-  }
-  reduce_finalize(acc, 0.0, partials, sc, FIN_SPMV);
-}
-
-// The PCG's SpMV as a stream over the z-slots of each tile.  In the tiled
-// layout the z-neighbours of a cell are its own lane's entries at the previous
-// and next slot, and its x-neighbours are the previous and next lanes' entries
-// at those slots.  A warp that owns row ty of a tile and walks the slots in
-// order therefore holds every x and z neighbour in a three-slot register window
-// (x neighbours by shuffle); the y neighbours are the adjacent rows of the same
-// slot, read through L1 where the block's other warps have just loaded them.
-// Each array element comes from HBM once, and no cell pays for a division or a
-// tile-edge branch: only the two edge lanes of a row reach into the next tiles.
-// The sum is the same as apply_row_pcg's, term for term.  A work item is the
-// TY row warps of one tile over a run of consecutive slots.
+// The PCG's SpMV.  The rows and couplings that touch an inactive cell are zero
+// (k_sweep_system) and the PCG vectors are zero there, so no activity is tested.
+// A block of 8 warps owns a 32 x 8 column tile (two sweep tiles) and walks a run of
+// its slots: warp ty is row ty, and lane tx has cell z = (slot - tx) mod nz of its
+// column, so that the z neighbours of a lane's cell are its own at the previous and
+// next slot and the x neighbours the adjacent lanes' there.  A three-slot register
+// window holds both (x by shuffle); the y neighbours are the adjacent rows at the
+// same z, and only the two edge lanes of a row reach into the next tiles.  Every load
+// is issued one slot ahead.  The upper couplings come from the neighbours' lower ones
+// (A symmetric, checkSystemSymmetry, :41-57).
+// The order in which a thread adds its products, and the tree that adds the threads'
+// sums, decide the last bits of s.Az and with them the rounding of every later
+// iterate: on systems whose MIC(0) factor is far from A (the tau terms), another
+// order moved the FP64 solution by 2e-9 relative.  The walk is therefore part of the
+// result, whatever the layout underneath.
 template <class T>
 __global__ void __launch_bounds__(kThreads, 3)
-    k_spmv_stream(Tiled g, const int2* __restrict__ tiles, const T* __restrict__ adiag, const T* __restrict__ al,
-                  const T* __restrict__ ad, const T* __restrict__ ab, const uint8_t* __restrict__ act,
-                  const T* __restrict__ x, T* __restrict__ y, double* partials, PcgScalars* sc, int use_skip,
-                  int chunks) {
+    k_spmv(SweepLayout g, const int2* __restrict__ tiles, const T* __restrict__ adiag, const T* __restrict__ al,
+           const T* __restrict__ ad, const T* __restrict__ ab, const T* __restrict__ x, T* __restrict__ y,
+           double* partials, PcgScalars* sc, int use_skip, int runs) {
   if (use_skip && sc->done != DONE_RUNNING) return;
-  constexpr int TY = Tiled::TY, RS = Tiled::TY * 32;  // elements per slot of a tile
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int nz = g.nz;
   double acc = 0.0;
-  // the listed tiles (those with an active cell; y stays zero on the others)
-  const int items = tiles[-1].x * chunks;
+  const int items = tiles[-1].x * runs;
+  // element of step sigma of a column: wb its warp tile's first element, ln its lane there
+  auto at = [](int64_t wb, int sigma, int ln) { return wb + SweepLayout::within<T>(sigma, ln); };
   for (int it = blockIdx.x; it < items; it += gridDim.x) {
-    const int li = it / chunks, ch = it - li * chunks;
-    const int tile = tiles[li].y * g.ntx + (tiles[li].x & 0xffff);
-    const int s0 = (int)((int64_t)nz * ch / chunks), s1 = (int)((int64_t)nz * (ch + 1) / chunks);
-    const int Y = tile / g.ntx, X = tile - Y * g.ntx;
-    const int xg = X * 32 + tx, yg = Y * TY + ty;
+    const int li = it / runs, run = it - li * runs;
+    const int s0 = (int)((int64_t)nz * run / runs), s1 = (int)((int64_t)nz * (run + 1) / runs);
+    const int xg = tiles[li].x * 32 + tx, yg = tiles[li].y * 8 + ty;
     const bool inside = xg < g.nx && yg < g.ny;
-    const bool hx = xg > 0, px = xg < g.nx - 1, hy = yg > 0, py = yg < g.ny - 1;
-    const int64_t tb = (int64_t)tile * g.tile_elems;
-    const int64_t row = tb + ty * 32 + tx;
-    // the rows of the same slot at y - 1 and y + 1 (read only when hy / py)
-    const int64_t rym = ty > 0 ? row - 32 : tb - (int64_t)g.ntx * g.tile_elems + (TY - 1) * 32 + tx;
-    const int64_t ryp = ty < TY - 1 ? row + 32 : tb + (int64_t)g.ntx * g.tile_elems + tx;
-    // the lanes across the x edges: lane 0's x - 1 is lane 31 of tile X - 1 at
-    // slot s + 31, lane 31's x + 1 is lane 0 of tile X + 1 at slot s - 31
-    const int64_t rxm = tb - g.tile_elems + ty * 32 + 31, rxp = tb + g.tile_elems + ty * 32;
-    auto wrap = [nz](int v) { return v >= nz ? v - nz : (v < 0 ? v + nz : v); };
-    int sm = wrap(s0 - 1), sp = wrap(s0 + 1), s31 = wrap(wrap(s0 + 31 % nz)), sm31 = wrap(wrap(s0 - 31 % nz));
-    int z = wrap(s0 - tx % nz);
-    T x_m = __ldg(x + row + (int64_t)sm * RS), x_c = __ldg(x + row + (int64_t)s0 * RS),
-      x_p = __ldg(x + row + (int64_t)sp * RS);
-    T al_c = __ldg(al + row + (int64_t)s0 * RS), al_p = __ldg(al + row + (int64_t)sp * RS);
-    T ab_c = __ldg(ab + row + (int64_t)s0 * RS), ab_p = __ldg(ab + row + (int64_t)sp * RS);
-    // the other loads of a slot are issued one slot ahead too (slot sp is a
-    // valid slot index at the end of the run as well, so they stay in bounds)
+    const bool hx = inside && xg > 0, px = inside && xg < g.nx - 1, hy = inside && yg > 0, py = inside && yg < g.ny - 1;
+    // columns this lane reads: its own, the rows at y - 1 and y + 1 (read only when hy /
+    // py), and for the edge lanes those at x - 1 and x + 1; outside the grid its own
+    // stands in for padding that holds zeros, or for a column past the last tile
+    auto column = [&](int X, int Y, int64_t& wb, int& ln, int& skew) {
+      wb = g.chunk0(X >> 4, Y >> 3, ((Y >> 2) & 1) * 2 + ((X >> 3) & 1)) * 128;
+      ln = (Y & 3) * 8 + (X & 7);
+      skew = (Y & 3) + (X & 7);
+    };
     const bool ex0 = tx == 0 && hx, ex31 = tx == 31 && px;
-    T d_n = __ldg(adiag + row + (int64_t)s0 * RS), adc_n = __ldg(ad + row + (int64_t)s0 * RS);
-    uint8_t a_n = __ldg(act + row + (int64_t)s0 * RS);
-    T ym_n = hy ? __ldg(x + rym + (int64_t)s0 * RS) : T(0), yp_n = py ? __ldg(x + ryp + (int64_t)s0 * RS) : T(0),
-      adp_n = py ? __ldg(ad + ryp + (int64_t)s0 * RS) : T(0);
-    T xme_n = ex0 ? __ldg(x + rxm + (int64_t)s31 * RS) : T(0), xpe_n = ex31 ? __ldg(x + rxp + (int64_t)sm31 * RS) : T(0),
-      alpe_n = ex31 ? __ldg(al + rxp + (int64_t)sm31 * RS) : T(0);
+    int64_t wc, wym, wyp, wxe;
+    int lc, lym, lyp, lxe, kc, kym, kyp, kxe;
+    column(xg < g.ntx * 16 ? xg : xg - 16, yg, wc, lc, kc);
+    column(xg < g.ntx * 16 ? xg : xg - 16, hy ? yg - 1 : yg, wym, lym, kym);
+    column(xg < g.ntx * 16 ? xg : xg - 16, py ? yg + 1 : yg, wyp, lyp, kyp);
+    column(ex0 ? xg - 1 : ex31 ? xg + 1 : (xg < g.ntx * 16 ? xg : xg - 16), yg, wxe, lxe, kxe);
+    auto wrap = [nz](int v) { return v >= nz ? v - nz : v; };
+    int z = s0 - tx % nz;
+    if (z < 0) z += nz;
+    const int zm = z == 0 ? nz - 1 : z - 1;
+    int zp = wrap(z + 1);
+    T x_m = __ldg(x + at(wc, zm + kc, lc)), x_c = __ldg(x + at(wc, z + kc, lc)), x_p = __ldg(x + at(wc, zp + kc, lc));
+    T al_c = __ldg(al + at(wc, z + kc, lc)), al_p = __ldg(al + at(wc, zp + kc, lc));
+    T ab_c = __ldg(ab + at(wc, z + kc, lc)), ab_p = __ldg(ab + at(wc, zp + kc, lc));
+    T d_n = __ldg(adiag + at(wc, z + kc, lc)), adc_n = __ldg(ad + at(wc, z + kc, lc));
+    T ym_n = hy ? __ldg(x + at(wym, z + kym, lym)) : T(0), yp_n = py ? __ldg(x + at(wyp, z + kyp, lyp)) : T(0),
+      adp_n = py ? __ldg(ad + at(wyp, z + kyp, lyp)) : T(0);
+    T xe_n = ex0 || ex31 ? __ldg(x + at(wxe, z + kxe, lxe)) : T(0), ale_n = ex31 ? __ldg(al + at(wxe, z + kxe, lxe)) : T(0);
     for (int s = s0; s < s1; s++) {
-      const int64_t e = row + (int64_t)s * RS;
-      const int s2 = wrap(sp + 1);
-      const T d = d_n, adc = adc_n, ymv = ym_n, ypv = yp_n, adp = adp_n, xme = xme_n, xpe = xpe_n, alpe = alpe_n;
-      const bool a = inside && a_n;
-      // next window entries and the next slot's loads first: their latency
+      const int z2 = wrap(zp + 1);
+      const T d = d_n, adc = adc_n, ymv = ym_n, ypv = yp_n, adp = adp_n, xe = xe_n, ale = ale_n;
+      // the next window entries and the next slot's loads first: their latency
       // overlaps this slot's work
-      const T x_n = __ldg(x + row + (int64_t)s2 * RS), al_n = __ldg(al + row + (int64_t)s2 * RS),
-              ab_n = __ldg(ab + row + (int64_t)s2 * RS);
-      {
-        const int64_t en = row + (int64_t)sp * RS;
-        const int s31n = wrap(s31 + 1), sm31n = wrap(sm31 + 1);
-        d_n = __ldg(adiag + en);
-        adc_n = __ldg(ad + en);
-        a_n = __ldg(act + en);
-        ym_n = hy ? __ldg(x + rym + (int64_t)sp * RS) : T(0);
-        yp_n = py ? __ldg(x + ryp + (int64_t)sp * RS) : T(0);
-        adp_n = py ? __ldg(ad + ryp + (int64_t)sp * RS) : T(0);
-        xme_n = ex0 ? __ldg(x + rxm + (int64_t)s31n * RS) : T(0);
-        xpe_n = ex31 ? __ldg(x + rxp + (int64_t)sm31n * RS) : T(0);
-        alpe_n = ex31 ? __ldg(al + rxp + (int64_t)sm31n * RS) : T(0);
-      }
+      const int64_t o2 = at(wc, z2 + kc, lc), o1 = at(wc, zp + kc, lc);
+      const T x_n = __ldg(x + o2), al_n = __ldg(al + o2), ab_n = __ldg(ab + o2);
+      d_n = __ldg(adiag + o1);
+      adc_n = __ldg(ad + o1);
+      ym_n = hy ? __ldg(x + at(wym, zp + kym, lym)) : T(0);
+      yp_n = py ? __ldg(x + at(wyp, zp + kyp, lyp)) : T(0);
+      adp_n = py ? __ldg(ad + at(wyp, zp + kyp, lyp)) : T(0);
+      xe_n = ex0 || ex31 ? __ldg(x + at(wxe, zp + kxe, lxe)) : T(0);
+      ale_n = ex31 ? __ldg(al + at(wxe, zp + kxe, lxe)) : T(0);
       const bool hz = z > 0, pz = z < nz - 1;
-      const T ym = hy ? ymv : x_c;
-      const T yp = py ? ypv : x_c;
-      T xm = __shfl_up_sync(kFull, x_m, 1), xp = __shfl_down_sync(kFull, x_p, 1),
-        alp = __shfl_down_sync(kFull, al_p, 1);
-      if (tx == 0) xm = hx ? xme : x_c;
+      T xm = __shfl_up_sync(kFull, x_m, 1), xp = __shfl_down_sync(kFull, x_p, 1), alp = __shfl_down_sync(kFull, al_p, 1);
+      if (tx == 0) xm = xe;
       if (tx == 31) {
-        xp = px ? xpe : x_c;
-        alp = px ? alpe : T(0);
+        xp = xe;
+        alp = ale;
       }
-      if (!hx) xm = x_c;
-      if (!px) xp = x_c;
       const T cxm = hx ? al_c : T(0), cym = hy ? adc : T(0), czm = hz ? ab_c : T(0);
       const T cxp = px ? alp : T(0), cyp = py ? adp : T(0), czp = pz ? ab_p : T(0);
       T t = d * x_c;
       t += cxm * xm;
-      t += cym * ym;
-      t += czm * (hz ? x_m : x_c);
+      t += cym * ymv;
+      t += czm * x_m;
       t += cxp * xp;
-      t += cyp * yp;
-      t += czp * (pz ? x_p : x_c);
-      const T o = a ? t : T(0);
-      y[e] = o;
+      t += cyp * ypv;
+      t += czp * x_p;
+      const T o = inside ? t : T(0);
+      if (inside) y[at(wc, z + kc, lc)] = o;
       acc += (double)x_c * (double)o;
       x_m = x_c;
       x_c = x_p;
@@ -557,18 +565,16 @@ __global__ void __launch_bounds__(kThreads, 3)
       al_p = al_n;
       ab_c = ab_p;
       ab_p = ab_n;
-      sm = s;
-      sp = s2;
-      s31 = wrap(s31 + 1);
-      sm31 = wrap(sm31 + 1);
-      z = wrap(z + 1);
+      z = zp;
+      zp = z2;
     }
   }
   reduce_finalize(acc, 0.0, partials, sc, FIN_SPMV);
 }
 
 // b = A x with the reference's activity tests (x may be non-zero on inactive
-// cells): applyCompressedMatrix for the apply entry point.
+// cells): applyCompressedMatrix for the apply entry point.  x and b in the
+// reference layout.
 __global__ void __launch_bounds__(kThreads)
     k_apply_checked(Tiled g, const double* __restrict__ adiag, const double* __restrict__ al,
                     const double* __restrict__ ad, const double* __restrict__ ab,
@@ -576,7 +582,11 @@ __global__ void __launch_bounds__(kThreads)
   SC_ROWBLOCK_LOOP(g) {
     Cell c;
     c.init(g, rb, threadIdx.x);
-    b[c.e] = (c.inside && act[c.e]) ? apply_row(g, c, adiag, al, ad, ab, act, x) : 0.0;
+    if (!c.inside) continue;
+    const int64_t r = lin(c.x, c.y, c.z, g.ny, g.nz);
+    b[r] = act[c.e] ? apply_row(g, c, adiag, al, ad, ab, act,
+                                [&](int dx, int dy, int dz) { return x[r + lin(dx, dy, dz, g.ny, g.nz)]; })
+                    : 0.0;
   }
 }
 
@@ -609,41 +619,30 @@ __global__ void __launch_bounds__(kThreads)
 
 // saxpy(pg, s, alpha); saxpy(r, z, -alpha); residual (:332-335, util.cc:394-402).
 // s and Az are zero on inactive cells, so the masked updates of the reference
-// are the plain updates here; four independent elements per thread per pass.
+// are the plain updates here.
 template <class T>
 __global__ void __launch_bounds__(kThreads)
-    k_axpy(Tiled g, const int2* __restrict__ tiles, const T* __restrict__ s,
+    k_axpy(SweepLayout g, const int2* __restrict__ tiles, const T* __restrict__ s,
            const T* __restrict__ Az, T* __restrict__ p, T* __restrict__ r, double* partials,
            PcgScalars* sc, int fin = FIN_AXPY) {
   if (sc->done != DONE_RUNNING) return;
   const T alpha = (T)sc->alpha;
   double s2 = 0.0, mx = 0.0;
-  const int nch = slot_count(g, tiles);
-  for (int c0 = blockIdx.x; c0 < nch; c0 += 4 * gridDim.x) {
-    T sv[4], av[4], pv[4], rv[4];
-    int64_t ee[4];
+  const int nch = unit_count(g, tiles);
+  for (int c = first_unit(); c < nch; c += kUnits * gridDim.x) {
+    const int64_t e = unit_elem(g, tiles, c);
+    const Vec4<T> sv = vload(s + e), av = vload(Az + e);
+    Vec4<T> pv = vload(p + e), rv = vload(r + e);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const int c = c0 + k * (int)gridDim.x;
-      const bool in = c < nch;
-      const int64_t e = in ? slot_elem(g, tiles, c) : 0;
-      ee[k] = in ? e : -1;
-      sv[k] = in ? s[e] : T(0);
-      av[k] = in ? Az[e] : T(0);
-      pv[k] = in ? p[e] : T(0);
-      rv[k] = in ? r[e] : T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int64_t e = ee[k];
-      if (e < 0) continue;
-      p[e] = pv[k] + alpha * sv[k];
-      const T rn = rv[k] + (-alpha) * av[k];
-      r[e] = rn;
-      const double dv = (double)rn;
+      pv.e[k] = pv.e[k] + alpha * sv.e[k];
+      rv.e[k] = rv.e[k] + (-alpha) * av.e[k];
+      const double dv = (double)rv.e[k];
       s2 += dv * dv;
       mx = fmax(mx, fabs(dv));
     }
+    vstore(p + e, pv);
+    vstore(r + e, rv);
   }
   reduce_finalize(s2, mx, partials, sc, fin);
 }
@@ -652,62 +651,148 @@ __global__ void __launch_bounds__(kThreads)
 // on inactive cells.
 template <class T>
 __global__ void __launch_bounds__(kThreads)
-    k_sa(Tiled g, const int2* __restrict__ tiles, const T* __restrict__ z, T* __restrict__ s,
+    k_sa(SweepLayout g, const int2* __restrict__ tiles, const T* __restrict__ z, T* __restrict__ s,
          double* partials, PcgScalars* sc) {
   if (sc->done != DONE_RUNNING) return;
   const T beta = (T)sc->beta;
-  const int nch = slot_count(g, tiles);
-  for (int c0 = blockIdx.x; c0 < nch; c0 += 4 * gridDim.x) {
-    T zv[4], sv[4];
-    int64_t ee[4];
+  const int nch = unit_count(g, tiles);
+  for (int c = first_unit(); c < nch; c += kUnits * gridDim.x) {
+    const int64_t e = unit_elem(g, tiles, c);
+    const Vec4<T> zv = vload(z + e);
+    Vec4<T> sv = vload(s + e);
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int c = c0 + k * (int)gridDim.x;
-      const bool in = c < nch;
-      const int64_t e = in ? slot_elem(g, tiles, c) : 0;
-      ee[k] = in ? e : -1;
-      zv[k] = in ? z[e] : T(0);
-      sv[k] = in ? s[e] : T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < 4; k++)
-      if (ee[k] >= 0) s[ee[k]] = zv[k] + beta * sv[k];
+    for (int k = 0; k < 4; k++) sv.e[k] = zv.e[k] + beta * sv.e[k];
+    vstore(s + e, sv);
   }
   reduce_finalize(0.0, 0.0, partials, sc, FIN_SA);
 }
 
-// Upper couplings in own-cell form for the backward sweep:
-// uR(p) = cL(p+x) = A_L(p+x) E(p), etc. (the products of project-solver.cc:296-302).
-template <class T>
+// The system in the SweepLayout, from the Tiled arrays: the diagonal and the
+// lower couplings, zero in inactive rows and where they couple to an inactive
+// cell (the reference never reads those), and the tau-weighted neighbour products
+// of the pivot recurrence (project-solver.cc:244-265).  For the Left term these are
+//   tau*A_L(p)*A_L(p-x+y) [if p-x+y active] + tau*A_L(p)*A_L(p-x+z) [if p-x+z active]
+// and likewise for Down and Back; they only depend on A.  PivotOp uses a
+// neighbour's terms only where that neighbour's pivot is not zero.  tile_act
+// (optional, zero on entry): 1 for the tiles holding an active cell.
 __global__ void __launch_bounds__(kThreads)
-    k_upper(Tiled g, const T* __restrict__ cL, const T* __restrict__ cD,
-            const T* __restrict__ cB, T* __restrict__ uR, T* __restrict__ uU, T* __restrict__ uF) {
-  SC_ROWBLOCK_LOOP(g) {
-    Cell c;
-    c.init(g, rb, threadIdx.x);
-    T a = T(0), b = T(0), d = T(0);
-    if (c.inside) {
-      if (c.x < g.nx - 1) a = cL[c.xp(g)];
-      if (c.y < g.ny - 1) b = cD[c.yp(g)];
-      if (c.z < g.nz - 1) d = cB[c.zp(g)];
+    k_sweep_system(SweepLayout g, Tiled tg, const double* __restrict__ adiag, const double* __restrict__ al,
+                   const double* __restrict__ ad, const double* __restrict__ ab, const uint8_t* __restrict__ act,
+                   double tau, double* __restrict__ o_d, double* __restrict__ o_l, double* __restrict__ o_dn,
+                   double* __restrict__ o_b, double* __restrict__ dL, double* __restrict__ dD,
+                   double* __restrict__ dB, uint8_t* __restrict__ tile_act) {
+  SC_CHUNK_LOOP(i, g) {
+    const ChunkPos c = chunk_pos<double>(g, i);
+    double v[7][4] = {};
+    bool any = false;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int x = c.x, y = c.y, z = c.z0 + j;
+      if (!c.inside || z < 0 || z >= g.nz) continue;
+      const int64_t e = tg.off(x, y, z);
+      if (!act[e]) continue;
+      any = true;
+      v[0][j] = adiag[e];
+      if (x > 0 && act[tg.off(x - 1, y, z)]) {
+        const double a = al[e];
+        v[1][j] = a;
+        if (y < g.ny - 1) {
+          const int64_t o = tg.off(x - 1, y + 1, z);
+          if (act[o]) v[4][j] += tau * a * al[o];
+        }
+        if (z < g.nz - 1) {
+          const int64_t o = tg.off(x - 1, y, z + 1);
+          if (act[o]) v[4][j] += tau * a * al[o];
+        }
+      }
+      if (y > 0 && act[tg.off(x, y - 1, z)]) {
+        const double a = ad[e];
+        v[2][j] = a;
+        if (x < g.nx - 1) {
+          const int64_t o = tg.off(x + 1, y - 1, z);
+          if (act[o]) v[5][j] += tau * a * ad[o];
+        }
+        if (z < g.nz - 1) {
+          const int64_t o = tg.off(x, y - 1, z + 1);
+          if (act[o]) v[5][j] += tau * a * ad[o];
+        }
+      }
+      if (z > 0 && act[tg.off(x, y, z - 1)]) {
+        const double a = ab[e];
+        v[3][j] = a;
+        if (x < g.nx - 1) {
+          const int64_t o = tg.off(x + 1, y, z - 1);
+          if (act[o]) v[6][j] += tau * a * ab[o];
+        }
+        if (y < g.ny - 1) {
+          const int64_t o = tg.off(x, y + 1, z - 1);
+          if (act[o]) v[6][j] += tau * a * ab[o];
+        }
+      }
     }
-    uR[c.e] = a;
-    uU[c.e] = b;
-    uF[c.e] = d;
+    double* const out[7] = {o_d, o_l, o_dn, o_b, dL, dD, dB};
+#pragma unroll
+    for (int k = 0; k < 7; k++) chunk_store(out[k] + c.e, v[k]);
+    // a warp holds one chunk
+    if (tile_act && __any_sync(kFull, any) && c.lane == 0) tile_act[c.tile] = 1;
   }
 }
 
-// Diagonals of the Eisenstat operator (FwdEisenstatOp), from the FP64 pivots:
-// Pinv = 1/E and Dt = 2/E^2 - Adiag where E != 0, else 0.
+// The factor streams of a precision, from the FP64 forward stream the pivot sweep
+// wrote (cL, cD, cB, E): the upper couplings in own-cell form for the backward
+// sweep, uR(p) = cL(p+x) = A_L(p+x) E(p) etc. (the products of
+// project-solver.cc:296-302), and in FP32 the forward stream with the diagonals of
+// the Eisenstat operator, Pinv = 1/E and Dt = 2/E^2 - Adiag where E != 0, else 0.
+template <class T>
 __global__ void __launch_bounds__(kThreads)
-    k_eisenstat_diag(int64_t n, const double* __restrict__ E, const double* __restrict__ adiag,
-                     float* __restrict__ pinv, float* __restrict__ dt) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
-    const double v = E[e];
-    const double pi = v != 0.0 ? 1.0 / v : 0.0;
-    pinv[e] = (float)pi;
-    dt[e] = v != 0.0 ? (float)(2.0 * pi * pi - adiag[e]) : 0.0f;
+    k_sweep_factor(SweepLayout g, const double* __restrict__ fwd64, const double* __restrict__ adiag, SysArrays<T> o) {
+  constexpr int S = kFwdStream<double>;
+  SC_CHUNK_LOOP(i, g) {
+    const ChunkPos c = chunk_pos<T>(g, i);
+    T b[4][4] = {}, f[6][4] = {};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int x = c.x, y = c.y, z = c.z0 + j;
+      if (!c.inside || z < 0 || z >= g.nz) continue;
+      const int64_t e = g.off<double>(x, y, z, S);  // cL; cD, cB, E 128 elements apart
+      const double E = fwd64[e + 3 * 128];
+      b[0][j] = (T)E;
+      if (x < g.nx - 1) b[1][j] = (T)fwd64[g.off<double>(x + 1, y, z, S, 0)];
+      if (y < g.ny - 1) b[2][j] = (T)fwd64[g.off<double>(x, y + 1, z, S, 1)];
+      if (z < g.nz - 1) b[3][j] = (T)fwd64[g.off<double>(x, y, z + 1, S, 2)];
+      if constexpr (sizeof(T) == 4) {
+        const double pi = E != 0.0 ? 1.0 / E : 0.0;
+        f[0][j] = (T)pi;
+        f[1][j] = E != 0.0 ? (T)(2.0 * pi * pi - adiag[g.off<double>(x, y, z)]) : T(0);
+        f[2][j] = (T)fwd64[e];
+        f[3][j] = (T)fwd64[e + 128];
+        f[4][j] = (T)fwd64[e + 256];
+        f[5][j] = (T)E;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) chunk_store(o.bwd + c.in_stream<T>(kBwdStream, k), b[k]);
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int k = 0; k < 6; k++) chunk_store(o.fwd + c.in_stream<T>(kFwdStream<T>, k), f[k]);
+    }
+  }
+}
+// The matrix in FP32 (the FP32 SpMV of the restarted defect correction).
+__global__ void __launch_bounds__(kThreads)
+    k_sweep_matrix32(SweepLayout g, const double* __restrict__ d, const double* __restrict__ l,
+                     const double* __restrict__ dn, const double* __restrict__ b, SysArrays<float> o) {
+  SC_CHUNK_LOOP(i, g) {
+    const int64_t c = i >> 5;
+    const int lane = (int)(i & 31);
+    const double* const in[4] = {d, l, dn, b};
+    float* const out[4] = {o.adiag, o.al, o.ad, o.ab};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const Quad<double> q = chunk_load(in[k] + c * 128 + lane * 2);
+      const float f[4] = {(float)q.e[0], (float)q.e[1], (float)q.e[2], (float)q.e[3]};
+      chunk_store(out[k] + c * 128 + lane * 4, f);
+    }
   }
 }
 
@@ -722,7 +807,9 @@ __global__ void __launch_bounds__(kThreads)
     Cell c;
     c.init(g, rb, threadIdx.x);
     if (c.inside && act[c.e]) {
-      double rv = b[c.e] - apply_row(g, c, adiag, al, ad, ab, act, x);
+      const double rv = b[c.e] - apply_row(g, c, adiag, al, ad, ab, act, [&](int dx, int dy, int dz) {
+                          return x[dx < 0 ? c.xm(g) : dx > 0 ? c.xp(g) : dy < 0 ? c.ym(g) : dy > 0 ? c.yp(g) : dz < 0 ? c.zm(g) : dz > 0 ? c.zp(g) : c.e];
+                        });
       s2 += rv * rv;
       mx = fmax(mx, fabs(rv));
     }
@@ -730,9 +817,10 @@ __global__ void __launch_bounds__(kThreads)
   reduce_finalize(s2, mx, partials, sc, FIN_NORMS);
 }
 
-// Mixed precision defect correction: x += scale d ; r -= scale A d (FP64 A, FP64 r).
+// Mixed precision defect correction: x += scale d ; r -= scale A d (FP64 A, x and r
+// in the Tiled layout; the FP32 correction d in the SweepLayout).
 __global__ void __launch_bounds__(kThreads)
-    k_mixed_update(Tiled g, const double* __restrict__ adiag, const double* __restrict__ al,
+    k_mixed_update(Tiled g, SweepLayout sg, const double* __restrict__ adiag, const double* __restrict__ al,
                    const double* __restrict__ ad, const double* __restrict__ ab,
                    const uint8_t* __restrict__ act, const float* __restrict__ d, double scale,
                    double* __restrict__ x, double* __restrict__ r, double* partials,
@@ -742,8 +830,10 @@ __global__ void __launch_bounds__(kThreads)
     Cell c;
     c.init(g, rb, threadIdx.x);
     if (!(c.inside && act[c.e])) continue;
-    const double t = apply_row(g, c, adiag, al, ad, ab, act, d);
-    x[c.e] += scale * (double)d[c.e];
+    const double t = apply_row(g, c, adiag, al, ad, ab, act, [&](int dx, int dy, int dz) {
+      return (double)d[sg.off<float>(c.x + dx, c.y + dy, c.z + dz)];
+    });
+    x[c.e] += scale * (double)d[sg.off<float>(c.x, c.y, c.z)];
     const double rv = r[c.e] - scale * t;
     r[c.e] = rv;
     s2 += rv * rv;
@@ -752,941 +842,30 @@ __global__ void __launch_bounds__(kThreads)
   reduce_finalize(s2, mx, partials, sc, FIN_NORMS);
 }
 
-// ---------------------------------------------------------------------------------
-// Wavefront sweeps.
-//
-// A persistent kernel: each CTA repeatedly takes a ticket, maps it to a tile in
-// dependency order, and sweeps the tile's i+j+k wavefront with TY compute warps
-// (warp = tile row ty, lane = tx).  At step s, lane tx of warp ty owns cell
-// z = s - ty - tx (forward) and reads one contiguous row of the tiled arrays.
-// Neighbour values inside the tile travel by shuffle (x), shared memory (y) and
-// registers (z).  Values from the neighbouring tiles arrive through a
-// communication warp that polls the neighbours' published progress and streams
-// their boundary rows into shared-memory rings; the same warp publishes this
-// tile's progress.  Every wait is bounded: on timeout the kernel raises
-// DEV_ERR_TIMEOUT, releases its dependants and finishes.
-
-// Cell operations of the three sweeps.  Each reads NV arrays at its own cell
-// (staged into shared memory by cp.async) plus the three already-computed
-// neighbour values xn, yn, zn.
-// compute() returns the value the recurrence passes on to the neighbours and
-// stores the op's outputs at element e itself.
-template <class T, bool SELFDOT = false>
-struct FwdOp {  // L q = r (project-solver.cc:276-288), c* = A_* E(neighbour); SELFDOT: acc q.q
-  static constexpr int NV = 5;
-  const T* src[NV];  // r, cL, cD, cB, E
-  T* out;            // q
-  __device__ __forceinline__ T compute(const T* v, T xn, T yn, T zn, int64_t e, double& acc) const {
-    T t = v[0];
-    t -= v[1] * xn;
-    t -= v[2] * yn;
-    t -= v[3] * zn;
-    const T q = t * v[4];
-    out[e] = q;
-    if (SELFDOT) acc += (double)q * (double)q;
-    return q;
-  }
-};
-
-template <class T>
-struct BwdOp {  // L^T z = q (project-solver.cc:293-305), u* = A_*(p+dir) E(p); sigma = z.r
-  static constexpr int NV = 6;
-  const T* src[NV];  // q, E, uR, uU, uF, r
-  T* out;            // z
-  __device__ __forceinline__ T compute(const T* v, T xn, T yn, T zn, int64_t e, double& acc) const {
-    T t = v[0];
-    t -= v[2] * xn;
-    t -= v[3] * yn;
-    t -= v[4] * zn;
-    T z = t * v[1];
-    out[e] = z;
-    acc += (double)z * (double)v[5];
-    return z;
-  }
-};
-
-// Eisenstat backward sweep with the search-direction update folded in:
-//   s = rh + beta s  (scaleAndAdd of the CG step), then t = L^-T s.
-// beta comes from the device scalars, read once per CTA (prepare).
-template <class T>
-struct BwdEisenstatOp {
-  static constexpr int NV = 6;
-  const T* src[NV];  // rh, s (previous), E, uR, uU, uF
-  T* out;            // t
-  T* s_out;          // s (in place of src[1]: each element is read before it is written)
-  T beta;
-  __device__ __forceinline__ void prepare(const PcgScalars* sc) { beta = (T)sc->beta; }
-  __device__ __forceinline__ T compute(const T* v, T xn, T yn, T zn, int64_t e, double&) const {
-    const T sv = v[0] + beta * v[1];
-    s_out[e] = sv;
-    T u = sv;
-    u -= v[3] * xn;
-    u -= v[4] * yn;
-    u -= v[5] * zn;
-    const T t = u * v[2];
-    out[e] = t;
-    return t;
-  }
-};
-
-// Ops without per-launch scalars.
-template <class Op, class = void>
-struct HasPrepare : std::false_type {};
-template <class Op>
-struct HasPrepare<Op, std::void_t<decltype(std::declval<Op&>().prepare(nullptr))>> : std::true_type {};
-
-// Eisenstat's form of the preconditioned operator (S. C. Eisenstat, "Efficient
-// implementation of a class of preconditioned conjugate gradient methods",
-// SIAM J. Sci. Stat. Comput. 2 (1981) 1-4).  With the MIC(0) factor
-// L = (P^-2 + F) P (P = diag(E), F the strictly lower part of A) and
-// A = K + K^T - Dt, K = P^-2 + F, Dt = 2 P^-2 - diag(A), the split operator is
-//   L^-1 A L^-T v = P^-1 t + L^-1 (P^-1 v - Dt t),   t = L^-T v,
-// so one backward sweep (t) and this forward sweep apply it: no SpMV.  The
-// recurrence carries q = L^-1 (P^-1 v - Dt t); the output is w = P^-1 t + q
-// and acc gathers v.w.  Pinv = 1/E and Dt are 0 on cells where E = 0.
-template <class T>
-struct FwdEisenstatOp {
-  static constexpr int NV = 8;
-  const T* src[NV];  // v, t, Pinv, Dt, cL, cD, cB, E
-  T* out;            // w
-  __device__ __forceinline__ T compute(const T* v, T xn, T yn, T zn, int64_t e, double& acc) const {
-    T u = v[2] * v[0];
-    u -= v[3] * v[1];
-    u -= v[4] * xn;
-    u -= v[5] * yn;
-    u -= v[6] * zn;
-    const T q = u * v[7];
-    const T w = v[2] * v[1] + q;
-    out[e] = w;
-    acc += (double)v[0] * (double)w;
-    return q;
-  }
-};
-
-// MIC(0) pivot (project-solver.cc:237-274), FP64.  The exchanged value is E.
-// E(q) != 0 exactly when q is active with Adiag(q) != 0, which is the guard the
-// reference tests before using E(q).  adm is Adiag masked by the active flag;
-// dL/dD/dB hold the tau-weighted products with the diagonal neighbours'
-// couplings (k_pivot_diag), so the sweep only streams its own row.
-struct PivotOp {
-  static constexpr int NV = 7;
-  const double* src[NV];  // adm, al, ad, ab, dL, dD, dB
-  double sigma;
-  double *out, *cL, *cD, *cB;
-  __device__ __forceinline__ double compute(const double* v, double EL, double ED, double EB,
-                                            int64_t e, double&) const {
-    const double adiag = v[0], al = v[1], ad = v[2], ab = v[3];
-    double E = 0.0;
-    if (adiag != 0.0) {
-      double ee = adiag;
-      if (EL != 0.0) {
-        ee -= (al * EL) * (al * EL);
-        ee -= v[4] / (EL * EL);
-      }
-      if (ED != 0.0) {
-        ee -= (ad * ED) * (ad * ED);
-        ee -= v[5] / (ED * ED);
-      }
-      if (EB != 0.0) {
-        ee -= (ab * EB) * (ab * EB);
-        ee -= v[6] / (EB * EB);
-      }
-      if (ee < sigma * adiag) ee = adiag;
-      E = 1.0 / sqrt(ee);
-    }
-    out[e] = E;
-    cL[e] = al * EL;
-    cD[e] = ad * ED;
-    cB[e] = ab * EB;
-    return E;
-  }
-};
-
-// The tau-weighted neighbour products of the pivot recurrence
-// (project-solver.cc:244-265): for the Left term
-//   tau*A_L(p)*A_L(p-x+y) [if p-x+y active] + tau*A_L(p)*A_L(p-x+z) [if p-x+z active]
-// and likewise for Down and Back.  They only depend on A.
-__global__ void __launch_bounds__(kThreads)
-    k_pivot_diag(Tiled g, const double* __restrict__ adiag, const double* __restrict__ al,
-                 const double* __restrict__ ad, const double* __restrict__ ab,
-                 const uint8_t* __restrict__ act, double tau, double* __restrict__ adm,
-                 double* __restrict__ dL, double* __restrict__ dD, double* __restrict__ dB) {
-  SC_ROWBLOCK_LOOP(g) {
-    Cell c;
-    c.init(g, rb, threadIdx.x);
-    double l = 0.0, d = 0.0, b = 0.0;
-    if (c.inside) {
-      const int x = c.x, y = c.y, z = c.z;
-      if (x > 0) {
-        const double a = al[c.e];
-        if (y < g.ny - 1) {
-          int64_t o = g.off(x - 1, y + 1, z);
-          if (act[o]) l += tau * a * al[o];
-        }
-        if (z < g.nz - 1) {
-          int64_t o = g.off(x - 1, y, z + 1);
-          if (act[o]) l += tau * a * al[o];
-        }
-      }
-      if (y > 0) {
-        const double a = ad[c.e];
-        if (x < g.nx - 1) {
-          int64_t o = g.off(x + 1, y - 1, z);
-          if (act[o]) d += tau * a * ad[o];
-        }
-        if (z < g.nz - 1) {
-          int64_t o = g.off(x, y - 1, z + 1);
-          if (act[o]) d += tau * a * ad[o];
-        }
-      }
-      if (z > 0) {
-        const double a = ab[c.e];
-        if (x < g.nx - 1) {
-          int64_t o = g.off(x + 1, y, z - 1);
-          if (act[o]) b += tau * a * ab[o];
-        }
-        if (y < g.ny - 1) {
-          int64_t o = g.off(x, y + 1, z - 1);
-          if (act[o]) b += tau * a * ab[o];
-        }
-      }
-    }
-    dL[c.e] = l;
-    dD[c.e] = d;
-    dB[c.e] = b;
-    adm[c.e] = (c.inside && act[c.e]) ? adiag[c.e] : 0.0;
-  }
-}
-
-template <int TY, bool FWD>
-__device__ __forceinline__ int wave_slot(const Tiled& g, int s, int ty) {
-  return FWD ? wrap_mod(s - ty, g.nz) : wrap_mod(g.nz + 29 + TY - s - ty, g.nz);
-}
-
-// Mailbox sentinel: a NaN payload that arithmetic never produces (the GPU's
-// canonical NaN has all mantissa bits set).
-template <class T>
-struct Sentinel;
-template <>
-struct Sentinel<double> {
-  using Bits = unsigned long long;
-  static constexpr Bits bits = 0x7ff4deadbeefcafeull;
-};
-template <>
-struct Sentinel<float> {
-  using Bits = unsigned int;
-  static constexpr Bits bits = 0x7fa5deadu;
-};
-template <class T>
-__device__ __forceinline__ typename Sentinel<T>::Bits mb_load(const T* p) {
-  typename Sentinel<T>::Bits v;
-  if constexpr (sizeof(T) == 8)
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  else
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-template <class T>
-__device__ __forceinline__ T mb_value(typename Sentinel<T>::Bits b) {
-  T v;
-  memcpy(&v, &b, sizeof(T));
-  return v;
-}
-// Every mailbox access is a strong (relaxed, gpu-scope) operation, so writes by
-// one CTA and polls by another are coherent under the PTX memory model.
-template <class T>
-__device__ __forceinline__ void mb_store_bits(T* p, typename Sentinel<T>::Bits b) {
-  if constexpr (sizeof(T) == 8)
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(b) : "memory");
-  else
-    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(b) : "memory");
-}
-template <class T>
-__device__ __forceinline__ void mb_store(T* p, T v) {
-  typename Sentinel<T>::Bits b;
-  memcpy(&b, &v, sizeof(T));
-  mb_store_bits(p, b);
-}
-template <class T>
-__device__ __forceinline__ void mb_reset(T* p) {
-  mb_store_bits(p, Sentinel<T>::bits);
-}
-
-// B-byte copy global -> shared (B = 4, 8 or 16; both addresses B-byte aligned);
-// 16-byte copies bypass L1.
-template <int B, class T>
-__device__ __forceinline__ void cp_async_bytes(T* dst, const T* src) {
-  unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (B == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-  else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(B) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// Shared state of one wavefront CTA.
-template <class T, int TY>
-struct WaveShared {
-  T xch[2][TY][32];
-  T bufX[kRing][TY];
-  T bufY[kRing][32];
-  volatile int done;     // compute steps completed
-  volatile int availX;   // ring entries loaded
-  volatile int availY;
-  volatile int abort;
-  int tile;
-  bool last;
-  double ssum[TY + 3];
-};
-
-// Hand-off ring between the CTAs of a thread-block cluster (distributed shared
-// memory): the y-boundary row a tile passes to the next tile of the same
-// cluster goes straight into that CTA's ring.  One 64-bit word per lane and
-// entry holds the FP32 value in its low half and a stamp (the cluster tile's
-// ticket << 12 | the entry) in its high half, written with one store, so a
-// consumer that sees the stamp it expects sees the value: no fence and no
-// reset.  Each CTA fills its ring with an impossible stamp at launch.
-constexpr int kClRing = 32;
-constexpr unsigned kClNoStamp = 0xffffffffu;
-__device__ __forceinline__ unsigned cl_stamp(int ticket, int e) { return ((unsigned)ticket << 12) | (unsigned)e; }
-__device__ __forceinline__ void st_relaxed_cluster_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.cluster.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed_cluster_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.relaxed.cluster.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ int ld_relaxed_cluster_s32(const int* p) {
-  int v;
-  asm volatile("ld.relaxed.cluster.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-template <class T>
-__device__ __forceinline__ T cl_value(unsigned long long w) {
-  if constexpr (sizeof(T) == 4)
-    return __uint_as_float((unsigned)(w & 0xffffffffull));
-  else
-    return T(0);
-}
-template <class T>
-__device__ __forceinline__ unsigned long long cl_word(int ticket, int e, T v) {
-  if constexpr (sizeof(T) == 4)
-    return ((unsigned long long)cl_stamp(ticket, e) << 32) | (unsigned long long)__float_as_uint(v);
-  else
-    return 0ull;
-}
-
-// Give up: flag the error and release the compute warps.
-template <class T, int TY>
-__device__ __forceinline__ void wave_abort(const WaveArgs& a, WaveShared<T, TY>& sh, int NS) {
-  atomicOr(&a.sc->err, DEV_ERR_TIMEOUT);
-  sh.abort = 1;
-  sh.availX = NS;
-  sh.availY = NS;
-}
-
-// A wait ends early only when another wait of the sweep gave up (the timeout
-// bit): the other status bits (a breakdown, a non-finite dot product) belong
-// to the iteration, and a sweep run after one of them still completes.
-__device__ __forceinline__ bool wave_should_stop(const WaveArgs& a, int& spins,
-                                                 volatile int* s_abort, int limit) {
-  if (*s_abort) return true;
-#if SC_WAVE_CTL_NS > 0
-  __nanosleep(SC_WAVE_CTL_NS);
-#endif
-  ++spins;
-  if ((spins & 63) == 0 && (ld_relaxed_gpu_u32(&a.sc->err) & DEV_ERR_TIMEOUT)) return true;
-  return spins > limit;
-}
-
-// Mailboxes.  The producer tile writes each boundary value it computes into
-// the mailbox of the tile that consumes it, at the consumer's ring-entry index:
-//   x: mbx[consumer][e][ty]  (e = producer step - 31)
-//   y: mby[consumer][e][tx]  (e = producer step - (TY-1))
-// The consumer's loader warps poll those words until they stop holding the
-// sentinel, copy them to the shared-memory rings and write the sentinel back,
-// which leaves the mailboxes ready for the next sweep.  No fences are needed:
-// every mailbox word carries exactly one value per sweep.
-template <class T, int TY, bool FWD>
-__device__ void wave_load_x(const WaveArgs& a, WaveShared<T, TY>& sh, T* mb, int NS, int limit) {
-  const Tiled& g = a.g;
-  const int lane = threadIdx.x & 31;
-  constexpr int EPB = 32 / TY;  // entries per 32 lanes
-  int lx = 0, spins = 0;
-  while (lx < NS) {
-    const int want = min(NS, sh.done + kRing);
-    if (lx >= want) {
-      if (wave_should_stop(a, spins, &sh.abort, limit)) break;
-      continue;
-    }
-    // poll up to 8*EPB entries: lane handles (entry lx + k*EPB + lane/TY, ty = lane%TY)
-    const int ty = lane % TY;
-    typename Sentinel<T>::Bits v[8];
-    unsigned ready = 0;  // bit k*EPB+j: entry lx+k*EPB+j fully ready
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int e = lx + k * EPB + lane / TY;
-      const int z = FWD ? e - ty : g.nz - 1 - e + (TY - 1 - ty);
-      const bool need = e < want && z >= 0 && z < g.nz;
-      v[k] = need ? mb_load(mb + (int64_t)e * TY + ty) : (typename Sentinel<T>::Bits)0;
-      const bool ok = e < want && (!need || v[k] != Sentinel<T>::bits);
-      const unsigned bal = __ballot_sync(kFull, ok);
-#pragma unroll
-      for (int j = 0; j < EPB; j++)
-        if (((bal >> (j * TY)) & ((1u << TY) - 1u)) == ((1u << TY) - 1u)) ready |= 1u << (k * EPB + j);
-    }
-    const int nready = __ffs(~ready) - 1;  // leading ready entries
-    const int take = nready < 0 ? 8 * EPB : nready;
-    if (take > 0) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int j = k * EPB + lane / TY;
-        if (j < take) {
-          const int e = lx + j;
-          const int z = FWD ? e - ty : g.nz - 1 - e + (TY - 1 - ty);
-          const bool need = z >= 0 && z < g.nz;
-          sh.bufX[e % kRing][ty] = need ? mb_value<T>(v[k]) : T(0);
-          if (need) mb_reset(mb + (int64_t)e * TY + ty);
-        }
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) sh.availX = lx + take;
-      lx += take;
-      spins = 0;
-      continue;
-    }
-    if (wave_should_stop(a, spins, &sh.abort, limit)) break;
-  }
-  if (lx < NS && lane == 0) wave_abort(a, sh, NS);
-}
-
-template <class T, int TY, bool FWD>
-__device__ void wave_load_y(const WaveArgs& a, WaveShared<T, TY>& sh, T* mb, int NS, int limit) {
-  const Tiled& g = a.g;
-  const int lane = threadIdx.x & 31;
-  int ly = 0, spins = 0;
-  while (ly < NS) {
-    const int want = min(NS, sh.done + kRing);
-    if (ly >= want) {
-      if (wave_should_stop(a, spins, &sh.abort, limit)) break;
-      continue;
-    }
-    typename Sentinel<T>::Bits v[8];
-    unsigned ready = 0;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      const int e = ly + k;
-      // the consumer is warp 0 (forward) or warp TY-1 (backward), lane = tx
-      const int z = FWD ? e - lane : g.nz - 1 - (e - (31 - lane));
-      const bool need = e < want && z >= 0 && z < g.nz;
-      v[k] = need ? mb_load(mb + (int64_t)e * 32 + lane) : (typename Sentinel<T>::Bits)0;
-      const bool ok = e < want && (!need || v[k] != Sentinel<T>::bits);
-      if (__all_sync(kFull, ok)) ready |= 1u << k;
-    }
-    const int nready = __ffs(~ready) - 1;
-    const int take = nready < 0 ? 8 : nready;
-    if (take > 0) {
-#pragma unroll
-      for (int k = 0; k < 8; k++) {
-        if (k < take) {
-          const int e = ly + k;
-          const int z = FWD ? e - lane : g.nz - 1 - (e - (31 - lane));
-          const bool need = z >= 0 && z < g.nz;
-          sh.bufY[e % kRing][lane] = need ? mb_value<T>(v[k]) : T(0);
-          if (need) mb_reset(mb + (int64_t)e * 32 + lane);
-        }
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) sh.availY = ly + take;
-      ly += take;
-      spins = 0;
-      continue;
-    }
-    if (wave_should_stop(a, spins, &sh.abort, limit)) break;
-  }
-  if (ly < NS && lane == 0) wave_abort(a, sh, NS);
-}
-
-// One CTA per SM: the sweep is issue-bound, and capping registers for two
-// CTAs per SM measured slower at 128^3, 256^3 and 512^3.
-//
-// CL > 0 (FP32 only): the grid is made of thread-block clusters of CL CTAs.  A
-// ticket then names a cluster tile, CL tiles stacked along y in one column
-// (X, Yc * CL + rank), and a tile hands its y-boundary row to the next tile of
-// its cluster through that CTA's shared memory (kClRing) instead of a global
-// mailbox; only the hand-offs between clusters (along y at the cluster edges,
-// and along x) use the mailboxes.  The CTAs of a cluster take each ticket
-// together and meet at a cluster barrier after each cluster tile.
-template <class T, int TY, bool FWD, class Op, int CL = 0>
-__global__ void __launch_bounds__((TY + 3) * 32, 1) k_wave(const WaveArgs a, const Op op_arg) {
-  // warps 0..TY-1: tile rows (compute only, no fences: a fence would wait for
-  // the prefetch loads in flight); warp TY: control (flags, ring waits);
-  // warps TY+1, TY+2: x and y mailbox loaders.
-  constexpr bool CLU = CL > 0;
-  static_assert(!CLU || sizeof(T) == 4, "cluster hand-off rings carry FP32 values");
-  constexpr int NBAR = (TY + 1) * 32;
-  __shared__ WaveShared<T, TY> sh;
-  __shared__ unsigned long long ringY[CLU ? kClRing : 1][32];
-  extern __shared__ __align__(16) unsigned char wave_dyn[];
-  T* stage = reinterpret_cast<T*>(wave_dyn);  // [kStage][TY][NV][32]
-  if (a.use_skip && a.sc->done != DONE_RUNNING) return;
-  // an earlier sweep gave up: do not wait again (a cluster decides together,
-  // below, since CTAs could read the status word at different moments)
-  if (!CLU && (a.sc->err & DEV_ERR_TIMEOUT)) return;
-  int rank = 0;
-  if constexpr (CLU) {
-    rank = (int)cooperative_groups::this_cluster().block_rank();
-    for (int i = threadIdx.x; i < kClRing * 32; i += blockDim.x) ringY[i / 32][i % 32] = (unsigned long long)kClNoStamp << 32;
-    cooperative_groups::this_cluster().sync();  // every CTA of the cluster runs before any remote access
-  }
-  Op op = op_arg;
-  if constexpr (HasPrepare<Op>::value) op.prepare(a.sc);
-  const int slim = a.sc->spin_limit > 0 ? a.sc->spin_limit : kSpinLimit;  // bound of every wait
-  const Tiled& g = a.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ntiles = g.ntiles();
-  const int NS = g.nz + 31 + TY - 1;
-  T* mbx = reinterpret_cast<T*>(a.mbx);
-  T* mby = reinterpret_cast<T*>(a.mby);
-  double acc = 0.0;
-  // the tickets: entries of the order list (tiles, or cluster tiles of CL
-  // tiles along y), whose length sits in the header entry before the first
-  const int nticket = a.order[-1].x;
-  for (;;) {
-    if constexpr (CLU) {
-      if (threadIdx.x == 0) {
-        sh.done = 0;
-        sh.availX = 0;
-        sh.availY = 0;
-        sh.abort = 0;
-      }
-      if (rank == 0 && threadIdx.x == 0) {
-        const int tk = atomicAdd(a.ticket, 1);
-        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-        for (int r = 0; r < CL; r++) *cl.map_shared_rank(&sh.tile, r) = tk;
-      }
-      cooperative_groups::this_cluster().sync();
-    } else {
-      if (threadIdx.x == 0) {
-        sh.tile = atomicAdd(a.ticket, 1);
-        sh.done = 0;
-        sh.availX = 0;
-        sh.availY = 0;
-        sh.abort = 0;
-      }
-      __syncthreads();
-    }
-    const int t = sh.tile;
-    if (t >= nticket) break;
-    // entry: x = X | neighbour bits << 16, y = the tile row (cluster tile row);
-    // bit 0/1: the unit at X - 1 / X + 1 is swept, bit 2/3: the unit below /
-    // above.  A unit that is not swept (no active cell) holds zeros and has
-    // zero couplings to this one, so its boundary values are zeros.
-    const int2 XY = a.order[FWD ? t : nticket - 1 - t];
-    const int X = XY.x & 0xffff, nb = XY.x >> 16;
-    const int Y = CLU ? XY.y * CL + rank : XY.y;
-    // a cluster tile at the top edge can have CTAs without a tile
-    if (Y < g.nty) {
-    const int tid = Y * g.ntx + X;
-    // producers within this cluster tile (along y, through the rings), and
-    // consumers within it
-    const bool inner_in = CLU && (FWD ? rank > 0 : rank < CL - 1);
-    const bool inner_out = CLU && (FWD ? rank < CL - 1 : rank > 0);
-    const bool hasX = FWD ? (nb & 1) : (nb & 2);
-    const bool hasY = (FWD ? Y > 0 : Y < g.nty - 1) && (inner_in || (FWD ? (nb & 4) : (nb & 8)));
-    // consumers of this tile's boundary values
-    const bool outX = FWD ? (nb & 2) : (nb & 1);
-    const bool outY = (FWD ? Y < g.nty - 1 : Y > 0) && (inner_out || (FWD ? (nb & 8) : (nb & 4)));
-    const int cX = FWD ? tid + 1 : tid - 1, cY = FWD ? tid + g.ntx : tid - g.ntx;
-    // y boundary rows within a cluster travel through the rings
-    const bool ydin = CLU && hasY && inner_in;
-    const bool ydout = CLU && outY && inner_out;
-    const int64_t base = g.tile_base(X, Y);
-    if (warp == TY) {
-      // control warp: keeps the compute warps one step behind the rings; it
-      // waits up to four times the loaders' bound
-      const int ctl_limit = slim > (1 << 28) ? (1 << 30) : 4 * slim;
-      auto wait_avail = [&](int s) {
-        int spins = 0;
-        if (ydin) {
-          // this lane's word of ring entry s, where the consumer row needs it
-          // (the same z test as the mailbox loader's)
-          const int zc = FWD ? s - lane : g.nz - 1 - (s - (31 - lane));
-          const bool need = zc >= 0 && zc < g.nz;
-          const unsigned want = cl_stamp(t, s);
-          const unsigned long long* w = &ringY[s % kClRing][lane];
-          for (;;) {
-            const bool mine = !need || (unsigned)(ld_relaxed_cluster_u64(w) >> 32) == want;
-            const bool ok = mine && !(hasX && sh.availX <= s);
-            if (__all_sync(kFull, ok) || __any_sync(kFull, sh.abort)) break;
-            if (++spins > ctl_limit) {
-              if (lane == 0) wave_abort(a, sh, NS);
-              break;
-            }
-#if SC_WAVE_CTL_NS > 0
-            __nanosleep(SC_WAVE_CTL_NS);
-#endif
-          }
-        } else {
-          while (((hasX && sh.availX <= s) || (hasY && sh.availY <= s)) && !sh.abort) {
-            if (++spins > ctl_limit) {
-              if (lane == 0) wave_abort(a, sh, NS);
-              break;
-            }
-#if SC_WAVE_CTL_NS > 0
-            __nanosleep(SC_WAVE_CTL_NS);
-#endif
-          }
-        }
-        __syncwarp();
-        __threadfence_block();
-      };
-      wait_avail(0);
-      named_bar_sync(1, NBAR);
-      for (int s = 0; s < NS; s++) {
-        if (lane == 0) sh.done = s;  // steps < s are complete
-        if (s + 1 < NS) wait_avail(s + 1);
-        named_bar_sync(1, NBAR);
-      }
-      if (lane == 0) sh.done = NS;
-    } else if (warp == TY + 1) {
-      if (hasX) wave_load_x<T, TY, FWD>(a, sh, mbx + (int64_t)tid * a.mb_stride_x, NS, slim);
-    } else if (warp == TY + 2) {
-      if (hasY && !ydin) wave_load_y<T, TY, FWD>(a, sh, mby + (int64_t)tid * a.mb_stride_y, NS, slim);
-    } else {
-      const int ty = warp;
-      T* outx = outX ? mbx + (int64_t)cX * a.mb_stride_x : nullptr;
-      T* outy = (outY && !ydout) ? mby + (int64_t)cY * a.mb_stride_y : nullptr;
-      const bool xsrc = FWD ? (lane == 31) : (lane == 0);        // lane feeding the x consumer
-      const bool ysrc = FWD ? (ty == TY - 1) : (ty == 0);        // warp feeding the y consumer
-      // the ring of the cluster CTA this tile feeds along y, and its progress
-      unsigned long long* rring = nullptr;
-      const int* rdone = nullptr;
-      int cdone = 0;  // the consumer's completed steps, as last read
-      if constexpr (CLU) {
-        if (ydout && ysrc) {
-          cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-          const int cr = FWD ? rank + 1 : rank - 1;
-          rring = cl.map_shared_rank(&ringY[0][0], cr);
-          rdone = const_cast<const int*>(cl.map_shared_rank(const_cast<int*>(&sh.done), cr));
-        }
-      }
-      // slot of the row this warp touches at step s: forward (s - ty) mod nz,
-      // backward (nz + 29 + TY - s - ty) mod nz; advanced incrementally.
-      int cslot = wave_slot<TY, FWD>(g, 0, ty);
-      int pslot = cslot;
-      const int64_t rowbase = base + (int64_t)ty * 32 + lane;
-      const int64_t rstride = (int64_t)TY * 32;
-      auto advance = [&](int& sl) {
-        if (FWD) {
-          if (++sl == g.nz) sl = 0;
-        } else {
-          if (--sl < 0) sl = g.nz - 1;
-        }
-      };
-      // The warp stages the NV input rows of step s + kStage into ring slot
-      // s mod kStage at the end of step s, as kChunk-byte cp.async chunks spread
-      // over the lanes (CPL per lane, pointers fixed per tile): after the step's
-      // dependent chain, so the copies are issued while the other warps are
-      // still on theirs.  The warp's lanes read that slot at the start of step s
-      // (a __syncwarp orders the reads before the refill); each lane waits for
-      // its own chunks of step s + 1 before the barrier of step s, and the
-      // barrier makes every lane's chunks visible to the warp.
-      constexpr int kStage = wave_stages<T, Op::NV>();
-      constexpr int kChunk = sizeof(T) == 8 ? SC_WAVE_CHUNK64 : SC_WAVE_CHUNK32;  // bytes
-      constexpr int EPC = kChunk / (int)sizeof(T);           // elements per chunk
-      constexpr int CPR = 32 / EPC;                          // chunks per row
-      constexpr int CPL = (Op::NV * CPR + 31) / 32;          // chunks per lane
-      constexpr size_t kStageStride = (size_t)TY * Op::NV * 32;  // elements per ring slot
-      const T* my_stage = stage + (size_t)ty * Op::NV * 32 + lane;
-      const T* cg[CPL];
-      int coff[CPL];
-#pragma unroll
-      for (int i = 0; i < CPL; i++) {
-        const int j = lane + 32 * i;
-        const int k = j / CPR, c = j - k * CPR;
-        const T* src = op.src[0];
-#pragma unroll
-        for (int kk = 1; kk < Op::NV; kk++)
-          if (k == kk) src = op.src[kk];
-        cg[i] = j < Op::NV * CPR ? src + base + (int64_t)ty * 32 + c * EPC : nullptr;
-        coff[i] = (ty * Op::NV + k) * 32 + c * EPC;
-      }
-      auto issue = [&](int sl, int ridx) {
-        const int64_t so = (int64_t)sl * rstride;
-#pragma unroll
-        for (int i = 0; i < CPL; i++)
-          if (Op::NV * CPR % 32 == 0 || cg[i]) cp_async_bytes<kChunk>(stage + ridx * kStageStride + coff[i], cg[i] + so);
-      };
-#pragma unroll
-      for (int r = 0; r < kStage; r++) {
-        if (r < NS) issue(pslot, r);
-        cp_async_commit();
-        advance(pslot);
-      }
-      cp_async_wait<kStage - 1>();
-      T prev = T(0);
-      named_bar_sync(1, NBAR);
-      for (int s0 = 0; s0 < NS; s0 += kStage) {
-#pragma unroll
-        for (int u = 0; u < kStage; u++) {
-          const int s = s0 + u;
-          if (s < NS) {
-            T v[Op::NV];
-#pragma unroll
-            for (int k = 0; k < Op::NV; k++) v[k] = my_stage[u * kStageStride + k * 32];
-            const int z = FWD ? (s - ty - lane) : (g.nz - 1 - (s - (TY - 1 - ty) - (31 - lane)));
-            const bool valid = (z >= 0) && (z < g.nz);
-            const T shv = FWD ? __shfl_up_sync(kFull, prev, 1) : __shfl_down_sync(kFull, prev, 1);
-            const bool xedge = FWD ? (lane == 0) : (lane == 31);
-            const T xn = xedge ? (hasX ? sh.bufX[s % kRing][ty] : T(0)) : shv;
-            T yn;
-            // the y neighbour across the tile edge: a cluster ring entry or the
-            // mailbox ring the loader filled
-            T yedge = T(0);
-            if (hasY) {
-              if (CLU && ydin)
-                yedge = cl_value<T>(*(volatile unsigned long long*)&ringY[s % kClRing][lane]);
-              else
-                yedge = sh.bufY[s % kRing][lane];
-            }
-            if (FWD)
-              yn = ty > 0 ? sh.xch[(s + 1) & 1][ty - 1][lane] : yedge;
-            else
-              yn = ty < TY - 1 ? sh.xch[(s + 1) & 1][ty + 1][lane] : yedge;
-            if constexpr (CLU) {
-              // before writing entry s - (TY-1) into the consumer's ring, that
-              // slot's previous entry must have been used (its step completed)
-              if (rring && s >= TY - 1 && s - (TY - 1) - kClRing >= cdone) {
-                int spins = 0;
-                for (;;) {
-                  cdone = ld_relaxed_cluster_s32(rdone);
-                  if (s - (TY - 1) - kClRing < cdone) break;
-                  if (++spins > slim) {
-                    atomicOr(&a.sc->err, DEV_ERR_TIMEOUT);
-                    break;
-                  }
-                }
-              }
-            }
-            T val = T(0);
-            if (valid) {
-              const int64_t e = rowbase + (int64_t)cslot * rstride;
-              val = op.compute(v, xn, yn, prev, e, acc);
-              if (xsrc && outx) mb_store(outx + (int64_t)(s - 31) * TY + ty, val);
-              if (ysrc) {
-                if (CLU && rring) {
-                  const int en = s - (TY - 1);
-                  st_relaxed_cluster_u64(rring + (en % kClRing) * 32 + lane, cl_word<T>(t, en, val));
-                } else if (outy) {
-                  mb_store(outy + (int64_t)(s - (TY - 1)) * 32 + lane, val);
-                }
-              }
-            }
-            sh.xch[s & 1][ty][lane] = val;
-            prev = val;
-            advance(cslot);
-            __syncwarp();
-            if (s + kStage < NS) issue(pslot, u);
-            cp_async_commit();
-            advance(pslot);
-            cp_async_wait<kStage - 1>();
-            named_bar_sync(1, NBAR);
-          }
-        }
-      }
-      cp_async_wait<0>();
-    }
-    // this tile's share of the dot product (summed later in tile order, so the
-    // result does not depend on which CTA swept which tile)
-    {
-      double v = warp_sum(acc);
-      acc = 0.0;
-      if (lane == 0) sh.ssum[warp] = v;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        double S = 0.0;
-        for (int i = 0; i < TY + 3; i++) S += sh.ssum[i];
-        a.tile_partials[tid] = S;
-      }
-    }
-    __syncthreads();
-    }  // Y < nty
-    if constexpr (CLU) cooperative_groups::this_cluster().sync();  // no ring traffic crosses cluster tiles
-  }
-  // CTA partial of the accumulated dot product, then exit accounting.  The last
-  // CTA to exit finalizes the reduction and resets the ticket counters.
-  {
-    if (threadIdx.x == 0) {
-      __threadfence();
-      int prev = atomicAdd(a.exits, 1);
-      sh.last = (prev == (int)gridDim.x - 1);
-    }
-    __syncthreads();
-    if (sh.last && warp == 0) {
-      // the tiles' shares, lane l summing tiles l, l + 32, ... in order, then a
-      // fixed shuffle tree: the same sum whichever CTA gets here
-      __threadfence();
-      double S = 0.0;
-      for (int b = lane; b < ntiles; b += 32) S += __ldcg(&a.tile_partials[b]);
-      S = warp_sum(S);
-      if (lane == 0) {
-        *a.ticket = 0;
-        *a.exits = 0;
-        if (a.fin_kind != FIN_NONE) finalize(a.fin_kind, a.sc, S, 0.0);
-        if (a.sc->err & DEV_ERR_TIMEOUT) a.sc->done = DONE_BREAKDOWN;
-        __threadfence();
-      }
-    }
-  }
-}
-
-template <class T, bool FWD, class Op>
-constexpr size_t wave_dyn_smem() {
-  return sizeof(T) * (size_t)wave_stages<T, Op::NV>() * Tiled::TY * Op::NV * 32;
-}
-template <class T, bool FWD, class Op>
-void wave_set_attr() {
-  cudaFuncSetAttribute(k_wave<T, Tiled::TY, FWD, Op>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)wave_dyn_smem<T, FWD, Op>());
-}
-// Wavefront CTAs resident per SM (shared memory and registers permitting).
-// Tiles are handed out in ticket order to running CTAs only, so a grid larger
-// than what fits at once cannot deadlock; it just queues.
-template <class T, bool FWD, class Op>
-int wave_occupancy() {
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_wave<T, Tiled::TY, FWD, Op>, (Tiled::TY + 3) * 32,
-                                                    wave_dyn_smem<T, FWD, Op>()) != cudaSuccess)
-    nb = 1;
-  return std::max(1, nb);
-}
-template <class T, bool FWD, class Op>
-void launch_wave(const WaveArgs& a, const Op& op, cudaStream_t st, int grid) {
-  k_wave<T, Tiled::TY, FWD, Op><<<grid, (Tiled::TY + 3) * 32, wave_dyn_smem<T, FWD, Op>(), st>>>(a, op);
-}
-
-// Cluster launches of the FP32 sweeps (CL CTAs per cluster along y).
-template <int CL>
-cudaLaunchAttribute cluster_attr() {
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = CL;
-  at.val.clusterDim.y = 1;
-  at.val.clusterDim.z = 1;
-  return at;
-}
-template <class T, bool FWD, class Op, int CL>
-void wave_set_attr_cl() {
-  cudaFuncSetAttribute(k_wave<T, Tiled::TY, FWD, Op, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)wave_dyn_smem<T, FWD, Op>());
-  if (CL > 8) cudaFuncSetAttribute(k_wave<T, Tiled::TY, FWD, Op, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-}
-// Clusters of the sweep that fit on the GPU at once (0: cannot launch).
-template <class T, bool FWD, class Op, int CL>
-int wave_max_clusters() {
-  wave_set_attr_cl<T, FWD, Op, CL>();
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(CL * 64);
-  cfg.blockDim = dim3((Tiled::TY + 3) * 32);
-  cfg.dynamicSmemBytes = wave_dyn_smem<T, FWD, Op>();
-  cudaLaunchAttribute at = cluster_attr<CL>();
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_wave<T, Tiled::TY, FWD, Op, CL>, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return n;
-}
-template <class T, bool FWD, class Op, int CL>
-void launch_wave_cl(const WaveArgs& a, const Op& op, cudaStream_t st, int nclusters) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(nclusters * CL);
-  cfg.blockDim = dim3((Tiled::TY + 3) * 32);
-  cfg.dynamicSmemBytes = wave_dyn_smem<T, FWD, Op>();
-  cfg.stream = st;
-  cudaLaunchAttribute at = cluster_attr<CL>();
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, k_wave<T, Tiled::TY, FWD, Op, CL>, a, op);
-}
-// The FP32 sweep kinds (all of them take the cluster path together).
-template <int CL>
-int fp32_max_clusters() {
-  return std::min({wave_max_clusters<float, true, FwdOp<float>, CL>(),
-                   wave_max_clusters<float, false, BwdOp<float>, CL>(),
-                   wave_max_clusters<float, true, FwdOp<float, true>, CL>(),
-                   wave_max_clusters<float, false, BwdEisenstatOp<float>, CL>(),
-                   wave_max_clusters<float, true, FwdEisenstatOp<float>, CL>()});
-}
-
-// Fill the mailboxes with the sentinel (at allocation and after an error).
-template <class T>
-__global__ void k_mb_reset(int64_t n, T* mb) {
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride)
-    mb_reset(mb + e);
-}
-
-// Per tile: 1 when any of its cells is active (one block per tile).
-__global__ void __launch_bounds__(kThreads) k_tile_activity(Tiled g, const uint8_t* __restrict__ act,
-                                                            uint8_t* __restrict__ tile_act) {
-  // tile_elems = 256 nz bytes, and each tile starts 256-byte aligned
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(act + (int64_t)blockIdx.x * g.tile_elems);
-  const int64_t nw = g.tile_elems / 4;
-  int any = 0;
-  for (int64_t i = threadIdx.x; i < nw; i += blockDim.x) any |= __ldg(w + i) != 0u;
-  any = __syncthreads_or(any);
-  if (threadIdx.x == 0) tile_act[blockIdx.x] = any ? 1 : 0;
-}
-
-// The sweep order of the iterations: the entries of `all` (n units in
-// dependency order, tiles when CL == 0, else cluster tiles of CL tiles along
-// y) whose unit holds an active tile, in the same order, each with the bits
-// of its swept neighbours (x: X | bits << 16), and their count in the header
-// entry dst[-1].  The dot-product shares of tiles left out are set to zero
-// (nothing writes them while their unit is left out).  One block.
-__global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int CL, const uint8_t* __restrict__ tile_act,
+// The units the iterations visit: the entries of `all` (n of them, in dependency
+// order; a unit is cx by cy tiles) that hold an active tile, in the same order, and
+// their count in the header entry dst[-1].  The dot-product shares (optional) of
+// tiles that are not swept are set to zero: nothing writes them meanwhile.  One block.
+__global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int cx, int cy,
+                                                        const uint8_t* __restrict__ tile_act,
                                                         const int2* __restrict__ all, int n, int2* __restrict__ dst,
                                                         double* __restrict__ tile_partials) {
   __shared__ int wsum[32];
   __shared__ int carry;
-  const int nyu = CL ? (nty + CL - 1) / CL : nty;
-  auto swept = [&](int X, int Yu) -> bool {
-    if (X < 0 || X >= ntx || Yu < 0 || Yu >= nyu) return false;
-    if (!CL) return tile_act[Yu * ntx + X] != 0;
-    for (int r = 0; r < CL; r++) {
-      const int Y = Yu * CL + r;
-      if (Y < nty && tile_act[Y * ntx + X]) return true;
-    }
-    return false;
-  };
   if (threadIdx.x == 0) carry = 0;
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int b0 = 0; b0 < n; b0 += blockDim.x) {
     const int i = b0 + threadIdx.x;
     bool on = false;
-    int2 e = make_int2(0, 0);
     if (i < n) {
-      const int X = all[i].x & 0xffff, Yu = all[i].y;
-      on = swept(X, Yu);
-      const int bits = (swept(X - 1, Yu) ? 1 : 0) | (swept(X + 1, Yu) ? 2 : 0) | (swept(X, Yu - 1) ? 4 : 0) |
-                       (swept(X, Yu + 1) ? 8 : 0);
-      e = make_int2(X | (bits << 16), Yu);
-      if (!on)
-        for (int r = 0; r < (CL ? CL : 1); r++) {
-          const int Y = CL ? Yu * CL + r : Yu;
-          if (Y < nty) tile_partials[Y * ntx + X] = 0.0;
+      const int2 u = all[i];
+      for (int X = u.x * cx; X < min(ntx, (u.x + 1) * cx); X++)
+        for (int Y = u.y * cy; Y < min(nty, (u.y + 1) * cy); Y++) {
+          const bool act = tile_act[Y * ntx + X] != 0;
+          on |= act;
+          if (!act && tile_partials)
+            for (int w = 0; w < kSweepWarps; w++) tile_partials[(Y * ntx + X) * kSweepWarps + w] = 0.0;
         }
     }
     const unsigned m = __ballot_sync(0xffffffffu, on);
@@ -1695,7 +874,7 @@ __global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int CL
     int before = carry;
     for (int w = 0; w < warp; w++) before += wsum[w];
     before += __popc(m & ((1u << lane) - 1u));
-    if (on) dst[before] = e;
+    if (on) dst[before] = all[i];
     __syncthreads();
     if (threadIdx.x == 0) {
       int t = 0;
@@ -1708,8 +887,7 @@ __global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int CL
 }
 
 // Writes a header entry (the count) followed by the units of an ntx x nyu
-// grid in anti-diagonal order, each with the bits of the neighbours that
-// exist, into `o` (ntx nyu + 1 entries).
+// grid in anti-diagonal order into `o` (ntx nyu + 1 entries).
 void all_units_order(int ntx, int nyu, int2* o) {
   int n = 0;
   o[n++] = make_int2(ntx * nyu, 0);
@@ -1717,14 +895,26 @@ void all_units_order(int ntx, int nyu, int2* o) {
     for (int X = 0; X < ntx; X++) {
       const int Y = d - X;
       if (Y < 0 || Y >= nyu) continue;
-      const int bits = (X > 0 ? 1 : 0) | (X < ntx - 1 ? 2 : 0) | (Y > 0 ? 4 : 0) | (Y < nyu - 1 ? 8 : 0);
-      o[n++] = make_int2(X | (bits << 16), Y);
+      o[n++] = make_int2(X, Y);
     }
 }
 std::vector<int2> all_units_order(int ntx, int nyu) {
   std::vector<int2> o((size_t)ntx * nyu + 1);
   all_units_order(ntx, nyu, o.data());
   return o;
+}
+
+// The sweeps of a solver's arrays.
+inline PivotOp pivot_op(const SysArrays<double>& A, double sigma) {
+  return {{A.adiag, A.al, A.ad, A.ab, A.z, A.q, A.Az}, nullptr, {A.fwd, A.fwd + 128, A.fwd + 256, A.fwd + 384}, sigma};
+}
+template <class T, bool SELFDOT = false>
+FwdOp<T, SELFDOT> fwd_op(const SysArrays<T>& A) {  // q = L^-1 r
+  return {{A.r}, A.fwd + 128 * kFwdFactor<T>, {A.q}};
+}
+template <class T>
+BwdOp<T> bwd_op(const SysArrays<T>& A) {  // z = L^-T q, z.r
+  return {{A.q, A.r}, A.bwd, {A.z}};
 }
 
 inline int grid_for(int64_t n, int sm) {
@@ -1748,52 +938,48 @@ cudaGraphExec_t& PcgSolver::graph_for<float>(bool eis) {
 }
 
 void PcgSolver::reset_mailboxes(bool f32) {
-  const int ntiles = g_.ntiles();
-  const int64_t nx_ = mb_stride_x_ * ntiles, ny_ = mb_stride_y_ * ntiles;
-  const int grid = grid_for(std::max(nx_, ny_), ctx_->sm_count);
+  const int64_t qx = sweep_mbx_elems(sg_) * sg_.ntiles() / 4, qy = sweep_mby_elems(sg_) * sg_.ntiles() / 4;
+  const int grid = grid_for(std::max(qx, qy), ctx_->sm_count);
   if (f32) {
-    k_mb_reset<float><<<grid, kThreads, 0, ctx_->stream>>>(nx_, mbx32_);
-    k_mb_reset<float><<<grid, kThreads, 0, ctx_->stream>>>(ny_, mby32_);
+    k_mb_reset<float><<<grid, kThreads, 0, ctx_->stream>>>(qx, mbx32_);
+    k_mb_reset<float><<<grid, kThreads, 0, ctx_->stream>>>(qy, mby32_);
   } else {
-    k_mb_reset<double><<<grid, kThreads, 0, ctx_->stream>>>(nx_, mbx64_);
-    k_mb_reset<double><<<grid, kThreads, 0, ctx_->stream>>>(ny_, mby64_);
+    k_mb_reset<double><<<grid, kThreads, 0, ctx_->stream>>>(qx, mbx64_);
+    k_mb_reset<double><<<grid, kThreads, 0, ctx_->stream>>>(qy, mby64_);
   }
 }
 
-// FP32 sweeps go through clusters when the solver set them up; everything
-// else (FP64, or no clusters) through the plain persistent grid.
-template <class T, bool FWD, class Op>
-void PcgSolver::launch_sweep(const WaveArgs& a, const Op& op, cudaStream_t st, int grid) {
-  if constexpr (sizeof(T) == 4) {
-    if (cl_size_ > 0) {
-      WaveArgs c = a;
-      c.order = a.order == ws_.order_all ? order_cl_all_ : order_cl_;
-      if (cl_size_ == 16)
-        launch_wave_cl<T, FWD, Op, 16>(c, op, st, cl_grid_);
-      else
-        launch_wave_cl<T, FWD, Op, 8>(c, op, st, cl_grid_);
-      return;
-    }
+// A sweep of this solver: plan.run<T, FWD>(op, stream).  all_tiles: every tile
+// (the pivot sweep), else those with an active cell.
+struct PcgSolver::SweepPlan {
+  SweepArgs a;
+  int clusters;
+  template <class T, bool FWD, class Op>
+  void run(const Op& op, cudaStream_t st) const {
+    launch_sweep<T, FWD>(a, op, st, clusters);
   }
-  launch_wave<T, FWD>(a, op, st, grid);
-}
-
-WaveArgs PcgSolver::wave_args(bool f32, int use_skip, int fin, bool all_tiles) const {
-  WaveArgs w{};
-  w.g = g_;
+};
+PcgSolver::SweepPlan PcgSolver::sweep(bool f32, int use_skip, int fin, bool all_tiles) const {
+  SweepPlan p{};
+  SweepArgs& w = p.a;
+  w.g = sg_;
+  w.cx = cl_x_;
+  w.cy = cl_y_;
   w.mbx = f32 ? (void*)mbx32_ : (void*)mbx64_;
   w.mby = f32 ? (void*)mby32_ : (void*)mby64_;
-  w.mb_stride_x = mb_stride_x_;
-  w.mb_stride_y = mb_stride_y_;
-  w.ticket = ws_.ticket;
-  w.exits = ws_.exits;
-  w.order = all_tiles ? ws_.order_all : ws_.order_fwd;
+  w.ticket = ticket_;
+  w.exits = ticket_ + 1;
+  w.order = all_tiles ? order_cl_all_ : order_cl_act_;
+  w.active = all_tiles ? nullptr : tile_act_;
   w.sc = sc_;
-  w.partials = partials_;
   w.tile_partials = tile_partials_;
+  w.col_sums = col_sums_;
+  w.t32_sums = t32_sums_;
+  w.t32_count = t32_count_;
   w.use_skip = use_skip;
   w.fin_kind = fin;
-  return w;
+  p.clusters = cl_grid_;
+  return p;
 }
 
 int PcgSolver::spin_limit() const { return ctx_->wait_limit > 0 ? ctx_->wait_limit : kSpinLimit; }
@@ -1803,6 +989,7 @@ int PcgSolver::recover_after_timeout() {
   reset_mailboxes(false);
   if (have_f32_) reset_mailboxes(true);
   cudaMemsetAsync(sc_, 0, sizeof(PcgScalars), st);
+  cudaMemsetAsync(t32_count_, 0, sizeof(int) * (size_t)g_.ntiles(), st);
   pivots_valid_ = false;
   cudaStreamSynchronize(st);
   return ctx_->set_error(-6, "wavefront wait timed out");
@@ -1815,108 +1002,99 @@ PcgSolver::PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt
     return;
   }
   g_ = Tiled::make(nx, ny, nz);
-  wave_set_attr<double, true, PivotOp>();
-  wave_set_attr<double, true, FwdOp<double>>();
-  wave_set_attr<double, false, BwdOp<double>>();
-  wave_set_attr<float, true, FwdOp<float>>();
-  wave_set_attr<float, false, BwdOp<float>>();
-  wave_set_attr<float, true, FwdOp<float, true>>();
-  wave_set_attr<float, false, BwdEisenstatOp<float>>();
-  wave_set_attr<float, true, FwdEisenstatOp<float>>();
+  sg_ = SweepLayout::make(nx, ny, nz);
+  sweep_set_attr<double, true, PivotOp>();
+  sweep_set_attr<double, true, FwdOp<double>>();
+  sweep_set_attr<double, false, BwdOp<double>>();
+  sweep_set_attr<float, true, FwdOp<float>>();
+  sweep_set_attr<float, false, BwdOp<float>>();
+  sweep_set_attr<float, true, FwdOp<float, true>>();
+  sweep_set_attr<float, false, BwdEisenstatOp<float>>();
+  sweep_set_attr<float, true, FwdEisenstatOp<float>>();
   nblocks_ = ctx->sm_count * 8;
-  const int ntiles = g_.ntiles();
-  wave_grid_ = std::min(ntiles, ctx->sm_count);
-  {
-    const int occ64 = std::min(wave_occupancy<double, true, FwdOp<double>>(),
-                               wave_occupancy<double, false, BwdOp<double>>());
-    const int occ32 = std::min({wave_occupancy<float, true, FwdOp<float>>(),
-                                wave_occupancy<float, false, BwdOp<float>>(),
-                                wave_occupancy<float, true, FwdEisenstatOp<float>>(),
-                                wave_occupancy<float, false, BwdEisenstatOp<float>>()});
-    wave_grid64_ = std::min(ntiles, ctx->sm_count * occ64);
-    wave_grid32_ = std::min(ntiles, ctx->sm_count * occ32);
-  }
+  const int ntiles = sg_.ntiles();
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;
     if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;
     allocs_.push_back(p);
     return p;
   };
-  const size_t n64 = sizeof(double) * (size_t)g_.total;
-  double** arr64[] = {&d64_.adiag, &d64_.al, &d64_.ad, &d64_.ab, &d64_.E, &d64_.cL,
-                      &d64_.cD,    &d64_.cB, &d64_.uR, &d64_.uU, &d64_.uF, &d64_.r,
-                      &d64_.p,     &d64_.z,  &d64_.s,  &d64_.q,  &d64_.Az, &rhs_};
-  for (double** a : arr64) {
-    *a = (double*)alloc(n64);
-    if (!*a) {
-      init_status_ = -3;
-      return;
-    }
-  }
-  active_ = (uint8_t*)alloc((size_t)g_.total);
-  partials_ = (double*)alloc(sizeof(double) * 2 *
-                             (size_t)std::max({nblocks_, wave_grid_, wave_grid64_, wave_grid32_}));
-  sc_ = (PcgScalars*)alloc(sizeof(PcgScalars));
-  ws_.ticket = (int*)alloc(sizeof(int) * 2);
-  tile_partials_ = (double*)alloc(sizeof(double) * (size_t)ntiles);
-  tile_act_ = (uint8_t*)alloc((size_t)ntiles);
-  // order lists: a header entry (the count) and up to ntiles entries
-  int2* order_all = (int2*)alloc(sizeof(int2) * (size_t)(ntiles + 1));
-  int2* order = (int2*)alloc(sizeof(int2) * (size_t)(ntiles + 1));
-  // mailboxes (FP64; the FP32 ones are allocated with the FP32 arrays)
-  const int NS = nz + 31 + Tiled::TY - 1;
-  mb_stride_x_ = (int64_t)NS * Tiled::TY;
-  mb_stride_y_ = (int64_t)NS * 32;
-  mbx64_ = (double*)alloc(sizeof(double) * (size_t)(mb_stride_x_ * ntiles));
-  mby64_ = (double*)alloc(sizeof(double) * (size_t)(mb_stride_y_ * ntiles));
-  if (!active_ || !partials_ || !sc_ || !ws_.ticket || !order || !order_all || !mbx64_ || !mby64_ ||
-      !tile_partials_ || !tile_act_) {
+  const size_t nt = sizeof(double) * (size_t)g_.total, ns = sizeof(double) * (size_t)sg_.total;
+  double** tiled[] = {&t_adiag_, &t_al_, &t_ad_, &t_ab_, &rhs_, &press_};
+  double** swept[] = {&d64_.adiag, &d64_.al, &d64_.ad, &d64_.ab, &d64_.r,
+                      &d64_.p,     &d64_.z,  &d64_.s,  &d64_.q,  &d64_.Az};
+  auto alloc_zero = [&](double** a, size_t bytes) {
+    *a = (double*)alloc(bytes);
+    if (*a) cudaMemsetAsync(*a, 0, bytes, ctx->stream);
+    return *a != nullptr;
+  };
+  bool ok = true;
+  for (double** a : tiled) ok = ok && alloc_zero(a, nt);
+  for (double** a : swept) ok = ok && alloc_zero(a, ns);
+  ok = ok && alloc_zero(&d64_.fwd, ns * kFwdStream<double>) && alloc_zero(&d64_.bwd, ns * kBwdStream);
+  if (!ok) {
     init_status_ = -3;
     return;
   }
-  ws_.exits = ws_.ticket + 1;
-  ws_.order_all = order_all + 1;
-  ws_.order_fwd = order + 1;
-  cudaMemsetAsync(ws_.ticket, 0, sizeof(int) * 2, ctx->stream);
-  for (double** a : arr64) cudaMemsetAsync(*a, 0, n64, ctx->stream);
+  active_ = (uint8_t*)alloc((size_t)g_.total);
+  partials_ = (double*)alloc(sizeof(double) * 2 * (size_t)nblocks_);
+  sc_ = (PcgScalars*)alloc(sizeof(PcgScalars));
+  ticket_ = (int*)alloc(sizeof(int) * 2);
+  tile_partials_ = (double*)alloc(sizeof(double) * (size_t)ntiles * kSweepWarps);
+  tile_act_ = (uint8_t*)alloc((size_t)ntiles);
+  // order lists: a header entry (the count) and up to ntiles entries
+  col_sums_ = (double*)alloc(sizeof(double) * (size_t)ntiles * kSweepWarps * 32);
+  t32_sums_ = (double*)alloc(sizeof(double) * (size_t)g_.ntiles());
+  t32_count_ = (int*)alloc(sizeof(int) * (size_t)g_.ntiles());
+  int2* order_all = (int2*)alloc(sizeof(int2) * (size_t)(ntiles + 1));
+  int2* order = (int2*)alloc(sizeof(int2) * (size_t)(ntiles + 1));
+  // mailboxes (FP64; the FP32 ones are allocated with the FP32 arrays)
+  mbx64_ = (double*)alloc(sizeof(double) * (size_t)(sweep_mbx_elems(sg_) * ntiles));
+  mby64_ = (double*)alloc(sizeof(double) * (size_t)(sweep_mby_elems(sg_) * ntiles));
+  if (!active_ || !partials_ || !sc_ || !ticket_ || !order || !order_all || !mbx64_ || !mby64_ ||
+      !tile_partials_ || !tile_act_ || !col_sums_ || !t32_sums_ || !t32_count_) {
+    init_status_ = -3;
+    return;
+  }
+  order_all_ = order_all + 1;
+  order_act_ = order + 1;
+  cudaMemsetAsync(ticket_, 0, sizeof(int) * 2, ctx->stream);
+  cudaMemsetAsync(t32_count_, 0, sizeof(int) * (size_t)g_.ntiles(), ctx->stream);
   cudaMemsetAsync(active_, 0, (size_t)g_.total, ctx->stream);
   cudaMemsetAsync(sc_, 0, sizeof(PcgScalars), ctx->stream);
-  cudaMemsetAsync(partials_, 0,
-                  sizeof(double) * 2 * (size_t)std::max({nblocks_, wave_grid_, wave_grid64_, wave_grid32_}),
-                  ctx->stream);
+  cudaMemsetAsync(partials_, 0, sizeof(double) * 2 * (size_t)nblocks_, ctx->stream);
   reset_mailboxes(false);
   // tile order: anti-diagonals of the tile grid, so every tile's forward
   // predecessors (X-1,Y), (X,Y-1) hold smaller tickets; reversed for backward.
   // Until the first system selects its active tiles, both lists hold all.
-  std::vector<int2> ord = all_units_order(g_.ntx, g_.nty);
+  std::vector<int2> ord = all_units_order(sg_.ntx, sg_.nty);
   cudaMemcpyAsync(order_all, ord.data(), sizeof(int2) * ord.size(), cudaMemcpyHostToDevice, ctx->stream);
   cudaMemcpyAsync(order, ord.data(), sizeof(int2) * ord.size(), cudaMemcpyHostToDevice, ctx->stream);
-  // FP32 sweeps in clusters of 16 (or 8) CTAs along y, when the tile rows fill
-  // such clusters, the GPU can run all of them at once, and the ring stamps
-  // hold the entries.  A cluster holds its CTAs until its last tile ends, so
-  // when cluster tiles have to queue for free clusters (256^3 and up) the
-  // plain persistent grid is faster: with clusters of 16 the 512^3 mixed solve
-  // measured 2.93 s against 1.80 s without, each FP32 sweep 2.3 ms.
-  if (NS < 4096) {
-    for (int CL : {16, 8}) {
-      if (g_.nty < CL) continue;
-      const int n = CL == 16 ? fp32_max_clusters<16>() : fp32_max_clusters<8>();
-      if (n < 1) continue;
-      const int nyc = (g_.nty + CL - 1) / CL;
-      if (g_.ntx * nyc > n) continue;
-      std::vector<int2> oc = all_units_order(g_.ntx, nyc);
-      int2* ca = (int2*)alloc(sizeof(int2) * oc.size());
-      int2* cc = (int2*)alloc(sizeof(int2) * oc.size());
-      if (!ca || !cc) break;
-      cudaMemcpyAsync(ca, oc.data(), sizeof(int2) * oc.size(), cudaMemcpyHostToDevice, ctx->stream);
-      cudaMemcpyAsync(cc, oc.data(), sizeof(int2) * oc.size(), cudaMemcpyHostToDevice, ctx->stream);
-      order_cl_all_ = ca + 1;
-      order_cl_ = cc + 1;
-      cl_size_ = CL;
-      cl_grid_ = std::min(n, g_.ntx * nyc);
-      break;
-    }
+  choose_clusters();
+  const int ncx = (sg_.ntx + cl_x_ - 1) / cl_x_, ncy = (sg_.nty + cl_y_ - 1) / cl_y_;
+  std::vector<int2> oc = all_units_order(ncx, ncy);
+  int2* ca = (int2*)alloc(sizeof(int2) * oc.size());
+  int2* cc = (int2*)alloc(sizeof(int2) * oc.size());
+  if (!ca || !cc) {
+    init_status_ = -3;
+    return;
   }
+  cudaMemcpyAsync(ca, oc.data(), sizeof(int2) * oc.size(), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(cc, oc.data(), sizeof(int2) * oc.size(), cudaMemcpyHostToDevice, ctx->stream);
+  order_cl_all_ = ca + 1;
+  order_cl_act_ = cc + 1;
+  // and the Tiled tiles (two sweep tiles along x), for the SpMV
+  std::vector<int2> ot = all_units_order(g_.ntx, g_.nty);
+  int2* ta = (int2*)alloc(sizeof(int2) * ot.size());
+  int2* tc = (int2*)alloc(sizeof(int2) * ot.size());
+  if (!ta || !tc) {
+    init_status_ = -3;
+    return;
+  }
+  cudaMemcpyAsync(ta, ot.data(), sizeof(int2) * ot.size(), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(tc, ot.data(), sizeof(int2) * ot.size(), cudaMemcpyHostToDevice, ctx->stream);
+  order_t32_all_ = ta + 1;
+  order_t32_act_ = tc + 1;
   if (cudaMallocHost(&sc_host_, sizeof(PcgScalars) * 2) != cudaSuccess) {
     init_status_ = -3;
     return;
@@ -1926,6 +1104,44 @@ PcgSolver::PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt
   cudaEventCreate(&evt0_);
   cudaEventCreate(&evt1_);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) init_status_ = -2;
+}
+
+// The sweeps' cluster shape.  Inside a cluster boundary values go straight into the
+// next block's shared memory, ~0.4 us sooner than through a mailbox.  Where the
+// clusters' blocks are no more than the SMs: the shape that leaves the fewest hand-offs
+// between clusters (128^3: 2 x 4 clusters of 4 x 4 tiles, FP32 forward sweep 69 us
+// against 78 without clusters).  Where tiles have to queue, a cluster holds its SMs
+// until its last block is through, and pairs along y are the best of both (256^3
+// mixed solve: 127 ms without, 122 with pairs, 130 with 4, 143 with 16).
+void PcgSolver::choose_clusters() {
+  auto shape = [&](int size, int& cx, int& cy) {  // fewest hand-offs for this size; false if the grid is smaller
+    int best = 1 << 30;
+    for (int x = 1; x <= size; x *= 2) {
+      const int y = size / x;
+      if ((x > 1 && x / 2 >= sg_.ntx) || (y > 1 && y / 2 >= sg_.nty)) continue;
+      const int n = (sg_.ntx + x - 1) / x + (sg_.nty + y - 1) / y;
+      if (n >= best) continue;
+      best = n;
+      cx = x;
+      cy = y;
+    }
+    return best < (1 << 30);
+  };
+  int best = 1 << 30;
+  for (int size : {1, 2, 4, 8, 16}) {
+    int cx, cy;
+    if (!shape(size, cx, cy)) continue;
+    const int nx = (sg_.ntx + cx - 1) / cx, ny = (sg_.nty + cy - 1) / cy;
+    if (nx + ny >= best || (size > 2 && nx * ny * size > ctx_->sm_count)) continue;
+    // 16 is beyond the portable size: where the GPU grants it
+    if (size > 8 && (sweep_max_clusters<double, true, PivotOp>(size) < 1 ||
+                     sweep_max_clusters<float, true, FwdEisenstatOp<float>>(size) < 1))
+      continue;
+    best = nx + ny;
+    cl_x_ = cx;
+    cl_y_ = cy;
+    cl_grid_ = std::min(nx * ny, ctx_->sm_count / size);
+  }
 }
 
 PcgSolver::~PcgSolver() {
@@ -1975,7 +1191,7 @@ int PcgSolver::upload(const double* adiag, const double* const an[6], const doub
   const int64_t N = (int64_t)g_.nx * g_.ny * g_.nz;
   const int grid = grid_for(g_.total, ctx_->sm_count);
   const double* src[5] = {adiag, an[0], an[3], an[5], rhs};
-  double* dst[5] = {d64_.adiag, d64_.al, d64_.ad, d64_.ab, rhs_};
+  double* dst[5] = {t_adiag_, t_al_, t_ad_, t_ab_, rhs_};
   // staging buffers for host input (one array at a time)
   double* stage = nullptr;
   uint8_t* stage_act = nullptr;
@@ -2054,7 +1270,7 @@ int PcgSolver::download_pressure(double* pg, bool device) {
   cudaStream_t st = ctx_->stream;
   const int64_t N = (int64_t)g_.nx * g_.ny * g_.nz;
   const int grid = grid_for(g_.total, ctx_->sm_count);
-  const double* src = d64_.p;  // the mixed solve copies its FP64 accumulator here
+  const double* src = press_;
   if (device) {
     k_from_tiled<double, double><<<grid, kThreads, 0, st>>>(g_, src, pg);
     launches_ += 1;
@@ -2072,23 +1288,19 @@ int PcgSolver::download_pressure(double* pg, bool device) {
 int PcgSolver::ensure_pivots() {
   if (pivots_valid_) return 0;
   cudaStream_t st = ctx_->stream;
-  const int grid = grid_for(g_.total, ctx_->sm_count);
-  WaveArgs wa = wave_args(false, 0, FIN_NONE, true);
+  const int grid = grid_for(g_.total, ctx_->sm_count), sgrid = grid_for(sg_.total / 4, ctx_->sm_count);
   // the pivot sweep reports a timeout through the status word: start it clean,
   // with this context's wait bound
   cudaMemsetAsync(&sc_->err, 0, sizeof(unsigned), st);
   pivot_limit_ = spin_limit();
   cudaMemcpyAsync(&sc_->spin_limit, &pivot_limit_, sizeof(int), cudaMemcpyHostToDevice, st);
-  k_mask_system<<<grid, kThreads, 0, st>>>(g_, active_, d64_.adiag, d64_.al, d64_.ad, d64_.ab);
-  // uR/uU/uF hold the pivot's diagonal products until k_upper overwrites them
-  // q holds Adiag masked by the active flag until the forward sweep overwrites it
-  k_pivot_diag<<<grid, kThreads, 0, st>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_,
-                                          opt_.tau, d64_.q, d64_.uR, d64_.uU, d64_.uF);
-  PivotOp op{{d64_.q, d64_.al, d64_.ad, d64_.ab, d64_.uR, d64_.uU, d64_.uF},
-             opt_.sigma, d64_.E, d64_.cL, d64_.cD, d64_.cB};
-  launch_wave<double, true>(wa, op, st, wave_grid_);
-  k_upper<double><<<grid, kThreads, 0, st>>>(g_, d64_.cL, d64_.cD, d64_.cB, d64_.uR, d64_.uU,
-                                              d64_.uF);
+  k_mask_system<<<grid, kThreads, 0, st>>>(g_, active_, t_adiag_, t_al_, t_ad_, t_ab_);
+  // z, q and Az hold the pivots' neighbour products until select_active_tiles clears them
+  cudaMemsetAsync(tile_act_, 0, (size_t)sg_.ntiles(), st);
+  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg_, g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, opt_.tau, d64_.adiag,
+                                             d64_.al, d64_.ad, d64_.ab, d64_.z, d64_.q, d64_.Az, tile_act_);
+  sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(d64_, opt_.sigma), st);
+  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d64_);
   launches_ += 4;
   {
     // the solve's scalars are set over the status word next: read it first
@@ -2099,27 +1311,26 @@ int PcgSolver::ensure_pivots() {
   }
   if (opt_.precision == PREC_MIXED) {
     if (!have_f32_) {
-      const size_t n32 = sizeof(float) * (size_t)g_.total;
-      float** arr32[] = {&d32_.adiag, &d32_.al, &d32_.ad, &d32_.ab, &d32_.E,    &d32_.cL,
-                         &d32_.cD,    &d32_.cB, &d32_.uR, &d32_.uU, &d32_.uF,   &d32_.r,
-                         &d32_.p,     &d32_.z,  &d32_.s,  &d32_.q,  &d32_.Az,   &d32_.Pinv,
-                         &d32_.Dt};
+      const size_t n32 = sizeof(float) * (size_t)sg_.total;
+      float** arr32[] = {&d32_.adiag, &d32_.al, &d32_.ad, &d32_.ab, &d32_.fwd, &d32_.bwd,
+                         &d32_.r,     &d32_.p,  &d32_.z,  &d32_.s,  &d32_.q,   &d32_.Az};
       for (float** a : arr32) {
         void* p = nullptr;
-        if (cudaMalloc(&p, n32) != cudaSuccess) return ctx_->set_error(-3, "FP32 allocation failed");
+        const size_t bytes = n32 * (a == &d32_.fwd ? kFwdStream<float> : a == &d32_.bwd ? kBwdStream : 1);
+        if (cudaMalloc(&p, bytes) != cudaSuccess) return ctx_->set_error(-3, "FP32 allocation failed");
         allocs_.push_back(p);
         *a = (float*)p;
-        cudaMemsetAsync(p, 0, n32, st);
+        cudaMemsetAsync(p, 0, bytes, st);
       }
       void* p = nullptr;
       if (cudaMalloc(&p, sizeof(double) * (size_t)g_.total) != cudaSuccess)
-        return ctx_->set_error(-3, "FP64 accumulator allocation failed");
+        return ctx_->set_error(-3, "FP64 residual allocation failed");
       allocs_.push_back(p);
-      xacc_ = (double*)p;
-      const int ntiles = g_.ntiles();
+      rres_ = (double*)p;
+      const int ntiles = sg_.ntiles();
       void *px = nullptr, *py = nullptr;
-      if (cudaMalloc(&px, sizeof(float) * (size_t)(mb_stride_x_ * ntiles)) != cudaSuccess ||
-          cudaMalloc(&py, sizeof(float) * (size_t)(mb_stride_y_ * ntiles)) != cudaSuccess)
+      if (cudaMalloc(&px, sizeof(float) * (size_t)(sweep_mbx_elems(sg_) * ntiles)) != cudaSuccess ||
+          cudaMalloc(&py, sizeof(float) * (size_t)(sweep_mby_elems(sg_) * ntiles)) != cudaSuccess)
         return ctx_->set_error(-3, "FP32 mailbox allocation failed");
       allocs_.push_back(px);
       allocs_.push_back(py);
@@ -2128,14 +1339,12 @@ int PcgSolver::ensure_pivots() {
       reset_mailboxes(true);
       have_f32_ = true;
     }
-    const double* s64[] = {d64_.adiag, d64_.al, d64_.ad, d64_.ab, d64_.E, d64_.cL,
-                           d64_.cD,    d64_.cB, d64_.uR, d64_.uU, d64_.uF};
-    float* d32[] = {d32_.adiag, d32_.al, d32_.ad, d32_.ab, d32_.E, d32_.cL,
-                    d32_.cD,    d32_.cB, d32_.uR, d32_.uU, d32_.uF};
-    for (int i = 0; i < 11; i++)
-      k_convert<double, float><<<grid, kThreads, 0, st>>>(g_.total, s64[i], d32[i]);
-    k_eisenstat_diag<<<grid, kThreads, 0, st>>>(g_.total, d64_.E, d64_.adiag, d32_.Pinv, d32_.Dt);
-    launches_ += 12;
+    k_sweep_factor<float><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d32_);
+    launches_ += 1;
+    if (opt_.inner_method != INNER_EISENSTAT) {
+      k_sweep_matrix32<<<sgrid, kThreads, 0, st>>>(sg_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, d32_);
+      launches_ += 1;
+    }
   }
   select_active_tiles();
   int e = check_dev_error("pivots");
@@ -2144,29 +1353,26 @@ int PcgSolver::ensure_pivots() {
   return 0;
 }
 
-// The tiles the iteration sweeps visit: those with an active cell (with
-// clusters: the cluster tiles holding one).  A tile left out is never written
-// by a sweep, so the vectors the iterations carry start at zero everywhere;
-// on a tile without an active cell they then stay zero, as a sweep over it
-// would leave them (its pivots and couplings are zero).
+// The tiles the iteration sweeps visit: those with an active cell.  A tile left
+// out is never written by a sweep, so the vectors the iterations carry start at
+// zero everywhere; on a tile without an active cell they then stay zero, as a
+// sweep over it would leave them (its pivots and couplings are zero).
 void PcgSolver::select_active_tiles() {
   cudaStream_t st = ctx_->stream;
-  const int ntiles = g_.ntiles();
-#if SC_SKIP_EMPTY_TILES
-  k_tile_activity<<<ntiles, kThreads, 0, st>>>(g_, active_, tile_act_);
-#else
+  const int ntiles = sg_.ntiles();
+#if !SC_SKIP_EMPTY_TILES
   cudaMemsetAsync(tile_act_, 1, (size_t)ntiles, st);  // every tile swept
 #endif
-  k_compact_order<<<1, 1024, 0, st>>>(g_.ntx, g_.nty, 0, tile_act_, ws_.order_all, ntiles, ws_.order_fwd,
-                                      tile_partials_);
-  launches_ += 2;
-  if (cl_size_ > 0) {
-    const int nyc = (g_.nty + cl_size_ - 1) / cl_size_;
-    k_compact_order<<<1, 1024, 0, st>>>(g_.ntx, g_.nty, cl_size_, tile_act_, order_cl_all_, g_.ntx * nyc,
-                                        order_cl_, tile_partials_);
-    launches_ += 1;
-  }
-  const size_t n64 = sizeof(double) * (size_t)g_.total, n32 = sizeof(float) * (size_t)g_.total;
+  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 1, 1, tile_act_, order_all_, ntiles, order_act_, tile_partials_);
+  const int ncx = (sg_.ntx + cl_x_ - 1) / cl_x_, ncy = (sg_.nty + cl_y_ - 1) / cl_y_;
+  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, cl_x_, cl_y_, tile_act_, order_cl_all_, ncx * ncy, order_cl_act_,
+                                      nullptr);
+  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 2, 1, tile_act_, order_t32_all_, g_.ntiles(), order_t32_act_, nullptr);
+  launches_ += 3;
+  // columns of tiles that are not swept add zeros
+  cudaMemsetAsync(col_sums_, 0, sizeof(double) * (size_t)ntiles * kSweepWarps * 32, st);
+  cudaMemsetAsync(t32_sums_, 0, sizeof(double) * (size_t)g_.ntiles(), st);
+  const size_t n64 = sizeof(double) * (size_t)sg_.total, n32 = sizeof(float) * (size_t)sg_.total;
   for (double* v : {d64_.r, d64_.p, d64_.z, d64_.s, d64_.q, d64_.Az}) cudaMemsetAsync(v, 0, n64, st);
   if (have_f32_)
     for (float* v : {d32_.r, d32_.p, d32_.z, d32_.s, d32_.q, d32_.Az}) cudaMemsetAsync(v, 0, n32, st);
@@ -2174,46 +1380,39 @@ void PcgSolver::select_active_tiles() {
 
 template <class T>
 void PcgSolver::launch_spmv(SysArrays<T>& A, cudaStream_t st, int use_skip) {
-  // slot runs per tile: about 12 work items per SM (3 resident blocks x 4),
-  // runs of at least 16 slots; whole tiles as items left a partial last wave
-  // at 512^3 (1024 tiles over 592 block slots)
+  // slot runs per tile: about 12 work items per SM (3 resident blocks x 4), runs of
+  // at least 16 slots
   const int ntiles = g_.ntiles();
   const int want = 12 * ctx_->sm_count;
-  const int chunks = std::max(1, std::min((want + ntiles - 1) / ntiles, g_.nz / 16));
-  const int grid = std::min(3 * ctx_->sm_count, ntiles * chunks);
-  k_spmv_stream<T><<<grid, kThreads, 0, st>>>(g_, ws_.order_fwd, A.adiag, A.al, A.ad, A.ab, active_, A.s, A.Az, partials_, sc_,
-                                              use_skip, chunks);
+  const int runs = std::max(1, std::min((want + ntiles - 1) / ntiles, g_.nz / 16));
+  const int grid = std::min(3 * ctx_->sm_count, ntiles * runs);
+  k_spmv<T><<<grid, kThreads, 0, st>>>(sg_, order_t32_act_, A.adiag, A.al, A.ad, A.ab, A.s, A.Az, partials_, sc_, use_skip,
+                                       runs);
 }
 
 template <class T>
 void PcgSolver::launch_iteration(SysArrays<T>& A, bool eis) {
   cudaStream_t st = ctx_->stream;
   const bool f32 = sizeof(T) == 4;
-  const int wg = sizeof(T) == 4 ? wave_grid32_ : wave_grid64_;
   if constexpr (sizeof(T) == 4) {
     if (eis) {
       // CG on L^-1 A L^-T: s = search direction, z = t = L^-T s,
       // Az = w = L^-1 A L^-T s, q = rh (split residual), p = d (FP32 correction).
       // s = rh + beta s ; t = L^-T s ; iteration count and bound
-      BwdEisenstatOp<T> bo{{A.q, A.s, A.E, A.uR, A.uU, A.uF}, A.z, A.s, T(0)};
-      launch_sweep<T, false>(wave_args(true, 1, FIN_SA), bo, st, wg);
-      FwdEisenstatOp<T> fo{{A.s, A.z, A.Pinv, A.Dt, A.cL, A.cD, A.cB, A.E}, A.Az};
-      launch_sweep<T, true>(wave_args(true, 1, FIN_SPMV), fo, st, wg);  // alpha = rho / s.w
+      sweep(true, 1, FIN_SA).template run<T, false>(
+          BwdEisenstatOp<T>{{A.q, A.s}, A.bwd, {A.z, A.s}, T(0)}, st);
+      sweep(true, 1, FIN_SPMV).template run<T, true>(
+          FwdEisenstatOp<T>{{A.s, A.z}, A.fwd, {A.Az}}, st);  // alpha = rho / s.w
       // x += alpha t ; rh -= alpha w ; beta = rho_new / rho
-      k_axpy<T><<<nblocks_, kThreads, 0, st>>>(g_, ws_.order_fwd, A.z, A.Az, A.p, A.q, partials_, sc_,
-                                               FIN_EAXPY);
+      k_axpy<T><<<nblocks_, kThreads, 0, st>>>(sg_, order_act_, A.z, A.Az, A.p, A.q, partials_, sc_, FIN_EAXPY);
       return;
     }
   }
-  WaveArgs wf = wave_args(f32, 1, FIN_NONE);
-  WaveArgs wb = wave_args(f32, 1, FIN_BWD);
   launch_spmv<T>(A, st, 1);
-  k_axpy<T><<<nblocks_, kThreads, 0, st>>>(g_, ws_.order_fwd, A.s, A.Az, A.p, A.r, partials_, sc_);
-  FwdOp<T> fo{{A.r, A.cL, A.cD, A.cB, A.E}, A.q};
-  launch_sweep<T, true>(wf, fo, st, wg);
-  BwdOp<T> bo{{A.q, A.E, A.uR, A.uU, A.uF, A.r}, A.z};
-  launch_sweep<T, false>(wb, bo, st, wg);
-  k_sa<T><<<nblocks_, kThreads, 0, st>>>(g_, ws_.order_fwd, A.z, A.s, partials_, sc_);
+  k_axpy<T><<<nblocks_, kThreads, 0, st>>>(sg_, order_act_, A.s, A.Az, A.p, A.r, partials_, sc_);
+  sweep(f32, 1, FIN_NONE).template run<T, true>(fwd_op<T>(A), st);
+  sweep(f32, 1, FIN_BWD).template run<T, false>(bwd_op<T>(A), st);
+  k_sa<T><<<nblocks_, kThreads, 0, st>>>(sg_, order_act_, A.z, A.s, partials_, sc_);
 }
 
 // A CUDA graph of `chunk` iterations, captured on first use.  The legacy
@@ -2254,26 +1453,21 @@ int PcgSolver::run_pcg(SysArrays<T>& A, double tol, int criterion, int max_iter,
   init.first = 1;
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
   // r = rhs (or the scaled FP64 residual for the mixed inner solve), p = 0
-  const double* src = scale_rhs ? d64_.r : rhs_;
+  const double* src = scale_rhs ? rres_ : rhs_;
   const double scale = scale_rhs ? 1.0 / inner_scale_ : 1.0;
-  k_init<T><<<nblocks_, kThreads, 0, s>>>(g_, src, scale, active_, A.r, A.p, partials_, sc_);
+  k_init<T><<<nblocks_, kThreads, 0, s>>>(g_, sg_, src, scale, active_, A.r, A.p, partials_, sc_);
   const bool f32 = sizeof(T) == 4;
-  const int wg = sizeof(T) == 4 ? wave_grid32_ : wave_grid64_;
   eis = eis && f32;
   if (eis) {
     // rh = L^-1 r ; s = rh ; rho = rh.rh
-    if constexpr (sizeof(T) == 4) {
-      FwdOp<T, true> fo{{A.r, A.cL, A.cD, A.cB, A.E}, A.q};
-      launch_sweep<T, true>(wave_args(true, 1, FIN_EINIT), fo, s, wg);
-    }
-    k_copy<T><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.q, A.s, sc_);
+    if constexpr (sizeof(T) == 4)
+      sweep(true, 1, FIN_EINIT).template run<T, true>(fwd_op<T, true>(A), s);
+    k_copy<T><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.q, A.s, sc_);
   } else {
     // z = M^-1 r ; s = z ; sigma = z.r
-    FwdOp<T> fo{{A.r, A.cL, A.cD, A.cB, A.E}, A.q};
-    launch_sweep<T, true>(wave_args(f32, 1, FIN_NONE), fo, s, wg);
-    BwdOp<T> bo{{A.q, A.E, A.uR, A.uU, A.uF, A.r}, A.z};
-    launch_sweep<T, false>(wave_args(f32, 1, FIN_BWD), bo, s, wg);
-    k_copy<T><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.z, A.s, sc_);
+    sweep(f32, 1, FIN_NONE).template run<T, true>(fwd_op<T>(A), s);
+    sweep(f32, 1, FIN_BWD).template run<T, false>(bwd_op<T>(A), s);
+    k_copy<T><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.z, A.s, sc_);
   }
   launches_ += eis ? 3 : 4;
   int e = check_dev_error("pcg init");
@@ -2322,7 +1516,10 @@ int PcgSolver::solve_fp64(PcgStats* st) {
   e = run_pcg<double>(d64_, opt_.tol, opt_.criterion, opt_.max_iter, false, st);
   if (e == 0 && (last_.err & DEV_ERR_NONFINITE))
     return ctx_->set_error(-8, "pcg: NaN or Inf in the system or the right-hand side");
-  return e;
+  if (e) return e;
+  k_sweep_to_tiled<double><<<grid_for(g_.total, ctx_->sm_count), kThreads, 0, ctx_->stream>>>(sg_, g_, d64_.p, press_);
+  launches_ += 1;
+  return check_dev_error("pcg");
 }
 
 // Mixed precision with reliable updates: FP32 CG on the split system
@@ -2345,9 +1542,8 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
   cudaStream_t s = ctx_->stream;
   const int grid = grid_for(g_.total, ctx_->sm_count);
   SysArrays<float>& A = d32_;
-  const int wg = wave_grid32_;
   // x = 0 ; r = b (FP64)
-  k_fill<double><<<grid, kThreads, 0, s>>>(g_.total, xacc_, 0.0);
+  k_fill<double><<<grid, kThreads, 0, s>>>(g_.total, press_, 0.0);
   PcgScalars init{};
   init.spin_limit = spin_limit();
   init.tol = 0.0;  // the FP32 recursion never stops itself
@@ -2355,8 +1551,7 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
   init.criterion = CRIT_REL_L2;
   init.done = DONE_RUNNING;
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_, sc_,
-                                               FIN_NORMS);
+  k_norms<<<nblocks_, kThreads, 0, s>>>(g_.total, rhs_, active_, rres_, partials_, sc_);
   launches_ += 2;
   cudaMemcpyAsync(sc_host_, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed init");
@@ -2370,10 +1565,9 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
   const double scale = bnorm;
   if (status == DONE_RUNNING) {
     // d = 0 ; r32 = r / scale ; rh = L^-1 r32 ; s = rh ; rho = rh.rh
-    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, d64_.r, 1.0 / scale, active_, A.r, A.p, partials_, sc_);
-    FwdOp<float, true> fo{{A.r, A.cL, A.cD, A.cB, A.E}, A.q};
-    launch_sweep<float, true>(wave_args(true, 1, FIN_EINIT), fo, s, wg);
-    k_copy<float><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.q, A.s, sc_);
+    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rres_, 1.0 / scale, active_, A.r, A.p, partials_, sc_);
+    sweep(true, 1, FIN_EINIT).run<float, true>(fwd_op<float, true>(A), s);
+    k_copy<float><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.q, A.s, sc_);
     launches_ += 3;
     e = ensure_graph<float>(A, true);
     if (e) return e;
@@ -2409,12 +1603,11 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
     // residual replacement after the chunks in flight
     if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed chunk");
     seen = launched;
-    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, A.p,
-                                                 scale, xacc_, d64_.r, partials_, sc_);
-    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, d64_.r, 1.0 / scale, active_, A.r, A.p, partials_, sc_,
+    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, t_adiag_, t_al_, t_ad_, t_ab_, active_, A.p, scale, press_,
+                                                 rres_, partials_, sc_);
+    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rres_, 1.0 / scale, active_, A.r, A.p, partials_, sc_,
                                                 FIN_NONE);
-    FwdOp<float, true> fo{{A.r, A.cL, A.cD, A.cB, A.E}, A.q};
-    launch_sweep<float, true>(wave_args(true, 0, FIN_EREPLACE), fo, s, wg);
+    sweep(true, 0, FIN_EREPLACE).run<float, true>(fwd_op<float, true>(A), s);
     launches_ += 3;
     cudaMemcpyAsync(&sc_host_[0], sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed update");
@@ -2438,7 +1631,7 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
       const unsigned keep = u.err & ~(unsigned)DEV_ERR_BREAKDOWN;
       cudaMemcpyAsync(&sc_->done, &running, sizeof(int), cudaMemcpyHostToDevice, s);
       cudaMemcpyAsync(&sc_->err, &keep, sizeof(unsigned), cudaMemcpyHostToDevice, s);
-      k_copy<float><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.q, A.s, sc_);
+      k_copy<float><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.q, A.s, sc_);
       cudaMemsetAsync(&sc_->beta, 0, sizeof(double), s);
       if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed restart");
       launches_ += 1;
@@ -2446,7 +1639,7 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
     } else if (u.done == DONE_MAXITER || launched >= max_chunks || updates >= opt_.max_outer) {
       status = DONE_MAXITER;
     } else if (grew || !(meas < meas_u)) {
-      k_copy<float><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.q, A.s, sc_);
+      k_copy<float><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.q, A.s, sc_);
       cudaMemsetAsync(&sc_->beta, 0, sizeof(double), s);
       launches_ += 1;
     }
@@ -2460,7 +1653,6 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
     st->status = status;
     st->device_flags |= flags;
   }
-  cudaMemcpyAsync(d64_.p, xacc_, sizeof(double) * (size_t)g_.total, cudaMemcpyDeviceToDevice, s);
   return check_dev_error("mixed");
 }
 
@@ -2474,7 +1666,7 @@ int PcgSolver::solve_mixed(PcgStats* st) {
   cudaStream_t s = ctx_->stream;
   const int grid = grid_for(g_.total, ctx_->sm_count);
   // x = 0, r = b
-  k_fill<double><<<grid, kThreads, 0, s>>>(g_.total, xacc_, 0.0);
+  k_fill<double><<<grid, kThreads, 0, s>>>(g_.total, press_, 0.0);
   launches_ += 2;
   PcgScalars init{};
   init.spin_limit = spin_limit();
@@ -2482,8 +1674,7 @@ int PcgSolver::solve_mixed(PcgStats* st) {
   init.max_iter = 1;
   init.criterion = CRIT_REL_L2;
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_,
-                                               sc_);
+  k_norms<<<nblocks_, kThreads, 0, s>>>(g_.total, rhs_, active_, rres_, partials_, sc_);
   cudaMemcpyAsync(sc_host_, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed init");
   if (!std::isfinite(sc_host_->rn2)) return ctx_->set_error(-8, "mixed solve: NaN or Inf in the right-hand side");
@@ -2508,9 +1699,8 @@ int PcgSolver::solve_mixed(PcgStats* st) {
     outer++;
     // x += rnorm d ; r -= rnorm A d   (FP64)
     launches_ += 1;
-    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab,
-                                                 active_, d32_.p, rnorm, xacc_, d64_.r, partials_,
-                                                 sc_);
+    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, t_adiag_, t_al_, t_ad_, t_ab_, active_, d32_.p, rnorm,
+                                                 press_, rres_, partials_, sc_);
     cudaMemcpyAsync(sc_host_, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed update");
     rnorm = sqrt(sc_host_->rn2);
@@ -2524,23 +1714,19 @@ int PcgSolver::solve_mixed(PcgStats* st) {
     st->residual = meas;
     st->status = meas < opt_.tol ? DONE_CONVERGED : DONE_MAXITER;
   }
-  // copy the FP64 solution into p64 for the consumers of pressure64()
-  cudaMemcpyAsync(d64_.p, xacc_, sizeof(double) * (size_t)g_.total, cudaMemcpyDeviceToDevice, s);
   return check_dev_error("mixed");
 }
 
 int PcgSolver::true_residual(PcgStats* st) {
   cudaStream_t s = ctx_->stream;
   launches_ += 2;
-  k_true_residual<<<nblocks_, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_,
-                                                d64_.p, rhs_, partials_, sc_);
+  k_true_residual<<<nblocks_, kThreads, 0, s>>>(g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, press_, rhs_, partials_, sc_);
   PcgScalars* h = sc_host_ + 1;
   cudaMemcpyAsync(h, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   // ||b||
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("true residual");
   const double rn = sqrt(h->rn2), rinf = h->rinf;
-  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, rhs_, 1.0, active_, d64_.Az, d64_.q, partials_,
-                                               sc_);
+  k_norms<<<nblocks_, kThreads, 0, s>>>(g_.total, rhs_, active_, nullptr, partials_, sc_);
   cudaMemcpyAsync(h, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("true residual");
   const double bn = sqrt(h->rn2);
@@ -2587,22 +1773,19 @@ int PcgSolver::solve(PcgStats* st) {
 
 int PcgSolver::precond_only(const double* r, double* z) {
   cudaStream_t s = ctx_->stream;
-  const int grid = grid_for(g_.total, ctx_->sm_count);
+  const int grid = grid_for(sg_.total / 4, ctx_->sm_count);
   int e = ensure_pivots();
   if (e) return e;
-  k_to_tiled<double, double><<<grid, kThreads, 0, s>>>(g_, r, d64_.r, nullptr);
+  k_ref_to_sweep<double><<<grid, kThreads, 0, s>>>(sg_, r, d64_.r);
   PcgScalars init{};
   init.spin_limit = spin_limit();
   init.done = DONE_RUNNING;
   init.first = 1;
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  WaveArgs wf = wave_args(false, 0, FIN_NONE);
-  WaveArgs wb = wave_args(false, 0, FIN_BWD);
-  FwdOp<double> fo{{d64_.r, d64_.cL, d64_.cD, d64_.cB, d64_.E}, d64_.q};
-  launch_wave<double, true>(wf, fo, s, wave_grid64_);
-  BwdOp<double> bo{{d64_.q, d64_.E, d64_.uR, d64_.uU, d64_.uF, d64_.r}, d64_.z};
-  launch_wave<double, false>(wb, bo, s, wave_grid64_);
-  k_from_tiled<double, double><<<grid, kThreads, 0, s>>>(g_, d64_.z, z);
+  sweep(false, 0, FIN_NONE).run<double, true>(fwd_op<double>(d64_), s);
+  sweep(false, 0, FIN_BWD).run<double, false>(
+      bwd_op<double>(d64_), s);
+  k_sweep_to_ref<double><<<grid, kThreads, 0, s>>>(sg_, d64_.z, z);
   cudaMemcpyAsync(sc_host_, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("precond");
   last_ = *sc_host_;
@@ -2613,10 +1796,7 @@ int PcgSolver::precond_only(const double* r, double* z) {
 int PcgSolver::apply_only(const double* x, double* b) {
   cudaStream_t s = ctx_->stream;
   const int grid = grid_for(g_.total, ctx_->sm_count);
-  k_to_tiled<double, double><<<grid, kThreads, 0, s>>>(g_, x, d64_.s, nullptr);
-  k_apply_checked<<<grid, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, d64_.s,
-                                            d64_.Az);
-  k_from_tiled<double, double><<<grid, kThreads, 0, s>>>(g_, d64_.Az, b);
+  k_apply_checked<<<grid, kThreads, 0, s>>>(g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, x, b);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("apply");
   return check_dev_error("apply");
 }
@@ -2637,48 +1817,43 @@ int PcgSolver::time_kernels(int reps, double* ms) {
   init.beta = 0.0;
   init.sigma = 1.0;
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_,
-                                               sc_);
+  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_, sc_);
   cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_copy<double><<<grid, kThreads, 0, s>>>(g_, ws_.order_fwd, d64_.r, d64_.s, sc_);
+  k_copy<double><<<grid, kThreads, 0, s>>>(sg_, order_act_, d64_.r, d64_.s, sc_);
   // The mixed solver iterates in FP32: time its FP32 kernels (the pivot sweep
   // is FP64 in both).
   const bool f32 = opt_.precision == PREC_MIXED && have_f32_;
   if (f32) {
-    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, rhs_, 1.0, active_, d32_.r, d32_.p, partials_, sc_);
+    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d32_.r, d32_.p, partials_, sc_);
     cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-    k_copy<float><<<grid, kThreads, 0, s>>>(g_, ws_.order_fwd, d32_.r, d32_.s, sc_);
+    k_copy<float><<<grid, kThreads, 0, s>>>(sg_, order_act_, d32_.r, d32_.s, sc_);
   }
   auto kernel = [&](auto& A, int which) {
     using T = std::remove_reference_t<decltype(*A.r)>;
-    const bool is32 = sizeof(T) == 4;
-    const int wg = is32 ? wave_grid32_ : wave_grid64_;
+    const SweepPlan plan = sweep(sizeof(T) == 4, 0, FIN_NONE);
     switch (which) {
       case 1:
-        this->template launch_sweep<T, true>(wave_args(is32, 0, FIN_NONE), FwdOp<T>{{A.r, A.cL, A.cD, A.cB, A.E}, A.q}, s, wg);
+        plan.template run<T, true>(fwd_op<T>(A), s);
         break;
       case 2:
-        this->template launch_sweep<T, false>(wave_args(is32, 0, FIN_NONE), BwdOp<T>{{A.q, A.E, A.uR, A.uU, A.uF, A.r}, A.z},
-                              s, wg);
+        plan.template run<T, false>(bwd_op<T>(A), s);
         break;
       case 3:
         launch_spmv<T>(A, s, 0);
         break;
       case 4:
-        k_axpy<T><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.s, A.Az, A.p, A.r, partials_, sc_);
+        k_axpy<T><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.s, A.Az, A.p, A.r, partials_, sc_);
         break;
       case 5:
-        k_sa<T><<<nblocks_, kThreads, 0, s>>>(g_, ws_.order_fwd, A.z, A.s, partials_, sc_);
+        k_sa<T><<<nblocks_, kThreads, 0, s>>>(sg_, order_act_, A.z, A.s, partials_, sc_);
         break;
       case 6:
         if constexpr (sizeof(T) == 4)
-          this->template launch_sweep<T, false>(wave_args(true, 0, FIN_NONE),
-                                BwdEisenstatOp<T>{{A.q, A.s, A.E, A.uR, A.uU, A.uF}, A.z, A.s, T(0)}, s, wg);
+          plan.template run<T, false>(BwdEisenstatOp<T>{{A.q, A.s}, A.bwd, {A.z, A.s}, T(0)}, s);
         break;
       case 7:
         if constexpr (sizeof(T) == 4)
-          this->template launch_sweep<T, true>(wave_args(true, 0, FIN_NONE),
-                               FwdEisenstatOp<T>{{A.s, A.z, A.Pinv, A.Dt, A.cL, A.cD, A.cB, A.E}, A.Az}, s, wg);
+          plan.template run<T, true>(FwdEisenstatOp<T>{{A.s, A.z}, A.fwd, {A.Az}}, s);
         break;
     }
   };
@@ -2690,16 +1865,11 @@ int PcgSolver::time_kernels(int reps, double* ms) {
     for (int i = 0; i < reps; i++) {
       switch (which) {
         case 0: {
-          WaveArgs wa = wave_args(false, 0, FIN_NONE, true);
-          PivotOp op{{d64_.q, d64_.al, d64_.ad, d64_.ab, d64_.uR, d64_.uU, d64_.uF},
-                     opt_.sigma, d64_.E, d64_.cL, d64_.cD, d64_.cB};
-          // the diag terms live in uR/uU/uF only until k_upper; rebuild them
-          k_pivot_diag<<<grid, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab,
-                                                 active_, opt_.tau, d64_.q, d64_.uR, d64_.uU,
-                                                 d64_.uF);
-          launch_wave<double, true>(wa, op, s, wave_grid_);
-          k_upper<double><<<grid, kThreads, 0, s>>>(g_, d64_.cL, d64_.cD, d64_.cB, d64_.uR,
-                                                    d64_.uU, d64_.uF);
+          // the neighbour products live in z, q and Az only until the sweeps use those; rebuild them
+          k_sweep_system<<<grid, kThreads, 0, s>>>(sg_, g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, opt_.tau, d64_.adiag,
+                                                   d64_.al, d64_.ad, d64_.ab, d64_.z, d64_.q, d64_.Az, nullptr);
+          sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(d64_, opt_.sigma), s);
+          k_sweep_factor<double><<<grid, kThreads, 0, s>>>(sg_, d64_.fwd, d64_.adiag, d64_);
           break;
         }
         default:
@@ -2740,7 +1910,7 @@ int PcgSolver::time_kernels(int reps, double* ms) {
 // counters) in the file-scope array below instead of allocating.  It launches
 // the same kernels as sc_pcg_precond_device.
 //
-// The array is kNoAllocBytes (about 4.4 MB) and lives on every GPU that loads
+// The array is kNoAllocBytes (about 7.6 MB) and lives on every GPU that loads
 // this library, until the process exits.  It bounds the problem size: at most
 // kNoAllocMaxTiled tiled elements (ceil(nx/32)*32 * ceil(ny/8)*8 * nz, e.g. a
 // 32^3 grid) in at most kNoAllocMaxTiles column tiles.  Every call shares the
@@ -2751,19 +1921,31 @@ namespace {
 
 constexpr int64_t kNoAllocMaxTiled = 32768;
 constexpr int kNoAllocMaxTiles = 8;
-constexpr int kNoAllocMaxNS = (int)(kNoAllocMaxTiled / (Tiled::TY * 32)) + 31 + Tiled::TY - 1;
-constexpr int kNoAllocArrays = 15;  // adiag al ad ab E cL cD cB uR uU uF r q z (spare)
+constexpr int kNoAllocTiledArrays = 4;   // adiag al ad ab
+constexpr int kNoAllocSweptArrays = 16;  // adiag al ad ab, fwd (4), bwd (4), r q z Az
 
+// chunks of a warp tile of the tallest grid of `tiles` column tiles, and the
+// largest SweepLayout among the grids accepted (the padding weighs most at 8
+// tiles of 16 cells)
+constexpr int na_chunks(int tiles) { return (int)(kNoAllocMaxTiled / (tiles * 256) + 10 + 3) / 4; }  // Tiled tiles, two sweep tiles each
+constexpr int64_t na_max_swept() {
+  int64_t m = 0;
+  for (int t = 1; t <= kNoAllocMaxTiles; t++) m = (int64_t)t * na_chunks(t) * 1024 > m ? (int64_t)t * na_chunks(t) * 1024 : m;
+  return m;
+}
 constexpr size_t na_align(size_t b) { return (b + 255) & ~(size_t)255; }
-constexpr size_t kNaArrBytes = na_align(sizeof(double) * kNoAllocMaxTiled);
+constexpr size_t kNaTiledBytes = na_align(sizeof(double) * kNoAllocMaxTiled);
+constexpr size_t kNaSweptBytes = na_align(sizeof(double) * na_max_swept());
 constexpr size_t kNaActBytes = na_align(kNoAllocMaxTiled);
-constexpr size_t kNaMbxBytes = na_align(sizeof(double) * kNoAllocMaxTiles * kNoAllocMaxNS * Tiled::TY);
-constexpr size_t kNaMbyBytes = na_align(sizeof(double) * kNoAllocMaxTiles * kNoAllocMaxNS * 32);
-constexpr size_t kNaSmallBytes =
-    na_align(sizeof(double) * kNoAllocMaxTiles + sizeof(int) * 2 + sizeof(int2) * (kNoAllocMaxTiles + 1)) +
-    na_align(sizeof(PcgScalars));
-constexpr size_t kNoAllocBytes =
-    kNaArrBytes * kNoAllocArrays + kNaActBytes + kNaMbxBytes + kNaMbyBytes + kNaSmallBytes;
+// mailboxes: 32 and 64 values per sweep tile and chunk, 512 cells per tile and chunk
+constexpr size_t kNaMbxBytes = na_align(sizeof(double) * na_max_swept() / 16);
+constexpr size_t kNaMbyBytes = na_align(sizeof(double) * na_max_swept() / 8);
+constexpr int kNaSweepTiles = 2 * kNoAllocMaxTiles;
+constexpr size_t kNaSmallBytes = na_align(sizeof(double) * kNaSweepTiles * kSweepWarps + sizeof(int) * 2 +
+                                          sizeof(int2) * (kNaSweepTiles + 1)) +
+                                 na_align(sizeof(PcgScalars));
+constexpr size_t kNoAllocBytes = kNaTiledBytes * kNoAllocTiledArrays + kNaSweptBytes * kNoAllocSweptArrays +
+                                 kNaActBytes + kNaMbxBytes + kNaMbyBytes + kNaSmallBytes;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
@@ -2800,35 +1982,38 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
         *msg = std::string("cudaGetSymbolAddress failed: ") + cudaGetErrorString(e);
         return -2;
       }
-      wave_set_attr<double, true, PivotOp>();
-      wave_set_attr<double, true, FwdOp<double>>();
-      wave_set_attr<double, false, BwdOp<double>>();
+      sweep_set_attr<double, true, PivotOp>();
+      sweep_set_attr<double, true, FwdOp<double>>();
+      sweep_set_attr<double, false, BwdOp<double>>();
       g_noalloc_base[device] = ptr;
     }
     base = (unsigned char*)g_noalloc_base[device];
   }
-  double* arr[kNoAllocArrays];
-  for (int i = 0; i < kNoAllocArrays; i++) arr[i] = (double*)(base + kNaArrBytes * i);
-  unsigned char* q = base + kNaArrBytes * kNoAllocArrays;
-  uint8_t* act = (uint8_t*)q;
-  q += kNaActBytes;
-  double* mbx = (double*)q;
-  q += kNaMbxBytes;
-  double* mby = (double*)q;
-  q += kNaMbyBytes;
+  const SweepLayout sg = SweepLayout::make(nx, ny, nz);
+  unsigned char* q = base;
+  auto take = [&q](size_t bytes) {
+    unsigned char* p = q;
+    q += bytes;
+    return p;
+  };
+  double* tl[kNoAllocTiledArrays];
+  for (double*& a : tl) a = (double*)take(kNaTiledBytes);
+  double* arr[kNoAllocSweptArrays];
+  for (double*& a : arr) a = (double*)take(kNaSweptBytes);
+  uint8_t* act = (uint8_t*)take(kNaActBytes);
+  double* mbx = (double*)take(kNaMbxBytes);
+  double* mby = (double*)take(kNaMbyBytes);
   double* tile_partials = (double*)q;
-  int* ticket = (int*)(tile_partials + kNoAllocMaxTiles);
+  int* ticket = (int*)(tile_partials + kNaSweepTiles * kSweepWarps);
   int2* order = (int2*)(ticket + 2);  // header entry, then the tiles
-  PcgScalars* scal = (PcgScalars*)(q + na_align(sizeof(double) * kNoAllocMaxTiles + sizeof(int) * 2 +
-                                                sizeof(int2) * (kNoAllocMaxTiles + 1)));
-  double *t_adiag = arr[0], *t_al = arr[1], *t_ad = arr[2], *t_ab = arr[3], *t_E = arr[4],
-         *t_cL = arr[5], *t_cD = arr[6], *t_cB = arr[7], *t_uR = arr[8], *t_uU = arr[9],
-         *t_uF = arr[10], *t_r = arr[11], *t_q = arr[12], *t_z = arr[13];
+  PcgScalars* scal = (PcgScalars*)(q + kNaSmallBytes - na_align(sizeof(PcgScalars)));
+  SysArrays<double> A;
+  A.adiag = arr[0], A.al = arr[1], A.ad = arr[2], A.ab = arr[3], A.r = arr[12], A.q = arr[13], A.z = arr[14], A.Az = arr[15];
+  A.fwd = arr[4], A.bwd = arr[8];  // four arrays each
   // The array keeps the previous call's contents: reset what must start at
   // zero (scheduling counters, scalars) and the mailbox sentinels.
-  const int ntiles = g.ntiles();
-  const int NS = g.nz + 31 + Tiled::TY - 1;
-  const int64_t sx = (int64_t)NS * Tiled::TY, sy = (int64_t)NS * 32;
+  const int ntiles = sg.ntiles();
+  const int64_t mqx = sweep_mbx_elems(sg) * ntiles / 4, mqy = sweep_mby_elems(sg) * ntiles / 4;
   // An error left pending by earlier, unrelated work is not this call's.
   cudaGetLastError();
   auto failed = [&](cudaError_t e, const char* step) {
@@ -2839,13 +2024,13 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   if (failed(cudaMemsetAsync(ticket, 0, sizeof(int) * 2, st), "clearing the tile tickets") ||
       failed(cudaMemsetAsync(scal, 0, sizeof(PcgScalars), st), "clearing the status word"))
     return -2;
-  const int rgrid = grid_for(sy * ntiles, sm_count);
-  k_mb_reset<double><<<rgrid, kThreads, 0, st>>>(sx * ntiles, mbx);
-  k_mb_reset<double><<<rgrid, kThreads, 0, st>>>(sy * ntiles, mby);
+  const int rgrid = grid_for(mqy, sm_count);
+  k_mb_reset<double><<<rgrid, kThreads, 0, st>>>(mqx, mbx);
+  k_mb_reset<double><<<rgrid, kThreads, 0, st>>>(mqy, mby);
   if (failed(cudaGetLastError(), "resetting the mailboxes")) return -2;
   // every tile is swept (the order of all tiles, its count in the header)
-  int2 ord[kNoAllocMaxTiles + 1];
-  all_units_order(g.ntx, g.nty, ord);
+  int2 ord[kNaSweepTiles + 1];
+  all_units_order(sg.ntx, sg.nty, ord);
   if (failed(cudaMemcpyAsync(order, ord, sizeof(int2) * (ntiles + 1), cudaMemcpyHostToDevice, st),
              "uploading the tile order"))
     return -2;
@@ -2854,39 +2039,37 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   // of non-finite values, as the allocating entry point does
   const int grid = grid_for(g.total, sm_count);
   k_to_tiled<uint8_t, uint8_t><<<grid, kThreads, 0, st>>>(g, active, act, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, adiag, t_adiag, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[0], t_al, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[3], t_ad, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[5], t_ab, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, r, t_r, nullptr);
-  k_mask_system<<<grid, kThreads, 0, st>>>(g, act, t_adiag, t_al, t_ad, t_ab);
-  if (failed(cudaGetLastError(), "converting the system to the tiled layout")) return -2;
+  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, adiag, tl[0], nullptr);
+  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[0], tl[1], nullptr);
+  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[3], tl[2], nullptr);
+  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[5], tl[3], nullptr);
+  k_mask_system<<<grid, kThreads, 0, st>>>(g, act, tl[0], tl[1], tl[2], tl[3]);
+  const int sgrid = grid_for(sg.total / 4, sm_count);
+  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg, g, tl[0], tl[1], tl[2], tl[3], act, tau, A.adiag, A.al, A.ad, A.ab, A.z,
+                                             A.q, A.Az, nullptr);
+  k_ref_to_sweep<double><<<sgrid, kThreads, 0, st>>>(sg, r, A.r);
+  if (failed(cudaGetLastError(), "converting the system to the solver's layouts")) return -2;
   // pivots, couplings, forward and backward sweeps
-  WaveArgs wa{};
-  wa.g = g;
+  SweepArgs wa{};
+  wa.g = sg;
+  wa.cx = wa.cy = 1;
   wa.mbx = mbx;
   wa.mby = mby;
-  wa.mb_stride_x = sx;
-  wa.mb_stride_y = sy;
   wa.ticket = ticket;
   wa.exits = ticket + 1;
   wa.order = order + 1;
+  wa.active = nullptr;
   wa.sc = scal;
-  wa.partials = tile_partials;
   wa.tile_partials = tile_partials;
+  wa.col_sums = nullptr;  // no dot product is wanted
   wa.use_skip = 0;
   wa.fin_kind = FIN_NONE;
-  const int wgrid = std::min(ntiles, sm_count);
-  k_pivot_diag<<<grid, kThreads, 0, st>>>(g, t_adiag, t_al, t_ad, t_ab, act, tau, t_q, t_uR, t_uU,
-                                          t_uF);
-  PivotOp pop{{t_q, t_al, t_ad, t_ab, t_uR, t_uU, t_uF}, sigma, t_E, t_cL, t_cD, t_cB};
-  launch_wave<double, true>(wa, pop, st, wgrid);
-  k_upper<double><<<grid, kThreads, 0, st>>>(g, t_cL, t_cD, t_cB, t_uR, t_uU, t_uF);
-  FwdOp<double> fo{{t_r, t_cL, t_cD, t_cB, t_E}, t_q};
-  launch_wave<double, true>(wa, fo, st, wgrid);
-  BwdOp<double> bo{{t_q, t_E, t_uR, t_uU, t_uF, t_r}, t_z};
-  launch_wave<double, false>(wa, bo, st, wgrid);
-  k_from_tiled<double, double><<<grid, kThreads, 0, st>>>(g, t_z, z);
+  const int wgrid = std::min(ntiles, 2 * sm_count);
+  launch_sweep<double, true>(wa, pivot_op(A, sigma), st, wgrid);
+  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg, A.fwd, A.adiag, A);
+  launch_sweep<double, true>(wa, fwd_op<double>(A), st, wgrid);
+  launch_sweep<double, false>(wa, bwd_op<double>(A), st, wgrid);
+  k_sweep_to_ref<double><<<sgrid, kThreads, 0, st>>>(sg, A.z, z);
   if (failed(cudaGetLastError(), "launching the pivot and sweep kernels")) return -2;
   unsigned err = 0;
   if (failed(cudaMemcpyAsync(&err, &scal->err, sizeof(unsigned), cudaMemcpyDeviceToHost, st),

@@ -77,44 +77,11 @@ struct PcgScalars {
   int spin_limit;  // polls before a sweep's wait gives up (0: the default bound)
 };
 
-struct PcgScalars;
-// Arguments of one wavefront sweep kernel launch.
-struct WaveArgs {
-  Tiled g;
-  void* mbx;           // x mailboxes: per consumer tile, mb_stride_x elements
-  void* mby;           // y mailboxes: per consumer tile, mb_stride_y elements
-  int64_t mb_stride_x, mb_stride_y;
-  int* ticket;
-  int* exits;
-  const int2* order;
-  PcgScalars* sc;
-  double* partials;
-  double* tile_partials;  // per tile share of the sweep's dot product
-  int use_skip;
-  int fin_kind;
-  // Nothing more: growing this parameter block past its 128 bytes measured the
-  // sweeps ~30% slower.  The wait bound travels in PcgScalars::spin_limit, a
-  // cluster launch passes its cluster-tile order through `order`, and the
-  // order's length sits in the header entry order[-1].x.
-};
-
-// Wavefront scheduling state (one per sweep kernel; reset by the kernel's last CTA).
-struct WaveSync {
-  int* ticket;        // next tile ticket
-  int* exits;         // CTAs that found no more tiles
-  // ticket -> tile for forward sweeps, entries after a header entry holding
-  // their count: every tile (pivot sweep), and the tiles with an active cell
-  int2* order_all;
-  int2* order_fwd;
-};
-
 template <class T>
-struct SysArrays {  // one precision's copy of everything the PCG touches (tiled layout)
+struct SysArrays {  // one precision's copy of everything the PCG iterates on (SweepLayout)
   T *adiag = nullptr, *al = nullptr, *ad = nullptr, *ab = nullptr;
-  T *E = nullptr, *cL = nullptr, *cD = nullptr, *cB = nullptr, *uR = nullptr, *uU = nullptr,
-    *uF = nullptr;
+  T *fwd = nullptr, *bwd = nullptr;  // the sweeps' factor streams (sc_sweep.cuh)
   T *r = nullptr, *p = nullptr, *z = nullptr, *s = nullptr, *q = nullptr, *Az = nullptr;
-  T *Pinv = nullptr, *Dt = nullptr;  // Eisenstat diagonals (FP32 copy only)
 };
 
 class PcgSolver {
@@ -141,13 +108,13 @@ class PcgSolver {
   const Tiled& geom() const { return g_; }
   uint64_t launches() const { return launches_; }
   // Direct access for in-device producers (FLIP buildSystem writes these).
-  double* adiag64() { return d64_.adiag; }
-  double* al64() { return d64_.al; }
-  double* ad64() { return d64_.ad; }
-  double* ab64() { return d64_.ab; }
+  double* adiag64() { return t_adiag_; }
+  double* al64() { return t_al_; }
+  double* ad64() { return t_ad_; }
+  double* ab64() { return t_ab_; }
   double* rhs64() { return rhs_; }
   uint8_t* active() { return active_; }
-  double* pressure64() { return d64_.p; }
+  double* pressure64() { return press_; }
   // Called after a producer wrote adiag/al/ad/ab/active/rhs in tiled layout.
   void mark_system_changed() { pivots_valid_ = false; }
   void set_options(const PcgOptions& o) { opt_ = o; }
@@ -176,17 +143,13 @@ class PcgSolver {
   int recover_after_timeout();
   int spin_limit() const;
   int pivot_limit_ = 0;  // host copy of the bound uploaded for the pivot sweep
-  // FP32 sweeps in thread-block clusters of cl_size_ CTAs along y (0: none),
-  // cl_grid_ clusters; the cluster tile order (anti-diagonals of (X, Yc))
-  int cl_size_ = 0, cl_grid_ = 0;
-  int2* order_cl_all_ = nullptr;  // every cluster tile (header + entries)
-  int2* order_cl_ = nullptr;      // the cluster tiles with an active cell
   // Per tile: any active cell (set with the pivots); the sweeps of the
-  // iterations visit only those tiles (or cluster tiles holding one).
+  // iterations visit only those tiles.
   uint8_t* tile_act_ = nullptr;
   void select_active_tiles();
-  template <class T, bool FWD, class Op>
-  void launch_sweep(const WaveArgs& a, const Op& op, cudaStream_t st, int grid);
+  void choose_clusters();
+  struct SweepPlan;  // what a sweep launch needs beside its operands
+  SweepPlan sweep(bool f32, int use_skip, int fin, bool all_tiles = false) const;
   int ensure_host_stage();
   double* hstage_ = nullptr;     // staging of the host-array entry points (N doubles)
   uint8_t* hstage_act_ = nullptr;  // and of the active flags (N bytes)
@@ -194,29 +157,37 @@ class PcgSolver {
   Context* ctx_;
   PcgOptions opt_;
   Tiled g_;
+  SweepLayout sg_;
   int init_status_ = 0;
   bool pivots_valid_ = false;
   bool have_f32_ = false;
   int nblocks_ = 0;     // elementwise grid
-  int wave_grid_ = 0;   // persistent wavefront grid (pivot sweep)
-  int wave_grid64_ = 0, wave_grid32_ = 0;  // iteration sweeps: SMs x resident CTAs, capped at the tiles
   SysArrays<double> d64_;
   SysArrays<float> d32_;
-  double* rhs_ = nullptr;   // tiled rhs (FP64)
-  double* xacc_ = nullptr;  // mixed: FP64 solution accumulator
+  // FP64, Tiled layout: the system, the solution, and the mixed solve's residual
+  double *t_adiag_ = nullptr, *t_al_ = nullptr, *t_ad_ = nullptr, *t_ab_ = nullptr, *rhs_ = nullptr;
+  double *press_ = nullptr, *rres_ = nullptr;
   uint8_t* active_ = nullptr;
   double* partials_ = nullptr;  // 2 per block
   double* tile_partials_ = nullptr;
   PcgScalars* sc_ = nullptr;
   PcgScalars* sc_host_ = nullptr;  // pinned
-  WaveSync ws_{};
-  // wavefront mailboxes (per consumer tile), FP64 and FP32
+  int* ticket_ = nullptr;  // sweep tickets and exit count (reset by each sweep's last block)
+  // tiles in the sweeps' dependency order, after a header entry holding their
+  // count: every tile (pivot sweep), and the tiles with an active cell
+  int2 *order_all_ = nullptr, *order_act_ = nullptr;
+  // the sweeps' cluster shape in tiles, clusters per launch, and the same lists of
+  // cluster tiles
+  int cl_x_ = 1, cl_y_ = 1, cl_grid_ = 1;
+  int2 *order_cl_all_ = nullptr, *order_cl_act_ = nullptr;
+  int2 *order_t32_all_ = nullptr, *order_t32_act_ = nullptr;  // of Tiled tiles
+  // the FP64 sweep's dot product: per column, per Tiled tile, warps that are done
+  double *col_sums_ = nullptr, *t32_sums_ = nullptr;
+  int* t32_count_ = nullptr;
+  // sweep mailboxes (per consumer tile), FP64 and FP32
   double *mbx64_ = nullptr, *mby64_ = nullptr;
   float *mbx32_ = nullptr, *mby32_ = nullptr;
-  int64_t mb_stride_x_ = 0, mb_stride_y_ = 0;
   void reset_mailboxes(bool f32);
-  // all_tiles: sweep every tile (the pivot sweep), else the active ones
-  WaveArgs wave_args(bool f32, int use_skip, int fin, bool all_tiles = false) const;
   std::vector<void*> allocs_;
   cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;    // chunk polling
   cudaEvent_t evt0_ = nullptr, evt1_ = nullptr;  // solve timing
