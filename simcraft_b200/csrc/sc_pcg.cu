@@ -842,14 +842,26 @@ __global__ void __launch_bounds__(kThreads)
   reduce_finalize(s2, mx, partials, sc, FIN_NORMS);
 }
 
+// SweepArgs::bits of one unit of cx by cy tiles.
+template <class Swept>
+__host__ __device__ void tile_bits(int2 u, int cx, int cy, Swept swept, uint8_t* out) {
+  for (int r = 0; r < cx * cy; r++) {
+    const int X = u.x * cx + r % cx, Y = u.y * cy + r / cx;
+    out[r] = !swept(X, Y) ? 0
+                          : kTileSwept | (swept(X - 1, Y) ? 1 : 0) | (swept(X + 1, Y) ? 2 : 0) | (swept(X, Y - 1) ? 4 : 0) |
+                                (swept(X, Y + 1) ? 8 : 0);
+  }
+}
+
 // The units the iterations visit: the entries of `all` (n of them, in dependency
 // order; a unit is cx by cy tiles) that hold an active tile, in the same order, and
-// their count in the header entry dst[-1].  The dot-product shares (optional) of
-// tiles that are not swept are set to zero: nothing writes them meanwhile.  One block.
+// their count in the header entry dst[-1].  Optional: per entry the bits of its tiles
+// (SweepArgs::bits), and zeros for the dot-product shares of tiles that are not swept
+// (nothing writes those meanwhile).  One block.
 __global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int cx, int cy,
                                                         const uint8_t* __restrict__ tile_act,
                                                         const int2* __restrict__ all, int n, int2* __restrict__ dst,
-                                                        double* __restrict__ tile_partials) {
+                                                        uint8_t* __restrict__ bits, double* __restrict__ tile_partials) {
   __shared__ int wsum[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -874,7 +886,12 @@ __global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int cx
     int before = carry;
     for (int w = 0; w < warp; w++) before += wsum[w];
     before += __popc(m & ((1u << lane) - 1u));
-    if (on) dst[before] = all[i];
+    if (on) {
+      dst[before] = all[i];
+      if (bits)
+        tile_bits(all[i], cx, cy, [&](int X, int Y) { return X >= 0 && X < ntx && Y >= 0 && Y < nty && tile_act[Y * ntx + X]; },
+                  bits + (int64_t)before * kMaxCluster);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       int t = 0;
@@ -904,6 +921,14 @@ std::vector<int2> all_units_order(int ntx, int nyu) {
   return o;
 }
 
+// SweepArgs::bits of an order list (header entry first) when every tile is swept.
+std::vector<uint8_t> all_tile_bits(const SweepLayout& g, int cx, int cy, const int2* order) {
+  std::vector<uint8_t> b((size_t)order[0].x * kMaxCluster, 0);
+  for (int i = 0; i < order[0].x; i++)
+    tile_bits(order[i + 1], cx, cy, [&](int X, int Y) { return X >= 0 && X < g.ntx && Y >= 0 && Y < g.nty; },
+              b.data() + (size_t)i * kMaxCluster);
+  return b;
+}
 // The sweeps of a solver's arrays.
 inline PivotOp pivot_op(const SysArrays<double>& A, double sigma) {
   return {{A.adiag, A.al, A.ad, A.ab, A.z, A.q, A.Az}, nullptr, {A.fwd, A.fwd + 128, A.fwd + 256, A.fwd + 384}, sigma};
@@ -970,7 +995,7 @@ PcgSolver::SweepPlan PcgSolver::sweep(bool f32, int use_skip, int fin, bool all_
   w.ticket = ticket_;
   w.exits = ticket_ + 1;
   w.order = all_tiles ? order_cl_all_ : order_cl_act_;
-  w.active = all_tiles ? nullptr : tile_act_;
+  w.bits = all_tiles ? bits_all_ : bits_act_;
   w.sc = sc_;
   w.tile_partials = tile_partials_;
   w.col_sums = col_sums_;
@@ -1083,6 +1108,15 @@ PcgSolver::PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt
   cudaMemcpyAsync(cc, oc.data(), sizeof(int2) * oc.size(), cudaMemcpyHostToDevice, ctx->stream);
   order_cl_all_ = ca + 1;
   order_cl_act_ = cc + 1;
+  const std::vector<uint8_t> bits = all_tile_bits(sg_, cl_x_, cl_y_, oc.data());
+  bits_all_ = (uint8_t*)alloc(bits.size());
+  bits_act_ = (uint8_t*)alloc(bits.size());
+  if (!bits_all_ || !bits_act_) {
+    init_status_ = -3;
+    return;
+  }
+  cudaMemcpyAsync(bits_all_, bits.data(), bits.size(), cudaMemcpyHostToDevice, ctx->stream);
+  cudaMemcpyAsync(bits_act_, bits.data(), bits.size(), cudaMemcpyHostToDevice, ctx->stream);
   // and the Tiled tiles (two sweep tiles along x), for the SpMV
   std::vector<int2> ot = all_units_order(g_.ntx, g_.nty);
   int2* ta = (int2*)alloc(sizeof(int2) * ot.size());
@@ -1363,11 +1397,13 @@ void PcgSolver::select_active_tiles() {
 #if !SC_SKIP_EMPTY_TILES
   cudaMemsetAsync(tile_act_, 1, (size_t)ntiles, st);  // every tile swept
 #endif
-  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 1, 1, tile_act_, order_all_, ntiles, order_act_, tile_partials_);
+  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 1, 1, tile_act_, order_all_, ntiles, order_act_, nullptr,
+                                      tile_partials_);
   const int ncx = (sg_.ntx + cl_x_ - 1) / cl_x_, ncy = (sg_.nty + cl_y_ - 1) / cl_y_;
   k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, cl_x_, cl_y_, tile_act_, order_cl_all_, ncx * ncy, order_cl_act_,
+                                      bits_act_, nullptr);
+  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 2, 1, tile_act_, order_t32_all_, g_.ntiles(), order_t32_act_, nullptr,
                                       nullptr);
-  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 2, 1, tile_act_, order_t32_all_, g_.ntiles(), order_t32_act_, nullptr);
   launches_ += 3;
   // columns of tiles that are not swept add zeros
   cudaMemsetAsync(col_sums_, 0, sizeof(double) * (size_t)ntiles * kSweepWarps * 32, st);
@@ -1942,7 +1978,7 @@ constexpr size_t kNaMbxBytes = na_align(sizeof(double) * na_max_swept() / 16);
 constexpr size_t kNaMbyBytes = na_align(sizeof(double) * na_max_swept() / 8);
 constexpr int kNaSweepTiles = 2 * kNoAllocMaxTiles;
 constexpr size_t kNaSmallBytes = na_align(sizeof(double) * kNaSweepTiles * kSweepWarps + sizeof(int) * 2 +
-                                          sizeof(int2) * (kNaSweepTiles + 1)) +
+                                          sizeof(int2) * (kNaSweepTiles + 1) + kNaSweepTiles * kMaxCluster) +
                                  na_align(sizeof(PcgScalars));
 constexpr size_t kNoAllocBytes = kNaTiledBytes * kNoAllocTiledArrays + kNaSweptBytes * kNoAllocSweptArrays +
                                  kNaActBytes + kNaMbxBytes + kNaMbyBytes + kNaSmallBytes;
@@ -2006,6 +2042,7 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   double* tile_partials = (double*)q;
   int* ticket = (int*)(tile_partials + kNaSweepTiles * kSweepWarps);
   int2* order = (int2*)(ticket + 2);  // header entry, then the tiles
+  uint8_t* bits = (uint8_t*)(order + kNaSweepTiles + 1);
   PcgScalars* scal = (PcgScalars*)(q + kNaSmallBytes - na_align(sizeof(PcgScalars)));
   SysArrays<double> A;
   A.adiag = arr[0], A.al = arr[1], A.ad = arr[2], A.ab = arr[3], A.r = arr[12], A.q = arr[13], A.z = arr[14], A.Az = arr[15];
@@ -2034,6 +2071,9 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   if (failed(cudaMemcpyAsync(order, ord, sizeof(int2) * (ntiles + 1), cudaMemcpyHostToDevice, st),
              "uploading the tile order"))
     return -2;
+  const std::vector<uint8_t> hbits = all_tile_bits(sg, 1, 1, ord);
+  if (failed(cudaMemcpyAsync(bits, hbits.data(), hbits.size(), cudaMemcpyHostToDevice, st), "uploading the tile bits"))
+    return -2;
   // system and right-hand side into the tiled layout, then the entries the
   // reference never reads (couplings to inactive cells, inactive rows) cleared
   // of non-finite values, as the allocating entry point does
@@ -2058,7 +2098,7 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   wa.ticket = ticket;
   wa.exits = ticket + 1;
   wa.order = order + 1;
-  wa.active = nullptr;
+  wa.bits = bits;
   wa.sc = scal;
   wa.tile_partials = tile_partials;
   wa.col_sums = nullptr;  // no dot product is wanted

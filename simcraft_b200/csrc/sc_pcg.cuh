@@ -180,6 +180,7 @@ class PcgSolver {
   // cluster tiles
   int cl_x_ = 1, cl_y_ = 1, cl_grid_ = 1;
   int2 *order_cl_all_ = nullptr, *order_cl_act_ = nullptr;
+  uint8_t *bits_all_ = nullptr, *bits_act_ = nullptr;  // SweepArgs::bits of these
   int2 *order_t32_all_ = nullptr, *order_t32_act_ = nullptr;  // of Tiled tiles
   // the FP64 sweep's dot product: per column, per Tiled tile, warps that are done
   double *col_sums_ = nullptr, *t32_sums_ = nullptr;

@@ -201,7 +201,10 @@ struct SweepArgs {
   void *mbx, *mby;        // mailboxes of each consumer tile: [nc][8 rows][4], [nc][16 columns][4]
   int *ticket, *exits;    // next ticket; blocks that found no more tiles
   const int2* order;      // cluster tiles (x, y) in dependency order, their count in order[-1].x
-  const uint8_t* active;  // per tile: swept or not (null: all are)
+  // per entry of order and rank of the cluster: kTileSwept if the rank's tile is swept,
+  // and 1, 2, 4, 8 if the tile at X - 1, X + 1, Y - 1, Y + 1 of it is.  A tile without an
+  // active cell is not: it holds zeros and has zero couplings to its neighbours.
+  const uint8_t* bits;
   PcgScalars* sc;
   double* tile_partials;  // per tile and warp: the warp's share of an FP32 sweep's dot product
   // FP64 sweeps: per column (tile, warp, lane) its share, per 32 x 8 columns their sum,
@@ -211,6 +214,8 @@ struct SweepArgs {
   int use_skip;
   int fin_kind;
 };
+constexpr int kMaxCluster = 16;  // blocks of a cluster (the stride of SweepArgs::bits)
+constexpr int kTileSwept = 16;
 inline int64_t sweep_mbx_elems(const SweepLayout& g) { return (int64_t)g.nc * SweepLayout::TY * 4; }  // per tile
 inline int64_t sweep_mby_elems(const SweepLayout& g) { return (int64_t)g.nc * SweepLayout::TX * 4; }
 
@@ -501,7 +506,10 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   constexpr int D = SM::D;
   constexpr int kLane = 16 / (int)sizeof(T);  // elements of a lane's vector
   extern __shared__ __align__(1024) unsigned char dyn[];
-  if (a.use_skip && a.sc->done != DONE_RUNNING) return;
+  // the scalars of the launch in one round trip
+  const int running = a.sc->done, spin_limit = a.sc->spin_limit, nticket = a.order[-1].x;
+  const unsigned err0 = ld_relaxed_gpu_u32(&a.sc->err);
+  if (a.use_skip && running != DONE_RUNNING) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const SweepLayout& g = a.g;
   const int NC = g.nc;
@@ -515,18 +523,19 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   for (int i = threadIdx.x; i < (SM::sums - SM::tick) / 4; i += blockDim.x) reinterpret_cast<int*>(dyn + SM::tick)[i] = 0;
   __syncthreads();
   // an earlier sweep gave up: sweep nothing
-  if (threadIdx.x == 0) s_misc[0] = (ld_relaxed_gpu_u32(&a.sc->err) & DEV_ERR_TIMEOUT) ? 1 : 0;
+  if (threadIdx.x == 0) s_misc[0] = (err0 & DEV_ERR_TIMEOUT) ? 1 : 0;
   cluster_sync();
-  const SweepWait W{a.sc, smem_u32(s_misc), a.sc->spin_limit > 0 ? a.sc->spin_limit : kSpinLimit};
+  const SweepWait W{a.sc, smem_u32(s_misc), spin_limit > 0 ? spin_limit : kSpinLimit};
   const int lim = W.limit > (1 << 28) ? (1 << 30) : 4 * W.limit;  // waits behind the mailbox loaders' own bound
-  const int nticket = a.order[-1].x;
-  // A ticket word: cluster tile x | y << 16 and the ticket's running number + 1 above;
-  // kNoTile: no more.
+  // A block's ticket word: its tile X | Y << 12 | the tile's bits << 24, and the ticket's
+  // running number + 1 above; kNoTile: no more.
   constexpr unsigned kNoTile = 0xffffffffu;
-  auto ticket_word = [&](int t) -> unsigned {
-    if (t >= nticket) return kNoTile;
-    const int2 e = a.order[FWD ? t : nticket - 1 - t];
-    return (unsigned)e.x | (unsigned)e.y << 16;
+  auto ticket_word = [&](int t) -> unsigned {  // lane r: the word of rank r
+    if (t >= nticket || lane >= nrank) return kNoTile;
+    const int at = FWD ? t : nticket - 1 - t;
+    const int2 e = a.order[at];
+    const unsigned b = a.bits[at * kMaxCluster + lane];
+    return (unsigned)(e.x * a.cx + lane % a.cx) | (unsigned)(e.y * a.cy + lane / a.cx) << 12 | b << 24;
   };
   // gives ticket n to the cluster's blocks, once all their warps have read the one
   // that held its place (one warp of the leader)
@@ -550,27 +559,20 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     bool ok = !__any_sync(kFull, W.aborted());
     while (ok && !peek(n, w)) {
       ok = __all_sync(kFull, W.more(spins, lim));
-      __nanosleep(40);
+      __nanosleep(n ? 40 : 0);
     }
     if (lane == 0) add_cluster(cluster_addr(s_acks + n % kTick * 4, leader), 1);
     return ok ? w : kNoTile;
   };
-  // This block's tile of a cluster tile: false if it is not swept.  Neighbour bits: 1, 2
-  // the tile at X - 1, X + 1 is swept, 4, 8 the one at Y - 1, Y + 1.  A tile without an
-  // active cell holds zeros and has zero couplings to its neighbours.
   struct Tile {
     int X, Y, nb;
   };
-  auto swept = [&](int X, int Y) {
-    return X >= 0 && X < g.ntx && Y >= 0 && Y < g.nty && (!a.active || a.active[Y * g.ntx + X]);
-  };
+  // this block's tile: false if it is not swept
   auto tile_of = [&](unsigned w, Tile& t) -> bool {
-    t.X = (int)(w & 0xffff) * a.cx + rkx;
-    t.Y = (int)(w >> 16) * a.cy + rky;
-    if (!swept(t.X, t.Y)) return false;
-    t.nb = (swept(t.X - 1, t.Y) ? 1 : 0) | (swept(t.X + 1, t.Y) ? 2 : 0) | (swept(t.X, t.Y - 1) ? 4 : 0) |
-           (swept(t.X, t.Y + 1) ? 8 : 0);
-    return true;
+    t.X = (int)(w & 0xfff);
+    t.Y = (int)(w >> 12 & 0xfff);
+    t.nb = (int)(w >> 24);
+    return t.nb & kTileSwept;
   };
   const int first = FWD ? 0 : kSweepWarps - 1;  // the compute warp that starts a tile's wave
   // the neighbouring blocks' tiles that are in the same cluster: producers and consumers
@@ -667,14 +669,21 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
       const int64_t c0 = (int64_t)(tid * kSweepWarps + cw) * NC;
       auto chunk_at = [&](int64_t first_chunk, int d) { return first_chunk + (FWD ? d : NC - 1 - d); };
       // the first groups, as far as they are not on their way
-      if (ahead < min(DG, NG)) {
+      const bool late = ahead < min(DG, NG);
+      if (late) {
         for (; ahead < min(DG, NG); ahead++)
-          for (int i = 0; i < 4 && 4 * ahead + i < NC; i++) {
-            const int64_t c = chunk_at(c0, 4 * ahead + i);
-            copy(c * 128 + lane * kLane, c * (Op::FS * 128) + lane * kLane, (4 * (group + ahead) + i) & (D - 1), 16);
+          for (int i = 0; i < 4; i++) {
+            const bool in = 4 * ahead + i < NC;
+            const int64_t c = chunk_at(c0, in ? 4 * ahead + i : 0);
+            copy(c * 128 + lane * kLane, c * (Op::FS * 128) + lane * kLane, (4 * (group + ahead) + i) & (D - 1), in ? 16 : 0);
+            if (n == 0) cp_async_commit();  // a group per chunk, as later
           }
-        cp_async_commit();
-        cp_async_wait<0>();
+        if (n == 0) {
+          for (int i = 4 * min(DG, NG); i < D; i++) cp_async_commit();
+        } else {
+          cp_async_commit();
+          cp_async_wait<0>();
+        }
       }
       ahead = 0;
       bool next_known = false;
@@ -766,21 +775,22 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           const int d = d0 + i;
           const bool live = kMain || d < NC;
           const int slot = (sbase + i) & (D - 1);
-          auto copy_ahead = [&] {
-            const int bytes = i < nf ? 16 : 0;
-            const int64_t o = i < nf ? kDir * i : 0;
-            copy(fv + o * 128, ff + o * (Op::FS * 128), slot, bytes);
-          };
+          const int bytes = i < nf ? 16 : 0;
+          const int64_t ahead_by = i < nf ? kDir * i : 0;
+          const int64_t av = fv + ahead_by * 128, af = ff + ahead_by * (Op::FS * 128);
           if (live) {
-            // this chunk's inputs and the neighbours' boundary values: x entry d + 2, y entry d + 1
+            // the neighbours' boundary values, x entry d + 2 and y entry d + 1, and this
+            // chunk's inputs.  (Fetching the next chunk's in the shadow of this one's
+            // shuffles instead measured 5% slower: they share the shuffles' pipe.)
             Quad<T> xq, yq, v[NV];
             const bool take_x = has_x && (kMain || d < NC - 2), take_y = has_y && (kMain || d < NC - 1);
             take(take_x, i < 2 ? rxa + (i + 2) * kSlotX : rxb + (i - 2) * kSlotX, take_y,
                  i < 3 ? rya + (i + 1) * kSlotY : ryb, xq, yq, [&] {
-                   cp_async_wait<D - 1>();  // one group is committed per chunk
+                   cp_async_wait<D - 1>();  // one group of copies is committed per chunk
 #pragma unroll
                    for (int k = 0; k < NV; k++) v[k] = chunk_load(stage + (slot * NV + k) * 128);
                  });
+
             if (!kMain && !take_x) xq = Quad<T>{};
             if (!kMain && !take_y) yq = Quad<T>{};
             const T xin[4] = {xc, xq.e[0], xq.e[1], xq.e[2]}, yin[4] = {yc, yq.e[0], yq.e[1], yq.e[2]};
@@ -800,7 +810,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
               val.e[j] = prev;
 #pragma unroll
               for (int k = 0; k < NO; k++) o[k][e] = ov[k];
-              if (j == 0) copy_ahead();
+              // into the slot this chunk's inputs came from
+              if (j == 0) copy(av, af, slot, bytes);
             }
             // hand the boundary on (entry d; x entry 0 is not needed)
             const bool ox = xlast & ((i > 0) | (d0 > 0));
@@ -811,7 +822,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 #pragma unroll
             for (int k = 0; k < NO; k++) chunk_store(op.out[k] + (ato + kDir * i * (Op::OS * 128)), o[k]);
           } else {
-            copy_ahead();
+            copy(av, af, slot, bytes);
           }
           cp_async_commit();
         }
@@ -841,7 +852,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           __threadfence();
           __syncwarp();
           const int X2 = tl.X >> 1, t32 = tl.Y * ((g.ntx + 1) >> 1) + X2;
-          const bool other = swept(tl.X ^ 1, tl.Y);
+          const bool other = nb & (tl.X & 1 ? 1 : 2);  // the other tile of the pair is swept
           int done = 0;
           if (lane == 0) done = atomicAdd(&a.t32_count[t32], 1) + 1;
           if (__shfl_sync(kFull, done, 0) == (other ? 2 : 1) * kSweepWarps) {
