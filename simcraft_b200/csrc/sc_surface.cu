@@ -10,15 +10,21 @@
 //   k_mc_count     one pass over the SDF: case mask per cube (1 byte), per-block
 //                  totals of vertices and index entries
 //   k_mc_scan      one block: exclusive scan of the block totals, grand totals
-//   k_mc_vertices  per-block scan of vertex counts; writes each creating cube's
-//                  first vertex number and its vertices and normals
-//   k_mc_indices   per-block scan of index counts; each entry is the owner
-//                  cube's first vertex number plus the edge's rank in its case
+//   k_mc_vertices  one scan per block over its cubes' vertex counts; writes each
+//                  creating cube's first vertex number, and the block's vertices
+//                  from a list in shared memory
+//   k_mc_indices   the same for the index entries, over a list of the crossing cubes;
+//                  each entry is the owner cube's first vertex number plus the edge's
+//                  rank in its case
 //
-// Blocks own contiguous runs of kChunk cubes; inside a block the cubes are
-// visited in kPer rounds of 256 consecutive cubes (z fastest, so the SDF reads
-// of a warp are contiguous).  HBM-bound: the SDF is read once (8 bytes per
-// sample), the masks three times (1 byte per cube), plus the mesh itself.
+// Blocks own contiguous runs of kChunk cubes.  A few percent of the cubes cross the
+// surface, so a thread per cube left one or two lanes of a warp in the long FP64 part
+// (192^3: vertices 403 us, indices 241 us, with 16 block scans of 256 cubes each): a
+// thread now reads the masks of 16 consecutive cubes in one load, one scan places all
+// of them, and the vertices and the crossing cubes are dense lists that all threads
+// share.  What remains is HBM and L2: the SDF once (8 bytes per sample; a lane loads
+// the four corners at its z and has the next four from its neighbour), the masks three
+// times (1 byte per cube), and the mesh itself.
 #include <string>
 
 #include "sc_surface.cuh"
@@ -31,16 +37,23 @@ constexpr int kThreads = 256;
 constexpr int kPer = 16;
 constexpr int64_t kChunk = (int64_t)kThreads * kPer;
 
-__constant__ uint64_t c_mc_cases[256] = {SC_MC_CASES_INIT};
-
-// The case table in shared memory: a warp's cubes index it divergently.
-struct SharedCases {
-  const uint64_t* t;
-  __host__ __device__ uint64_t operator()(int m) const { return t[m]; }
+// The cases and what the kernels need of each (mc::case_info), worked out by the
+// compiler: in each block of the kernels it took most of their time.
+__device__ const uint64_t d_mc_cases[256] = {SC_MC_CASES_INIT};
+struct CaseInfos {
+  uint32_t v[256];
 };
+constexpr CaseInfos make_case_infos() {
+  constexpr uint64_t cases[256] = {SC_MC_CASES_INIT};
+  CaseInfos t{};
+  for (int m = 0; m < 256; m++) t.v[m] = mc::case_info(cases[m]);
+  return t;
+}
+__device__ const CaseInfos d_mc_infos = make_case_infos();
 
-__device__ __forceinline__ void load_cases(uint64_t* s) {
-  for (int m = threadIdx.x; m < 256; m += blockDim.x) s[m] = c_mc_cases[m];
+// In shared memory: a warp's cubes index it divergently.
+__device__ __forceinline__ void load_cases(uint32_t* s) {
+  for (int m = threadIdx.x; m < 256; m += blockDim.x) s[m] = d_mc_infos.v[m];
   __syncthreads();
 }
 
@@ -98,28 +111,66 @@ Scratch carve(void* base, int64_t ncubes, int64_t nblocks) {
 }
 
 __global__ void __launch_bounds__(kThreads) k_mc_count(mc::Grid g, Scratch s) {
-  __shared__ uint64_t cases[256];
+  __shared__ uint32_t cases[256];
   __shared__ long long red[2][kThreads / 32];
   load_cases(cases);
   const int64_t nc = g.ncubes(), base = blockIdx.x * kChunk;
-  long long nv = 0, ni = 0;
-  for (int r = 0; r < kPer; r++) {
-    const int64_t c = base + (int64_t)r * kThreads + threadIdx.x;
-    if (c >= nc) break;
-    int i, j, k;
-    g.cube(c, i, j, k);
-    const int m = g.mask(i, j, k);
-    s.mask[c] = (uint8_t)m;
-    const uint64_t w = cases[m];
-    nv += mc::owned_count(w);
-    ni += SC_MC_COUNT(w);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // signs of the corners (x, y) = (i, j), (i, j + 1), (i + 1, j), (i + 1, j + 1) at z
+  // (32-bit offsets: there are fewer than 2^31 cubes, and so samples; i runs past the
+  // grid in a last block's cubes that do not exist)
+  const int sx = g.ny * g.nz;
+  auto corners = [&](int i, int j, int z) {
+    const int o = (i * g.ny + j) * g.nz + z;
+    const bool in = z >= 0 && z < g.nz, x0 = in && i >= 0 && i < g.nx, x1 = in && i + 1 < g.nx, y0 = j >= 0, y1 = j + 1 < g.ny;
+    const double a = x0 && y0 ? __ldg(g.sdf + o) : 1.0, b = x0 && y1 ? __ldg(g.sdf + o + g.nz) : 1.0,
+                 c = x1 && y0 ? __ldg(g.sdf + o + sx) : 1.0, d = x1 && y1 ? __ldg(g.sdf + o + sx + g.nz) : 1.0;
+    return (a < 0.0 ? 1 : 0) | (b < 0.0 ? 2 : 0) | (c < 0.0 ? 4 : 0) | (d < 0.0 ? 8 : 0);
+  };
+  int nv = 0, ni = 0;
+  const int64_t c0 = base + threadIdx.x;
+  int i, j, k;
+  g.cube(c0 < nc ? c0 : nc - 1, i, j, k);
+  for (int r = 0; r < kPer; r += 4) {
+    if (base + (int64_t)r * kThreads >= nc) break;  // uniform over the block
+    int lo[4], up[4];
+    bool top[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {  // four cubes' loads in flight
+      lo[u] = corners(i, j, k);
+      up[u] = lane == 31 ? corners(i, j, k + 1) : 0;
+      top[u] = k == g.nz - 1;
+      // kThreads cubes on
+      for (k += kThreads; k >= g.nz;) {
+        k -= g.nz + 1;
+        if (++j >= g.ny) {
+          j = -1;
+          i++;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      // the next lane's cube is the next one along z, except behind a row's last cube,
+      // whose upper corners lie outside the grid
+      int hi = __shfl_down_sync(0xffffffffu, lo[u], 1);
+      if (lane == 31) hi = up[u];
+      if (top[u]) hi = 0;
+      const int64_t c = c0 + (int64_t)(r + u) * kThreads;
+      if (c < nc) {
+        const int m = mc::Grid::mask_of(lo[u], hi);
+        s.mask[c] = (uint8_t)m;
+        const uint32_t w = cases[m];
+        nv += mc::info_owned(w);
+        ni += mc::info_entries(w);
+      }
+    }
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     nv += __shfl_xor_sync(0xffffffffu, nv, o);
     ni += __shfl_xor_sync(0xffffffffu, ni, o);
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) {
     red[0][warp] = ni;
     red[1][warp] = nv;
@@ -170,52 +221,99 @@ __global__ void __launch_bounds__(1024) k_mc_scan(int64_t nb, Scratch s) {
   }
 }
 
-__global__ void __launch_bounds__(kThreads) k_mc_vertices(mc::Grid g, Scratch s, double* V, double* N) {
-  __shared__ uint64_t cases[256];
-  __shared__ int sh[kThreads / 32];
-  load_cases(cases);
-  const int64_t nc = g.ncubes(), base = blockIdx.x * kChunk;
-  long long next = s.bsum[blockIdx.x].y;
-  for (int r = 0; r < kPer; r++) {
-    if (base + (int64_t)r * kThreads >= nc) break;  // uniform over the block
-    const int64_t c = base + (int64_t)r * kThreads + threadIdx.x;
-    const bool in = c < nc;
-    const uint64_t w = cases[in ? s.mask[c] : 0];
-    const int cnt = mc::owned_count(w);
-    int total;
-    const int pre = block_exclusive_scan(cnt, &total, sh);
-    if (cnt) {
-      int i, j, k;
-      g.cube(c, i, j, k);
-      const long long vb = next + pre;
-      s.vbase[c] = (uint32_t)vb;
-      mc::emit_vertices(g, i, j, k, w, vb, V, N);
-    }
-    next += total;
+// The masks of a thread's kPer consecutive cubes (zero beyond the last cube).
+struct Masks {
+  uint32_t w[kPer / 4];
+  __device__ __forceinline__ int operator[](int q) const { return (int)(w[q >> 2] >> 8 * (q & 3) & 0xffu); }
+};
+__device__ __forceinline__ Masks load_masks(const uint8_t* mask, int64_t c, int64_t nc) {
+  static_assert(kPer == 16, "one 16-byte load");
+  Masks m{};
+  if (c + kPer <= nc) {
+    const uint4 v = *reinterpret_cast<const uint4*>(mask + c);
+    m.w[0] = v.x, m.w[1] = v.y, m.w[2] = v.z, m.w[3] = v.w;
+  } else {
+    for (int q = 0; q < kPer; q++)
+      if (c + q < nc) m.w[q >> 2] |= (uint32_t)mask[c + q] << 8 * (q & 3);
   }
+  return m;
 }
 
-__global__ void __launch_bounds__(kThreads) k_mc_indices(mc::Grid g, Scratch s, uint32_t* I) {
-  __shared__ uint64_t cases[256];
+__global__ void __launch_bounds__(kThreads) k_mc_vertices(mc::Grid g, Scratch s, double* V, double* N) {
+  __shared__ uint32_t cases[256];
   __shared__ int sh[kThreads / 32];
+  __shared__ uint16_t items[3 * kChunk];  // the block's vertices: cube (12 bits), owned edge (2 bits)
   load_cases(cases);
-  const int64_t nc = g.ncubes(), base = blockIdx.x * kChunk;
-  long long next = s.bsum[blockIdx.x].x;
-  bool ok = true;
-  for (int r = 0; r < kPer; r++) {
-    if (base + (int64_t)r * kThreads >= nc) break;  // uniform over the block
-    const int64_t c = base + (int64_t)r * kThreads + threadIdx.x;
-    const bool in = c < nc;
-    const uint64_t w = cases[in ? s.mask[c] : 0];
-    const int cnt = SC_MC_COUNT(w);
-    int total;
-    const int pre = block_exclusive_scan(cnt, &total, sh);
-    if (cnt) {
-      int i, j, k;
-      g.cube(c, i, j, k);
-      ok &= mc::emit_indices(g, i, j, k, w, SharedCases{cases}, s.mask, s.vbase, next + pre, I);
+  const int64_t nc = g.ncubes(), base = blockIdx.x * kChunk, c0 = base + threadIdx.x * kPer;
+  const long long next = s.bsum[blockIdx.x].y;
+  const Masks m = load_masks(s.mask, c0, nc);
+  int cnt = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++) cnt += mc::info_owned(cases[m[q]]);
+  int total;
+  int at = block_exclusive_scan(cnt, &total, sh);
+  if (cnt)
+    for (int q = 0; q < kPer; q++) {
+      const uint32_t w = cases[m[q]];
+      const int n = mc::info_owned(w);
+      if (!n) continue;
+      s.vbase[c0 + q] = (uint32_t)(next + at);
+      for (int o = 0; o < 3; o++) {
+        const int r = mc::info_rank(w, o);
+        if (r < n) items[at + r] = (uint16_t)((threadIdx.x * kPer + q) | o << 12);
+      }
+      at += n;
     }
-    next += total;
+  __syncthreads();
+  for (int v = threadIdx.x; v < total; v += kThreads) {
+    const int it = items[v];
+    int i, j, k;
+    g.cube(base + (it & 4095), i, j, k);
+    double p[3], n[3];
+    g.vertex(i, j, k, mc::owned_edge(it >> 12), p, n);
+    for (int d = 0; d < 3; d++) {
+      V[3 * (next + v) + d] = p[d];
+      N[3 * (next + v) + d] = n[d];
+    }
+  }
+}
+static_assert(kChunk == 4096, "a cube's number within its block fits 12 bits");
+
+__global__ void __launch_bounds__(kThreads) k_mc_indices(mc::Grid g, Scratch s, uint32_t* I) {
+  __shared__ uint32_t cases[256];
+  __shared__ int sh[kThreads / 32];
+  __shared__ uint16_t cube[kChunk], first[kChunk];  // the block's crossing cubes and their first entries
+  __shared__ uint64_t table[256];
+  for (int q = threadIdx.x; q < 256; q += kThreads) table[q] = d_mc_cases[q];
+  load_cases(cases);
+  const int64_t nc = g.ncubes(), base = blockIdx.x * kChunk, c0 = base + threadIdx.x * kPer;
+  const long long next = s.bsum[blockIdx.x].x;
+  const Masks m = load_masks(s.mask, c0, nc);
+  // crossing cubes (at most 4096) above, their entries (at most 15 each) below
+  int cnt = 0;
+#pragma unroll
+  for (int q = 0; q < kPer; q++) {
+    const int n = mc::info_entries(cases[m[q]]);
+    cnt += n ? (1 << 17) + n : 0;
+  }
+  int total;
+  int at = block_exclusive_scan(cnt, &total, sh);
+  if (cnt)
+    for (int q = 0; q < kPer; q++) {
+      const int n = mc::info_entries(cases[m[q]]);
+      if (!n) continue;
+      cube[at >> 17] = (uint16_t)(threadIdx.x * kPer + q);
+      first[at >> 17] = (uint16_t)(at & 0x1ffff);
+      at += (1 << 17) + n;
+    }
+  __syncthreads();
+  bool ok = true;
+  for (int a = threadIdx.x; a < total >> 17; a += kThreads) {
+    const int64_t c = base + cube[a];
+    int i, j, k;
+    g.cube(c, i, j, k);
+    ok &= mc::emit_entries(g, i, j, k, table[s.mask[c]], [&](int mk, int oe) { return mc::info_find(cases[mk], oe); },
+                           s.mask, s.vbase, next + first[a], I);
   }
   if (!ok) atomicOr(s.status, 1u);
 }

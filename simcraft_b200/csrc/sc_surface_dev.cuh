@@ -57,10 +57,12 @@ struct Grid {
     return sdf[((int64_t)x * ny + y) * nz + z];
   }
   SC_HD void cube(int64_t c, int& i, int& j, int& k) const {
-    k = (int)(c % cz()) - 1;
-    const int64_t r = c / cz();
-    j = (int)(r % cy()) - 1;
-    i = (int)(r / cy()) - 1;
+    // 32-bit divisions: there are fewer than 2^31 cubes
+    const uint32_t u = (uint32_t)c, ncz = (uint32_t)nz + 1, ncy = (uint32_t)ny + 1;
+    const uint32_t r = u / ncz, q = r / ncy;
+    k = (int)(u - r * ncz) - 1;
+    j = (int)(r - q * ncy) - 1;
+    i = (int)q - 1;
   }
   SC_HD int64_t cube_index(int i, int j, int k) const {
     return ((int64_t)(i + 1) * cy() + (j + 1)) * cz() + (k + 1);
@@ -70,6 +72,14 @@ struct Grid {
     int m = 0;
     for (int c = 0; c < 8; c++)
       if (eval(i + SC_MC_CORNER_X(c), j + SC_MC_CORNER_Y(c), k + SC_MC_CORNER_Z(c)) < 0.0) m |= 1 << c;
+    return m;
+  }
+  // The same from the signs of the four corners (x, y) = (0, 0), (0, 1), (1, 0), (1, 1) at
+  // the lower and at the upper z.
+  SC_HD static int mask_of(int lo, int hi) {
+    int m = 0;
+    for (int c = 0; c < 8; c++)
+      if (((SC_MC_CORNER_Z(c) ? hi : lo) >> (2 * SC_MC_CORNER_X(c) + SC_MC_CORNER_Y(c))) & 1) m |= 1 << c;
     return m;
   }
   // grad (rebuild-surface.cc:666-686)
@@ -113,8 +123,8 @@ struct Grid {
 };
 
 // Edges a cube owns: the three at its (1,1,1) corner.
-SC_HD bool owned(int e) { return e == 5 || e == 6 || e == 10; }
-SC_HD int owned_bit(int e) { return e == 5 ? 1 : (e == 6 ? 2 : 4); }
+SC_HD constexpr bool owned(int e) { return e == 5 || e == 6 || e == 10; }
+SC_HD constexpr int owned_bit(int e) { return e == 5 ? 1 : (e == 6 ? 2 : 4); }
 
 // The cube that owns edge e of a cube, as an offset (d[0], d[1], d[2]) from it,
 // and the owner's number for the edge.  The owner has the edge at coordinate 1
@@ -136,7 +146,7 @@ SC_HD int owner_of(int e, int d[3]) {
 }
 
 // Vertices a cube creates: its crossing edges among {5, 6, 10}.
-SC_HD int owned_count(uint64_t w) {
+SC_HD constexpr int owned_count(uint64_t w) {
   int seen = 0;
   for (int q = 0; q < SC_MC_COUNT(w); q++) {
     const int e = SC_MC_ENTRY(w, q);
@@ -147,7 +157,7 @@ SC_HD int owned_count(uint64_t w) {
 
 // Rank of owned edge oe among the cube's own vertices: how many other owned
 // edges first appear before oe in the case (-1 if the case lacks oe).
-SC_HD int owned_rank(uint64_t w, int oe) {
+SC_HD constexpr int owned_rank(uint64_t w, int oe) {
   int seen = 0;
   for (int q = 0; q < SC_MC_COUNT(w); q++) {
     const int e = SC_MC_ENTRY(w, q);
@@ -155,6 +165,23 @@ SC_HD int owned_rank(uint64_t w, int oe) {
     if (owned(e)) seen |= owned_bit(e);
   }
   return -1;
+}
+
+// A case in one word: its entry count, how many of the cube's own edges 5, 6 and 10
+// (numbered 0, 1, 2) cross, and their ranks (3: does not cross).
+SC_HD constexpr int owned_edge(int o) { return o == 0 ? 5 : (o == 1 ? 6 : 10); }
+SC_HD constexpr uint32_t case_info(uint64_t w) {
+  uint32_t v = (uint32_t)SC_MC_COUNT(w) | (uint32_t)owned_count(w) << 4;
+  for (int o = 0; o < 3; o++) v |= (uint32_t)(owned_rank(w, owned_edge(o)) & 3) << (6 + 2 * o);
+  return v;
+}
+SC_HD int info_entries(uint32_t v) { return (int)(v & 15u); }
+SC_HD int info_owned(uint32_t v) { return (int)(v >> 4 & 3u); }
+SC_HD int info_rank(uint32_t v, int o) { return (int)(v >> (6 + 2 * o) & 3u); }
+// owned_rank of edge e from the word: -1 if it does not cross
+SC_HD int info_find(uint32_t v, int e) {
+  const int r = info_rank(v, e == 5 ? 0 : (e == 6 ? 1 : 2));
+  return r == 3 ? -1 : r;
 }
 
 // Writes the vertices and normals cube (i, j, k) with case word w creates,
@@ -182,9 +209,10 @@ SC_HD void emit_vertices(const Grid& g, int i, int j, int k, uint64_t w, int64_t
 // first vertex number) plus the edge's rank in the owner's case.  An owner
 // outside the cube range or a case without the edge (neither happens for a
 // sign-change edge) writes 0xffffffff and returns false.
-template <class Cases>
-SC_HD bool emit_indices(const Grid& g, int i, int j, int k, uint64_t w, const Cases& cases,
-                        const uint8_t* mask, const uint32_t* vbase, int64_t ibase, uint32_t* I) {
+// rank(m, e) is owned_rank of edge e in case m.
+template <class Rank>
+SC_HD bool emit_entries(const Grid& g, int i, int j, int k, uint64_t w, const Rank& rank, const uint8_t* mask,
+                        const uint32_t* vbase, int64_t ibase, uint32_t* I) {
   bool ok = true;
   for (int q = 0; q < SC_MC_COUNT(w); q++) {
     const int e = SC_MC_ENTRY(w, q);
@@ -194,13 +222,19 @@ SC_HD bool emit_indices(const Grid& g, int i, int j, int k, uint64_t w, const Ca
     uint32_t vid = 0xffffffffu;
     if (oi >= -1 && oj >= -1 && ok_ >= -1) {
       const int64_t oc = g.cube_index(oi, oj, ok_);
-      const int r = owned_rank(cases(mask[oc]), oe);
+      const int r = rank(mask[oc], oe);
       if (r >= 0) vid = vbase[oc] + (uint32_t)r;
     }
     if (vid == 0xffffffffu) ok = false;
     I[ibase + q] = vid;
   }
   return ok;
+}
+// The same with the cases themselves: cases(m) is the word of case m.
+template <class Cases>
+SC_HD bool emit_indices(const Grid& g, int i, int j, int k, uint64_t w, const Cases& cases, const uint8_t* mask,
+                        const uint32_t* vbase, int64_t ibase, uint32_t* I) {
+  return emit_entries(g, i, j, k, w, [&](int m, int e) { return owned_rank(cases(m), e); }, mask, vbase, ibase, I);
 }
 
 }  // namespace mc
