@@ -40,6 +40,12 @@ static void ctx_release(sc_context* c) {
     if (c->mesh_scratch) cudaFree(c->mesh_scratch);
     if (c->surf_scratch) cudaFree(c->surf_scratch);
     if (c->surf_stage) cudaFree(c->surf_stage);
+    if (c->c.arena.base) {
+      cudaStreamWaitEvent(c->own, c->c.arena.done, 0);
+      cudaFreeAsync(c->c.arena.base, c->own);
+      cudaStreamSynchronize(c->own);
+    }
+    if (c->c.arena.done) cudaEventDestroy(c->c.arena.done);
     if (c->own) cudaStreamDestroy(c->own);
     delete c;
   }
@@ -140,6 +146,10 @@ int sc_context_create(int device, sc_context** out) {
     return SC_ERR_CUDA;
   }
   c->c.stream = c->own;
+  if (cudaEventCreateWithFlags(&c->c.arena.done, cudaEventDisableTiming) != cudaSuccess) {
+    cudaGetLastError();  // the stage functions allocate per call
+    c->c.arena.done = nullptr;
+  }
   *out = c;
   return SC_OK;
 }
@@ -429,7 +439,7 @@ int sc_flip_p2g_device(sc_context* ctx, int64_t n, const double* pos, const doub
     return SC_ERR_INVALID;
   cudaSetDevice(ctx->c.device);
   return finish(ctx,
-                sc::flip_p2g(ctx->c.stream, n, pos, vel, nx, ny, nz, h, u, v, w, u_wt, v_wt, w_wt,
+                sc::flip_p2g(ctx->c, n, pos, vel, nx, ny, nz, h, u, v, w, u_wt, v_wt, w_wt,
                              u_valid, v_valid, w_valid, u_last, v_last, w_last),
                 "p2g");
 }
@@ -441,7 +451,7 @@ int sc_sample_velocity_device(sc_context* ctx, int64_t n, const double* pts, int
     return SC_ERR_INVALID;
   if (n == 0) return SC_OK;
   cudaSetDevice(ctx->c.device);
-  return finish(ctx, sc::flip_sample(ctx->c.stream, n, pts, nx, ny, nz, h, u, v, w, out),
+  return finish(ctx, sc::flip_sample(ctx->c, n, pts, nx, ny, nz, h, u, v, w, out),
                 "sample_velocity");
 }
 
@@ -455,7 +465,7 @@ int sc_flip_g2p_device(sc_context* ctx, int64_t n, const double* pos, double* ve
   if (n == 0) return SC_OK;
   cudaSetDevice(ctx->c.device);
   return finish(ctx,
-                sc::flip_g2p(ctx->c.stream, n, pos, vel, nx, ny, nz, h, u, v, w, u_last, v_last,
+                sc::flip_g2p(ctx->c, n, pos, vel, nx, ny, nz, h, u, v, w, u_last, v_last,
                              w_last, alpha),
                 "g2p");
 }
@@ -469,7 +479,7 @@ int sc_flip_advect_device(sc_context* ctx, int64_t n, double* pos, double* vel, 
   if (n == 0) return SC_OK;
   cudaSetDevice(ctx->c.device);
   return finish(ctx,
-                sc::flip_advect(ctx->c.stream, n, pos, vel, nx, ny, nz, h, u, v, w, collider_sdf,
+                sc::flip_advect(ctx->c, n, pos, vel, nx, ny, nz, h, u, v, w, collider_sdf,
                                 dt),
                 "advect");
 }
@@ -480,7 +490,7 @@ int sc_reconstruct_device(sc_context* ctx, int64_t n, const double* pos, int nx,
       !valid)
     return SC_ERR_INVALID;
   cudaSetDevice(ctx->c.device);
-  return finish(ctx, sc::flip_reconstruct(ctx->c.stream, n, pos, nx, ny, nz, h, radius, sdf, valid),
+  return finish(ctx, sc::flip_reconstruct(ctx->c, n, pos, nx, ny, nz, h, radius, sdf, valid),
                 "reconstruct");
 }
 

@@ -479,25 +479,23 @@ namespace {
 struct StageParticles {
   double* buf = nullptr;  // 6 SoA arrays
   int64_t* id = nullptr;
-  cudaStream_t st;
-  int64_t n;
+  int64_t n = 0;
   PartsT<double> P() const {
     return {buf, buf + n, buf + 2 * n, buf + 3 * n, buf + 4 * n, buf + 5 * n};
   }
-  ~StageParticles() {
-    if (buf) cudaFreeAsync(buf, st);
-    if (id) cudaFreeAsync(id, st);
-  }
 };
+size_t soa_bytes(int64_t n) { return sizeof(double) * 6 * (size_t)std::max<int64_t>(n, 1); }
 }  // namespace
 
-int flip_sample(cudaStream_t st, int64_t n, const double* pts, int nx, int ny, int nz, double h,
+int flip_sample(const Context& ctx, int64_t n, const double* pts, int nx, int ny, int nz, double h,
                 const double* u, const double* v, const double* w, double* out) {
+  cudaStream_t st = ctx.stream;
   // out = (sampleVelocity(p)) via the G2P kernel in PIC mode on a copy
+  ScratchLease lease(ctx, ScratchLease::padded(soa_bytes(n)), st);
+  if (!lease.ok()) return -3;
   StageParticles sp;
-  sp.st = st;
   sp.n = n;
-  if (cudaMallocAsync(&sp.buf, sizeof(double) * 6 * (size_t)std::max<int64_t>(n, 1), st) != cudaSuccess) return -3;
+  lease.take(&sp.buf, soa_bytes(n));
   k_aos_to_soa<double><<<nblk(n), kT, 0, st>>>(n, pts, nullptr, sp.P(), nullptr);
   k_g2p<double><<<nblk(n), kT, 0, st>>>(n, sp.P(), u, v, w, nullptr, nullptr, nullptr, Geo{nx, ny, nz}, h,
                                         -1.0);
@@ -505,13 +503,15 @@ int flip_sample(cudaStream_t st, int64_t n, const double* pts, int nx, int ny, i
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int flip_advect(cudaStream_t st, int64_t n, double* pos, double* vel, int nx, int ny, int nz,
+int flip_advect(const Context& ctx, int64_t n, double* pos, double* vel, int nx, int ny, int nz,
                 double h, const double* u, const double* v, const double* w,
                 const double* collider, double dt) {
+  cudaStream_t st = ctx.stream;
+  ScratchLease lease(ctx, ScratchLease::padded(soa_bytes(n)), st);
+  if (!lease.ok()) return -3;
   StageParticles sp;
-  sp.st = st;
   sp.n = n;
-  if (cudaMallocAsync(&sp.buf, sizeof(double) * 6 * (size_t)std::max<int64_t>(n, 1), st) != cudaSuccess) return -3;
+  lease.take(&sp.buf, soa_bytes(n));
   k_aos_to_soa<double><<<nblk(n), kT, 0, st>>>(n, pos, vel, sp.P(), nullptr);
   k_advect<double><<<nblk(n), kT, 0, st>>>(n, sp.P(), u, v, w, Geo{nx, ny, nz}, h, collider, dt);
   k_soa_to_aos<double><<<nblk(n), kT, 0, st>>>(n, sp.P(), nullptr, pos, vel);
@@ -523,29 +523,30 @@ namespace {
 struct Sorted {
   StageParticles a, b;
   int *key = nullptr, *cnt = nullptr, *start = nullptr, *cursor = nullptr, *bsum = nullptr;
-  cudaStream_t st;
-  ~Sorted() {
-    for (int* p : {key, cnt, start, cursor, bsum})
-      if (p) cudaFreeAsync(p, st);
+  static size_t id_bytes(int64_t n) { return sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1); }
+  static size_t key_bytes(int64_t n) { return sizeof(int) * (size_t)std::max<int64_t>(n, 1); }
+  static size_t cell_bytes(const Geo& G) { return sizeof(int) * (size_t)G.nx * G.ny * G.nz; }
+  static size_t sum_bytes(const Geo& G) { return sizeof(int) * (((size_t)G.nx * G.ny * G.nz + 1023) / 1024 + 1); }
+  static size_t bytes(int64_t n, const Geo& G) {
+    return 2 * (ScratchLease::padded(soa_bytes(n)) + ScratchLease::padded(id_bytes(n))) +
+           ScratchLease::padded(key_bytes(n)) + 3 * ScratchLease::padded(cell_bytes(G)) +
+           ScratchLease::padded(sum_bytes(G));
   }
 };
-int make_sorted(Sorted& s, cudaStream_t st, int64_t n, const double* pos, const double* vel,
+int make_sorted(Sorted& s, ScratchLease& lease, cudaStream_t st, int64_t n, const double* pos, const double* vel,
                 const Geo& G, double h) {
   const int64_t N = (int64_t)G.nx * G.ny * G.nz;
-  const int64_t m = std::max<int64_t>(n, 1);
-  s.st = st;
-  s.a.st = s.b.st = st;
+  if (!lease.ok()) return -3;
   s.a.n = s.b.n = n;
-  if (cudaMallocAsync(&s.a.buf, sizeof(double) * 6 * m, st) != cudaSuccess ||
-      cudaMallocAsync(&s.b.buf, sizeof(double) * 6 * m, st) != cudaSuccess ||
-      cudaMallocAsync(&s.a.id, sizeof(int64_t) * m, st) != cudaSuccess ||
-      cudaMallocAsync(&s.b.id, sizeof(int64_t) * m, st) != cudaSuccess ||
-      cudaMallocAsync(&s.key, sizeof(int) * m, st) != cudaSuccess ||
-      cudaMallocAsync(&s.cnt, sizeof(int) * N, st) != cudaSuccess ||
-      cudaMallocAsync(&s.start, sizeof(int) * N, st) != cudaSuccess ||
-      cudaMallocAsync(&s.cursor, sizeof(int) * N, st) != cudaSuccess ||
-      cudaMallocAsync(&s.bsum, sizeof(int) * ((N + 1023) / 1024 + 1), st) != cudaSuccess)
-    return -3;
+  lease.take(&s.a.buf, soa_bytes(n));
+  lease.take(&s.b.buf, soa_bytes(n));
+  lease.take(&s.a.id, Sorted::id_bytes(n));
+  lease.take(&s.b.id, Sorted::id_bytes(n));
+  lease.take(&s.key, Sorted::key_bytes(n));
+  lease.take(&s.cnt, Sorted::cell_bytes(G));
+  lease.take(&s.start, Sorted::cell_bytes(G));
+  lease.take(&s.cursor, Sorted::cell_bytes(G));
+  lease.take(&s.bsum, Sorted::sum_bytes(G));
   if (n == 0) {
     cudaMemsetAsync(s.cnt, 0, sizeof(int) * N, st);
     cudaMemsetAsync(s.start, 0, sizeof(int) * N, st);
@@ -558,13 +559,16 @@ int make_sorted(Sorted& s, cudaStream_t st, int64_t n, const double* pos, const 
 }
 }  // namespace
 
-int flip_p2g(cudaStream_t st, int64_t n, const double* pos, const double* vel, int nx, int ny,
+int flip_p2g(const Context& ctx, int64_t n, const double* pos, const double* vel, int nx, int ny,
              int nz, double h, double* u, double* v, double* w, double* uw, double* vw, double* ww,
              uint8_t* uvalid, uint8_t* vvalid, uint8_t* wvalid, double* ulast, double* vlast,
              double* wlast) {
+  cudaStream_t st = ctx.stream;
   const Geo G{nx, ny, nz};
+  const size_t slices = p2g_scratch_bytes(G, sizeof(double));
+  ScratchLease lease(ctx, Sorted::bytes(n, G) + ScratchLease::padded(slices), st);
   Sorted s;
-  int e = make_sorted(s, st, n, pos, vel, G, h);
+  int e = make_sorted(s, lease, st, n, pos, vel, G, h);
   if (e) return e;
   const int64_t f0 = (int64_t)(nx + 1) * ny * nz, f1 = (int64_t)nx * (ny + 1) * nz,
                 f2 = (int64_t)nx * ny * (nz + 1);
@@ -575,21 +579,22 @@ int flip_p2g(cudaStream_t st, int64_t n, const double* pos, const double* vel, i
   cudaMemsetAsync(vw, 0, sizeof(double) * f1, st);
   cudaMemsetAsync(ww, 0, sizeof(double) * f2, st);
   void* scr = nullptr;
-  if (cudaMallocAsync(&scr, p2g_scratch_bytes(G, sizeof(double)), st) != cudaSuccess) return -3;
+  lease.take(&scr, slices);
   launch_p2g<double>(st, G, h, s.start, s.cnt, s.b.P(), p2g_scratch_at(scr, G, sizeof(double)), u, v, w, uw, vw,
                      ww, uvalid, vvalid, wvalid, ulast, vlast, wlast);
-  cudaFreeAsync(scr, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 // solveG2P through the simulator's tile kernel: the particles are sorted by
 // cell first, and each velocity is written back at its particle's index.
-int flip_g2p(cudaStream_t st, int64_t n, const double* pos, double* vel, int nx, int ny, int nz,
+int flip_g2p(const Context& ctx, int64_t n, const double* pos, double* vel, int nx, int ny, int nz,
              double h, const double* u, const double* v, const double* w, const double* ulast,
              const double* vlast, const double* wlast, double alpha) {
+  cudaStream_t st = ctx.stream;
   const Geo G{nx, ny, nz};
+  ScratchLease lease(ctx, Sorted::bytes(n, G), st);
   Sorted s;
-  int e = make_sorted(s, st, n, pos, vel, G, h);
+  int e = make_sorted(s, lease, st, n, pos, vel, G, h);
   if (e) return e;
   if (n > 0) {
     launch_g2p_tiles<double>(st, G, h, alpha, s.start, s.cnt, s.b.P(), u, v, w, ulast, vlast, wlast);
@@ -598,11 +603,13 @@ int flip_g2p(cudaStream_t st, int64_t n, const double* pos, double* vel, int nx,
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-int flip_reconstruct(cudaStream_t st, int64_t n, const double* pos, int nx, int ny, int nz,
+int flip_reconstruct(const Context& ctx, int64_t n, const double* pos, int nx, int ny, int nz,
                      double h, double radius, double* sdf, uint8_t* valid) {
+  cudaStream_t st = ctx.stream;
   const Geo G{nx, ny, nz};
+  ScratchLease lease(ctx, Sorted::bytes(n, G), st);
   Sorted s;
-  int e = make_sorted(s, st, n, pos, nullptr, G, h);
+  int e = make_sorted(s, lease, st, n, pos, nullptr, G, h);
   if (e) return e;
   PartsT<double> P = s.b.P();
   if (launch_reconstruct<double>(st, G, h, radius, s.start, s.cnt, P.px, P.py, P.pz, sdf, valid)) return -1;

@@ -104,19 +104,19 @@ class FluidSim {
 
 // ---- stage functions on device arrays (reference layout, AoS double particles) ----
 // Used by the per-function C ABI (HybridAdvectionSolver3D seams).
-int flip_p2g(cudaStream_t st, int64_t n, const double* pos, const double* vel, int nx, int ny,
+int flip_p2g(const Context& ctx, int64_t n, const double* pos, const double* vel, int nx, int ny,
              int nz, double h, double* u, double* v, double* w, double* uw, double* vw, double* ww,
              uint8_t* uvalid, uint8_t* vvalid, uint8_t* wvalid, double* ulast, double* vlast,
              double* wlast);
-int flip_sample(cudaStream_t st, int64_t n, const double* pts, int nx, int ny, int nz, double h,
+int flip_sample(const Context& ctx, int64_t n, const double* pts, int nx, int ny, int nz, double h,
                 const double* u, const double* v, const double* w, double* out);
-int flip_g2p(cudaStream_t st, int64_t n, const double* pos, double* vel, int nx, int ny, int nz,
+int flip_g2p(const Context& ctx, int64_t n, const double* pos, double* vel, int nx, int ny, int nz,
              double h, const double* u, const double* v, const double* w, const double* ulast,
              const double* vlast, const double* wlast, double alpha);
-int flip_advect(cudaStream_t st, int64_t n, double* pos, double* vel, int nx, int ny, int nz,
+int flip_advect(const Context& ctx, int64_t n, double* pos, double* vel, int nx, int ny, int nz,
                 double h, const double* u, const double* v, const double* w,
                 const double* collider, double dt);
-int flip_reconstruct(cudaStream_t st, int64_t n, const double* pos, int nx, int ny, int nz,
+int flip_reconstruct(const Context& ctx, int64_t n, const double* pos, int nx, int ny, int nz,
                      double h, double radius, double* sdf, uint8_t* valid);
 
 }  // namespace sc

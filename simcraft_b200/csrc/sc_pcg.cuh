@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -25,11 +26,77 @@ struct Context {
   // polls; 0 selects each wait's default.  A wait that reaches it gives up and
   // the call returns SC_ERR_TIMEOUT.
   int wait_limit = 0;
+  // Scratch of the stage functions, one block kept between calls (see ScratchLease).
+  struct Arena {
+    std::mutex m;
+    void* base = nullptr;
+    size_t cap = 0;
+    cudaEvent_t done = nullptr;  // the last call's work on the block
+  };
+  mutable Arena arena;
   std::string last_error;
   int set_error(int code, const std::string& msg) {
     last_error = msg;
     return code;
   }
+};
+
+// One call's scratch on stream `st`.  A call takes the context's block, grown to what it
+// needs, holds it while it enqueues its work and hands it on with an event that the next
+// call waits for on its own stream, so calls from several threads and streams take turns.
+// The block stays with the context: with an allocation per call the default pool, which
+// keeps nothing across a wait for the GPU, mapped ~1 GB again each time (the transfers of
+// 4.2M particles: 12 ms a call, 2 of them work).  Above kScratchKeep bytes, and under
+// stream capture, the call allocates and frees its own.
+constexpr size_t kScratchKeep = (size_t)2 << 30;
+class ScratchLease {
+ public:
+  ScratchLease(const Context& ctx, size_t bytes, cudaStream_t st) : st_(st), lock_(ctx.arena.m, std::defer_lock) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool known = cudaStreamIsCapturing(st, &cap) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    if (!known || cap != cudaStreamCaptureStatusNone || !ctx.arena.done || bytes > kScratchKeep) {
+      if (cudaMallocAsync(&own_, bytes, st) == cudaSuccess) at_ = (char*)own_;
+      return;
+    }
+    lock_.lock();
+    Context::Arena& a = ctx.arena;
+    if (cudaStreamWaitEvent(st, a.done, 0) != cudaSuccess) return;
+    held_ = &a;
+    if (a.cap < bytes) {
+      if (a.base) cudaFreeAsync(a.base, st);
+      a.base = nullptr;
+      a.cap = 0;
+      const size_t want = (bytes + ((size_t)1 << 20) - 1) >> 20 << 20;
+      if (cudaMallocAsync(&a.base, want, st) != cudaSuccess) {
+        a.base = nullptr;
+        return;
+      }
+      a.cap = want;
+    }
+    at_ = (char*)a.base;
+  }
+  ~ScratchLease() {
+    if (own_) cudaFreeAsync(own_, st_);
+    if (held_) cudaEventRecord(held_->done, st_);
+  }
+  ScratchLease(const ScratchLease&) = delete;
+  ScratchLease& operator=(const ScratchLease&) = delete;
+  bool ok() const { return at_ != nullptr; }
+  static size_t padded(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
+  // The next `bytes` of the block; the sum of padded(bytes) is what the lease was made for.
+  template <class T>
+  void take(T** p, size_t bytes) {
+    *p = (T*)at_;
+    at_ += padded(bytes);
+  }
+
+ private:
+  cudaStream_t st_;
+  std::unique_lock<std::mutex> lock_;
+  Context::Arena* held_ = nullptr;
+  void* own_ = nullptr;
+  char* at_ = nullptr;
 };
 
 enum { CRIT_ABS_LINF = 0, CRIT_REL_L2 = 1 };
