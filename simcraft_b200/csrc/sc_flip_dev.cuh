@@ -1111,10 +1111,10 @@ int launch_iter_cells(cudaStream_t st, const Geo& G, int iters, double* const b[
 // ---- solveP2G (advect-solver.cc:188-271) ----
 // Two kernels, no global atomics and a summation order fixed by the data, so
 // the sums are the same bit for bit on every run:
-//  k_p2g_tiles:  a block owns an 8x8x8 tile of cells, one thread per cell, and
-//                sums its particles' contributions over the nodes they reach
-//                (the tile's "region") into shared memory, then writes the
-//                region to the tile's slice of a scratch buffer;
+//  k_p2g_tiles:  a block owns an 8x8x8 tile of cells for one face grid, four
+//                lanes per cell, and sums its particles' contributions over the
+//                nodes they reach (the tile's "region") into shared memory,
+//                then writes the region to the tile's slice of a scratch buffer;
 //  k_p2g_gather: each face node adds the slices of the tiles whose regions
 //                hold it (at most 2 per axis), in tile order, and normalises.
 // Within a tile the accumulation is a fixed sequence too.  The weights of a
@@ -1122,21 +1122,35 @@ int launch_iter_cells(cudaStream_t st, const Geo& G, int iters, double* const b[
 // (offset 0 along AX, 1/2 along the others).  Along AX the particle's stencil
 // starts at its cell - 1 or at its cell (nearest node below or above its
 // centre); along the other axes at cell - 1, rounding aside.  So the nodes of
-// one cell's particles lie in a 5 x 4 x 4 window.  The tile walks that window
-// in 5 passes, one node plane along AX at a time: in a pass each thread sums
-// its particles (in bucket order) into 16 registers per quantity for the 4 x 4
-// nodes of the plane, stages them, and after a barrier each region node adds
-// the staged values of the (up to 16) cells that reach it, in a fixed order.
+// one cell's particles lie in a 5 x 4 x 4 window.  A block takes its 8 planes of
+// cells across AX from the last to the first.  Lane j of a cell sums the cell's
+// particles (in bucket order) into 5 x 4 registers per quantity for the window's
+// nodes with index j across AX, stages them, and after a barrier each region
+// node adds the staged values of the (up to 16) cells that reach it, in a fixed
+// order: sums first, then weights, in the same shared memory.
+// What bounds it is instruction issue (56% of the slots, the FP64 pipe 40%), and
+// most of that was the spline: with a thread per cell and a pass per window plane
+// a particle's factors were worked out anew in each of 4 passes, 36 a grid.  Now
+// a lane reads one coordinate (or the velocity), works out three factors, and the
+// cell's lanes trade them by shuffle: 12 a grid, one division per lane.  The sums
+// are the ones that the passes gave, bit for bit.  4.2M particles in FP64 1185 ->
+// 826 us, 33.5M in FP32 7.3 -> 5.3 ms.  Slower: the next particle's factors worked
+// out ahead (988 us, spills), the axis factors by stencil index and shifted by
+// selection (877 us), three blocks an SM instead of four in FP32 (6.5 ms).
 // Particles whose stencil starts elsewhere (rounding of the half-offset
 // nearest-node test, particles outside the grid box, or recorded bases of the
-// differentiable step) are added one thread after another, in thread order,
+// differentiable step) are added by one thread, cell after cell,
 // straight into the region; the region spans cell - 2 .. cell + 3 across AX
 // and cell - 1 .. cell + 3 along it, which holds every in-grid node of any
 // such particle.  Only a node beyond it (a recorded base far from the
 // particle's cell) goes to the global sums with an atomic add, raising the
 // spill flag that makes the gather read them.
 constexpr int kPT = 8;                        // cells per tile edge
-constexpr int kPThreads = kPT * kPT * kPT;    // one thread per cell
+constexpr int kPThreads = kPT * kPT * kPT;    // cells of a tile
+constexpr int kP2GThreads = 4 * kPT * kPT;    // P2G: four lanes per cell of a plane
+constexpr int kP2GRow = kPT * kPT + 8;        // staged values of a plane, 8 spare: the 4 x 8 lanes of a warp
+                                              // fall on different banks
+constexpr int kP2GStage = 5 * 4 * 4 * kP2GRow;
 template <int AX, int D>
 struct P2GRegion {
   static constexpr int lo = AX == D ? 1 : 2;          // nodes below the tile's first cell
@@ -1150,8 +1164,8 @@ constexpr int kP2GRegion = p2g_region<0>();  // the same for all three grids
 static_assert(p2g_region<1>() == kP2GRegion && p2g_region<2>() == kP2GRegion, "region sizes");
 template <class T>
 constexpr size_t p2g_smem_bytes() {
-  // 2 x 16 staged values per thread, the region (sum and weight), outlier list
-  return sizeof(T) * (2 * 16 * (size_t)kPThreads + 2 * (size_t)kP2GRegion) + sizeof(int) * (kPThreads + 32);
+  // a plane's staged sums, the region (sum and weight), the cells' buckets, outlier bits
+  return sizeof(T) * (kP2GStage + 2 * (size_t)kP2GRegion) + sizeof(int) * (2 * kPThreads + kPThreads / 32);
 }
 
 // Device scratch of the two kernels: per tile the three grids' regions (sum
@@ -1181,16 +1195,15 @@ inline P2GScratch p2g_scratch_at(void* base, const Geo& G, size_t elem) {
 
 // Spacing of the P2G kernels: a division by h is a multiplication by 1/h,
 // exactly, when h is a power of two (the usual 1/2^k grids); otherwise divide.
-template <class T>
+template <class T, bool POW2>
 struct P2GSpacing {
   T h, inv;
-  bool pow2;
-  __device__ __forceinline__ T over(T x) const { return pow2 ? rmul(x, inv) : rdiv(x, h); }
+  __device__ __forceinline__ T over(T x) const { return POW2 ? rmul(x, inv) : rdiv(x, h); }
 };
 // Nearest-node base along axis D for face grid AX (TGrid::nearest, as
 // nearest1 computes it); tb: recorded bases, or null.
-template <class T, int AX, int D>
-__device__ __forceinline__ int p2g_base(T p, const P2GSpacing<T>& sp, const int16_t* tb) {
+template <class T, int AX, int D, bool POW2>
+__device__ __forceinline__ int p2g_base(T p, const P2GSpacing<T, POW2>& sp, const int16_t* tb) {
   constexpr int o = D == AX ? 0 : 1;
   if (tb) return (int)tb[D * 2 + o];
   return (int)radd(sp.over(rsub(rsub(p, T(0)), rmul(o ? T(0.5) : T(0), sp.h))), T(0.5)) - 1;
@@ -1198,8 +1211,8 @@ __device__ __forceinline__ int p2g_base(T p, const P2GSpacing<T>& sp, const int1
 // The per-axis factor N(|p - x_node| / h) of the cubic B-spline (bspline),
 // with the 1/6 of its outer piece as a multiplication: within an ulp of the
 // reference's factor, which divides.
-template <class T, int AX, int D>
-__device__ __forceinline__ T p2g_factor(T p, int node, const P2GSpacing<T>& sp) {
+template <class T, int AX, int D, bool POW2>
+__device__ __forceinline__ T p2g_factor(T p, int node, const P2GSpacing<T, POW2>& sp) {
   constexpr T off = D == AX ? T(0) : T(0.5);
   const T r = sp.over(fabs(rsub(p, coord1(node, off, sp.h))));
   if (r < T(1)) return radd(rsub(T(2.0 / 3.0), rmul(r, r)), rmul(rmul(rmul(T(0.5), r), r), r));
@@ -1231,192 +1244,170 @@ __device__ __forceinline__ T p2g_weight(T w0, T w1, T w2) {
   return rmul(rmul(w0, w1), w2);
 }
 
-template <class T, int AX>
-__device__ void p2g_tile_grid(const Geo& G, const P2GSpacing<T>& h, int x0, int y0, int z0, int cx, int cy, int cz, int s0, int m,
-                              const PartsT<T>& P, const T* __restrict__ vel, const int16_t* tape,
-                              const int64_t* ids, T* stage, T* Rs, int* olist, T* slice, T* gsum, T* gwt,
+// One face grid of a tile, a plane of 8 x 8 cells across AX at a time.
+template <class T, int AX, bool POW2>
+__device__ void p2g_tile_grid(const Geo& G, const P2GSpacing<T, POW2>& h, int x0, int y0, int z0, const PartsT<T>& P,
+                              const T* __restrict__ vel, const int16_t* tape, const int64_t* ids, T* stage, T* Rs,
+                              const int* cbeg, const int* ccnt, unsigned* outl, T* slice, T* gsum, T* gwt,
                               int* spill) {
   constexpr int D1 = AX == 0 ? 1 : 0, D2 = AX == 2 ? 1 : 2;  // the two axes across AX
   constexpr int n0 = P2GRegion<AX, 0>::n, n1 = P2GRegion<AX, 1>::n, n2 = P2GRegion<AX, 2>::n;
   constexpr int lo0 = P2GRegion<AX, 0>::lo, lo1 = P2GRegion<AX, 1>::lo, lo2 = P2GRegion<AX, 2>::lo;
-  T* Rw = Rs + kP2GRegion;
-  const int tid = threadIdx.x;
-  const int c[3] = {cx, cy, cz};
-  const int t0[3] = {x0, y0, z0};
-  for (int e = tid; e < 2 * kP2GRegion; e += kPThreads) Rs[e] = T(0);
-  int nout = 0;
-  // the stencil class of the cell's first 32 particles, computed once: bit l
-  // of `outm` marks a particle whose stencil starts elsewhere, of `shm` one
-  // whose stencil starts at its cell along AX (else at cell - 1)
-  unsigned shm = 0u, outm = 0u;
-  for (int l = s0; l < s0 + min(m, 32); l++) {
-    const T p[3] = {P.px[l], P.py[l], P.pz[l]};
-    const int16_t* tb = tape ? tape + 6 * ids[l] : nullptr;
-    const int bA = p2g_base<T, AX, AX>(p[AX], h, tb);
-    const int b1 = p2g_base<T, AX, D1>(p[D1], h, tb), b2 = p2g_base<T, AX, D2>(p[D2], h, tb);
-    const int sh = bA - (c[AX] - 1);
-    const unsigned bit = 1u << (l - s0);
-    if (sh < 0 || sh > 1 || b1 != c[D1] - 1 || b2 != c[D2] - 1) {
-      outm |= bit;
-      nout++;
-    } else if (sh) {
-      shm |= bit;
-    }
-  }
-  // region strides along AX and across it
+  // region strides along AX and across it, the tile's cell strides likewise
   constexpr int stA = AX == 0 ? n1 * n2 : (AX == 1 ? n2 : 1);
   constexpr int st1 = D1 == 0 ? n1 * n2 : (D1 == 1 ? n2 : 1);
   constexpr int st2 = D2 == 0 ? n1 * n2 : (D2 == 1 ? n2 : 1);
-  for (int ip = 0; ip < 5; ip++) {
-    T as[16], aw[16];
+  constexpr int csA = AX == 0 ? kPT * kPT : (AX == 1 ? kPT : 1);
+  constexpr int cs1 = D1 == 0 ? kPT * kPT : (D1 == 1 ? kPT : 1);
+  constexpr int cs2 = D2 == 0 ? kPT * kPT : (D2 == 1 ? kPT : 1);
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int j = lane >> 3, sub = lane & 7;        // window index along D1; cell of the warp
+  const int q1c = tid >> 5, q2c = sub;            // the cell's place across AX
+  const int t0[3] = {x0, y0, z0};
+  const T* coord[3] = {P.px, P.py, P.pz};
+  // lanes 0..2 of a cell read a coordinate each (AX, D1, D2), lane 3 the velocity
+  const T* mine = j == 0 ? coord[AX] : (j == 1 ? coord[D1] : (j == 2 ? coord[D2] : vel));
+  const T half = j == 0 ? T(0) : rmul(T(0.5), h.h);
+  const int c1 = t0[D1] + q1c, c2 = t0[D2] + q2c;
+  const int tcol = j == 0 ? AX * 2 : (j == 1 ? D1 * 2 + 1 : D2 * 2 + 1);  // this lane's recorded base
+  const T o1 = radd(radd((T)(c1 - 1), T(0.5)), (T)j), o2 = radd(radd((T)(c2 - 1), T(0.5)), (T)j);
+  for (int e = tid; e < 2 * kP2GRegion; e += kP2GThreads) Rs[e] = T(0);
+  // From the last plane to the first: a region node then gets its five planes'
+  // sums in the order of the window index along AX.
+  for (int a = kPT - 1; a >= 0; a--) {
+    const int tc = a * csA + q1c * cs1 + q2c * cs2;
+    const int s0 = cbeg[tc], m = ccnt[tc];
+    const int mw = __reduce_max_sync(0xffffffffu, m);
+    if (!__syncthreads_or(mw > 0)) continue;  // (and the staged values of the last plane are read)
+    const int cA = t0[AX] + a;
+    const int own = j == 0 ? cA : (j == 1 ? c1 : c2);
+    const T oA = (T)(cA - 1 + j), oA4 = (T)(cA + 3);
+    T as[5][4], aw[5][4];
 #pragma unroll
-    for (int q = 0; q < 16; q++) {
-      as[q] = T(0);
-      aw[q] = T(0);
-    }
-    for (int l = s0; l < s0 + m; l++) {
-      int sh;
-      if (l - s0 < 32) {
-        const unsigned bit = 1u << (l - s0);
-        if (outm & bit) continue;
-        sh = (shm & bit) ? 1 : 0;
-      } else {
-        const T p[3] = {P.px[l], P.py[l], P.pz[l]};
-        const int16_t* tb = tape ? tape + 6 * ids[l] : nullptr;
-        const int bA = p2g_base<T, AX, AX>(p[AX], h, tb);
-        const int b1 = p2g_base<T, AX, D1>(p[D1], h, tb), b2 = p2g_base<T, AX, D2>(p[D2], h, tb);
-        sh = bA - (c[AX] - 1);
-        if (sh < 0 || sh > 1 || b1 != c[D1] - 1 || b2 != c[D2] - 1) {
-          if (ip == 0) nout++;
-          continue;
-        }
+    for (int ip = 0; ip < 5; ip++)
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        as[ip][k] = T(0);
+        aw[ip][k] = T(0);
       }
-      const int t = ip - sh;
-      if (t < 0 || t > 3) continue;
-      const T p[3] = {P.px[l], P.py[l], P.pz[l]};
-      const int bA = c[AX] - 1 + sh, b1 = c[D1] - 1, b2 = c[D2] - 1;
-      // own axis: offset 0, across: 1/2
-      const T wA = p2g_factor_q(h.over(p[AX]), (T)(bA + t));
-      const T q1 = h.over(p[D1]), q2 = h.over(p[D2]);
-      const T c1 = radd((T)b1, T(0.5)), c2 = radd((T)b2, T(0.5));
-      T w1[4], w2[4];
+    bool any_out = false;
+    T x = m > 0 ? mine[s0] : T(0);
+    for (int l = 0; l < mw; l++) {
+      const bool in = l < m;
+      const T q = h.over(x);
+      int base = (int)radd(h.over(rsub(x, half)), T(0.5)) - 1;
+      if (tape && in && j < 3) base = (int)tape[6 * ids[s0 + l] + tcol];
+      const int sh = base - (own - 1);
+      const unsigned obit = __ballot_sync(0xffffffffu, in && (j == 0 ? (sh < 0 || sh > 1) : (j < 3 && sh != 0)));
+      const unsigned sbit = __ballot_sync(0xffffffffu, j == 0 && sh == 1);
+      // up: the stencil starts at the cell along AX, else one below
+      const bool out = ((obit >> sub) & 0x010101u) != 0u, up = ((sbit >> sub) & 1u) != 0u;
+      any_out = any_out || out;
+      const bool ok = in && !out;
+      const T qA = __shfl_sync(0xffffffffu, q, sub), q1 = __shfl_sync(0xffffffffu, q, 8 + sub),
+              q2 = __shfl_sync(0xffffffffu, q, 16 + sub), vv = __shfl_sync(0xffffffffu, x, 24 + sub);
+      if (l + 1 < m) x = mine[s0 + l + 1];
+      const T v = ok ? vv : T(0);
+      // own axis: offset 0, across: 1/2.  Along AX lane j takes plane j, and lane
+      // 0 the last plane when the stencil does not reach the first.
+      const T fA = p2g_factor_q(qA, j == 0 && up ? oA4 : oA);
+      const T wAj = ok ? fA : T(0);
+      const T w1 = p2g_factor_q(q1, o1);
+      const T w2j = p2g_factor_q(q2, o2);
+      T wA[4], w2[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        w1[j] = p2g_factor_q(q1, radd(c1, (T)j));
-        w2[j] = p2g_factor_q(q2, radd(c2, (T)j));
+      for (int k = 0; k < 4; k++) {
+        wA[k] = __shfl_sync(0xffffffffu, wAj, 8 * k + sub);
+        w2[k] = __shfl_sync(0xffffffffu, w2j, 8 * k + sub);
       }
-      const T v = vel[l];
+      // the window plane the particle does not reach gets weight and velocity zero
 #pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int ip = 0; ip < 5; ip++) {
+        const T wa = ip == 0 ? (up ? T(0) : wA[0]) : (ip == 4 ? (up ? wA[0] : T(0)) : wA[ip]);
+        const T vp = ip == 0 ? (up ? T(0) : v) : (ip == 4 ? (up ? v : T(0)) : v);
+        const T wa1 = rmul(wa, w1);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           // factors in axis order x, y, z
-          T f[3];
-          f[AX] = wA;
-          f[D1] = w1[j];
-          f[D2] = w2[k];
-          const T wt = p2g_weight(f[0], f[1], f[2]);
+          const T wt = AX == 2 ? rmul(rmul(w1, w2[k]), wa) : rmul(wa1, w2[k]);
           // one fused multiply-add (the sums' order is not the reference's
           // anyway, which adds from a parallel loop)
-          as[j * 4 + k] = fma(v, wt, as[j * 4 + k]);
-          aw[j * 4 + k] = radd(aw[j * 4 + k], wt);
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 16; q++) {
-      stage[q * kPThreads + tid] = as[q];
-      stage[(16 + q) * kPThreads + tid] = aw[q];
-    }
-    __syncthreads();
-    // region nodes of this pass: along AX the plane of cell + ip - 1 of each
-    // cell of the tile (region index cell + ip), across AX the nodes reached
-    // from the tile's cells at their typical bases (region indices 1..11)
-    // (the index that runs fastest over the threads is the one along z, in the
-    // staged values and in the region alike: consecutive threads read
-    // consecutive words)
-    constexpr int NA = kPT, NB = kPT + 3;
-    for (int e = tid; e < NA * NB * NB; e += kPThreads) {
-      int a, b, cc;
-      if (AX == 2) {
-        a = e % NA;
-        const int r = e / NA;
-        b = r / NB;
-        cc = r - b * NB;
-      } else {
-        a = e / (NB * NB);
-        const int r = e - a * (NB * NB);
-        b = r / NB;
-        cc = r - b * NB;
-      }
-      const int rb = b + 1, rc = cc + 1;  // region indices across AX
-      T S = T(0), W = T(0);
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int q1 = rb - 1 - j;  // the cell along D1 whose window index j is this node
-        if (q1 < 0 || q1 >= kPT) continue;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const int q2 = rc - 1 - k;
-          if (q2 < 0 || q2 >= kPT) continue;
-          int lc[3];
-          lc[AX] = a;
-          lc[D1] = q1;
-          lc[D2] = q2;
-          const int src = (lc[0] * kPT + lc[1]) * kPT + lc[2];
-          S = radd(S, stage[(j * 4 + k) * kPThreads + src]);
-          W = radd(W, stage[(16 + j * 4 + k) * kPThreads + src]);
+          as[ip][k] = fma(vp, wt, as[ip][k]);
+          aw[ip][k] = radd(aw[ip][k], wt);
         }
       }
-      const int ridx = (a + ip) * stA + rb * st1 + rc * st2;
-      Rs[ridx] = radd(Rs[ridx], S);
-      Rw[ridx] = radd(Rw[ridx], W);
     }
-    __syncthreads();
+    if (any_out && j == 0) atomicOr(outl + (tc >> 5), 1u << (tc & 31));
+#pragma unroll
+    for (int ph = 0; ph < 2; ph++) {
+#pragma unroll
+      for (int ip = 0; ip < 5; ip++)
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          stage[((ip * 4 + k) * 4 + j) * kP2GRow + q1c * kPT + q2c] = ph ? aw[ip][k] : as[ip][k];
+      __syncthreads();
+      // along AX the plane of cell + ip - 1 (region index cell + ip), across AX
+      // the nodes reached from the tile's cells at their typical bases (region
+      // indices 1..11); a thread adds the (up to 16) cells that reach its node
+      constexpr int NB = kPT + 3;
+      T* R = Rs + ph * kP2GRegion;
+      for (int e = tid; e < 5 * NB * NB; e += kP2GThreads) {
+        const int ip = e / (NB * NB), r = e - ip * (NB * NB), b = r / NB, cc = r - b * NB;
+        T S = T(0);
+#pragma unroll
+        for (int jj = 0; jj < 4; jj++) {
+          const int r1 = b - jj;  // the cell along D1 whose window index jj is this node
+          if (r1 < 0 || r1 >= kPT) continue;
+#pragma unroll
+          for (int k = 0; k < 4; k++) {
+            const int r2 = cc - k;
+            if (r2 < 0 || r2 >= kPT) continue;
+            S = radd(S, stage[((ip * 4 + k) * 4 + jj) * kP2GRow + r1 * kPT + r2]);
+          }
+        }
+        const int ridx = (a + ip) * stA + (b + 1) * st1 + (cc + 1) * st2;
+        R[ridx] = radd(R[ridx], S);
+      }
+      if (ph == 0) __syncthreads();
+    }
   }
-  // the particles outside the typical windows, thread after thread
-  if (__syncthreads_or(nout > 0)) {
-    const int lane = tid & 31, warp = tid >> 5;
-    int* wcnt = olist + kPThreads;
-    const unsigned bal = __ballot_sync(0xffffffffu, nout > 0);
-    if (lane == 0) wcnt[warp] = __popc(bal);
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < kPThreads / 32; w++) {
-      if (w < warp) before += wcnt[w];
-      total += wcnt[w];
-    }
-    if (nout > 0) olist[before + __popc(bal & ((1u << lane) - 1u))] = tid;
-    __syncthreads();
-    for (int qi = 0; qi < total; qi++) {
-      if (olist[qi] == tid) {
-        const int fx = G.fx(AX), fy = G.fy(AX), fz = G.fz(AX);
+  __syncthreads();
+  // the particles outside the typical windows, cell after cell
+  if (tid == 0) {
+    const int fx = G.fx(AX), fy = G.fy(AX), fz = G.fz(AX);
+    T* Rw = Rs + kP2GRegion;
+    for (int wd = 0; wd < kPThreads / 32; wd++) {
+      for (unsigned bits = outl[wd]; bits; bits &= bits - 1) {
+        const int tc = wd * 32 + __ffs(bits) - 1;
+        const int c[3] = {x0 + tc / (kPT * kPT), y0 + (tc / kPT) % kPT, z0 + tc % kPT};
+        const int s0 = cbeg[tc], m = ccnt[tc];
         for (int l = s0; l < s0 + m; l++) {
           const T p[3] = {P.px[l], P.py[l], P.pz[l]};
           const int16_t* tb = tape ? tape + 6 * ids[l] : nullptr;
           int b[3];
-          b[AX] = p2g_base<T, AX, AX>(p[AX], h, tb);
-          b[D1] = p2g_base<T, AX, D1>(p[D1], h, tb);
-          b[D2] = p2g_base<T, AX, D2>(p[D2], h, tb);
+          b[AX] = p2g_base<T, AX, AX, POW2>(p[AX], h, tb);
+          b[D1] = p2g_base<T, AX, D1, POW2>(p[D1], h, tb);
+          b[D2] = p2g_base<T, AX, D2, POW2>(p[D2], h, tb);
           const int sh = b[AX] - (c[AX] - 1);
           if (!(sh < 0 || sh > 1 || b[D1] != c[D1] - 1 || b[D2] != c[D2] - 1)) continue;
           const T v = vel[l];
           T w[3][4];
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            w[0][i] = p2g_factor<T, AX, 0>(p[0], b[0] + i, h);
-            w[1][i] = p2g_factor<T, AX, 1>(p[1], b[1] + i, h);
-            w[2][i] = p2g_factor<T, AX, 2>(p[2], b[2] + i, h);
+            w[0][i] = p2g_factor<T, AX, 0, POW2>(p[0], b[0] + i, h);
+            w[1][i] = p2g_factor<T, AX, 1, POW2>(p[1], b[1] + i, h);
+            w[2][i] = p2g_factor<T, AX, 2, POW2>(p[2], b[2] + i, h);
           }
           for (int i = 0; i < 4; i++) {
             const int ga = b[0] + i;
             if (ga < 0 || ga >= fx) continue;
-            for (int j = 0; j < 4; j++) {
-              const int gb = b[1] + j;
+            for (int jj = 0; jj < 4; jj++) {
+              const int gb = b[1] + jj;
               if (gb < 0 || gb >= fy) continue;
               for (int k = 0; k < 4; k++) {
                 const int gc = b[2] + k;
                 if (gc < 0 || gc >= fz) continue;
-                const T wt = p2g_weight(w[0][i], w[1][j], w[2][k]);
+                const T wt = p2g_weight(w[0][i], w[1][jj], w[2][k]);
                 const int la = ga - (t0[0] - lo0), lb = gb - (t0[1] - lo1), lcc = gc - (t0[2] - lo2);
                 if (la >= 0 && la < n0 && lb >= 0 && lb < n1 && lcc >= 0 && lcc < n2) {
                   const int ridx = (la * n1 + lb) * n2 + lcc;
@@ -1433,47 +1424,54 @@ __device__ void p2g_tile_grid(const Geo& G, const P2GSpacing<T>& h, int x0, int 
           }
         }
       }
-      __syncthreads();
     }
   }
-  for (int e = tid; e < 2 * kP2GRegion; e += kPThreads) slice[e] = Rs[e];
   __syncthreads();
+  for (int e = tid; e < 2 * kP2GRegion; e += kP2GThreads) slice[e] = Rs[e];
 }
 
-template <class T>
-__global__ void __launch_bounds__(kPThreads)
-    k_p2g_tiles(Geo G, double hd, int pow2, const int* __restrict__ start, const int* __restrict__ cnt, PartsT<T> P,
+template <class T, bool POW2>
+__global__ void __launch_bounds__(kP2GThreads, sizeof(T) == 4 ? 4 : 2)
+    k_p2g_tiles(Geo G, double hd, const int* __restrict__ start, const int* __restrict__ cnt, PartsT<T> P,
                 T* slices, int* occ, T* su, T* sv, T* sw, T* wu, T* wv, T* ww, int* spill, const int16_t* tape,
                 const int64_t* ids) {
   extern __shared__ __align__(16) unsigned char p2g_dyn[];
   T* stage = reinterpret_cast<T*>(p2g_dyn);
-  T* Rs = stage + 32 * kPThreads;
-  int* olist = reinterpret_cast<int*>(Rs + 2 * kP2GRegion);
-  P2GSpacing<T> h;
+  T* Rs = stage + kP2GStage;
+  int* cbeg = reinterpret_cast<int*>(Rs + 2 * kP2GRegion);
+  int* ccnt = cbeg + kPThreads;
+  unsigned* outl = reinterpret_cast<unsigned*>(ccnt + kPThreads);
+  P2GSpacing<T, POW2> h;
   h.h = (T)hd;
   h.inv = (T)(1.0 / hd);
-  h.pow2 = pow2 != 0;
+  const int tile = blockIdx.x / 3, ax = blockIdx.x % 3;
   const int ntz = (G.nz + kPT - 1) / kPT, nty = (G.ny + kPT - 1) / kPT;
-  const int tz = blockIdx.x % ntz, ty = (blockIdx.x / ntz) % nty, tx = blockIdx.x / (ntz * nty);
+  const int tz = tile % ntz, ty = (tile / ntz) % nty, tx = tile / (ntz * nty);
   const int x0 = tx * kPT, y0 = ty * kPT, z0 = tz * kPT;
-  const int lz = threadIdx.x % kPT, ly = (threadIdx.x / kPT) % kPT, lx = threadIdx.x / (kPT * kPT);
-  const int cx = x0 + lx, cy = y0 + ly, cz = z0 + lz;
-  int m = 0, s0 = 0;
-  if (cx < G.nx && cy < G.ny && cz < G.nz) {
-    const int cell = (int)lin(cx, cy, cz, G.ny, G.nz);
-    m = cnt[cell];
-    s0 = start[cell];
+  int most = 0;
+  for (int e = threadIdx.x; e < kPThreads; e += kP2GThreads) {
+    const int cx = x0 + e / (kPT * kPT), cy = y0 + (e / kPT) % kPT, cz = z0 + e % kPT;
+    int m = 0, s0 = 0;
+    if (cx < G.nx && cy < G.ny && cz < G.nz) {
+      const int cell = (int)lin(cx, cy, cz, G.ny, G.nz);
+      m = cnt[cell];
+      s0 = start[cell];
+    }
+    cbeg[e] = s0;
+    ccnt[e] = m;
+    most = max(most, m);
   }
-  const bool any = __syncthreads_or(m > 0);
-  if (threadIdx.x == 0) occ[blockIdx.x] = any ? 1 : 0;
+  if (threadIdx.x < kPThreads / 32) outl[threadIdx.x] = 0u;
+  const bool any = __syncthreads_or(most > 0);
+  if (ax == 0 && threadIdx.x == 0) occ[tile] = any ? 1 : 0;
   if (!any) return;  // no particle in this tile: its slices are never read
-  T* slice = slices + (int64_t)blockIdx.x * 6 * kP2GRegion;
-  p2g_tile_grid<T, 0>(G, h, x0, y0, z0, cx, cy, cz, s0, m, P, P.vx, tape, ids, stage, Rs, olist, slice, su, wu,
-                      spill);
-  p2g_tile_grid<T, 1>(G, h, x0, y0, z0, cx, cy, cz, s0, m, P, P.vy, tape, ids, stage, Rs, olist,
-                      slice + 2 * kP2GRegion, sv, wv, spill);
-  p2g_tile_grid<T, 2>(G, h, x0, y0, z0, cx, cy, cz, s0, m, P, P.vz, tape, ids, stage, Rs, olist,
-                      slice + 4 * kP2GRegion, sw, ww, spill);
+  T* slice = slices + ((int64_t)tile * 6 + 2 * ax) * kP2GRegion;
+  if (ax == 0)
+    p2g_tile_grid<T, 0, POW2>(G, h, x0, y0, z0, P, P.vx, tape, ids, stage, Rs, cbeg, ccnt, outl, slice, su, wu, spill);
+  else if (ax == 1)
+    p2g_tile_grid<T, 1, POW2>(G, h, x0, y0, z0, P, P.vy, tape, ids, stage, Rs, cbeg, ccnt, outl, slice, sv, wv, spill);
+  else
+    p2g_tile_grid<T, 2, POW2>(G, h, x0, y0, z0, P, P.vz, tape, ids, stage, Rs, cbeg, ccnt, outl, slice, sw, ww, spill);
 }
 
 // Tiles along one axis whose regions hold node x: [lo, hi] (empty if lo > hi).
@@ -1549,16 +1547,16 @@ int launch_p2g(cudaStream_t st, const Geo& G, double h, const int* start, const 
                uint8_t* vw, T* lu, T* lv, T* lw, const int16_t* tape = nullptr, const int64_t* ids = nullptr) {
   static bool attr = false;
   if (!attr) {
-    cudaFuncSetAttribute(k_p2g_tiles<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p2g_smem_bytes<T>());
+    cudaFuncSetAttribute(k_p2g_tiles<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p2g_smem_bytes<T>());
+    cudaFuncSetAttribute(k_p2g_tiles<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p2g_smem_bytes<T>());
     attr = true;
   }
   const int64_t tiles = p2g_ntiles(G);
   cudaMemsetAsync(scr.spill, 0, sizeof(int), st);
   int ex = 0;
-  const int pow2 = std::frexp(h, &ex) == 0.5 ? 1 : 0;
-  k_p2g_tiles<T><<<(unsigned)tiles, kPThreads, p2g_smem_bytes<T>(), st>>>(G, h, pow2, start, cnt, P, (T*)scr.slices,
-                                                                          scr.occ, gu, gv, gw, wu, wv, ww,
-                                                                          scr.spill, tape, ids);
+  auto* kernel = std::frexp(h, &ex) == 0.5 ? &k_p2g_tiles<T, true> : &k_p2g_tiles<T, false>;
+  kernel<<<(unsigned)(3 * tiles), kP2GThreads, p2g_smem_bytes<T>(), st>>>(
+      G, h, start, cnt, P, (T*)scr.slices, scr.occ, gu, gv, gw, wu, wv, ww, scr.spill, tape, ids);
   const int64_t nf = (int64_t)(G.nx + 1) * G.ny * G.nz + (int64_t)G.nx * (G.ny + 1) * G.nz +
                      (int64_t)G.nx * G.ny * (G.nz + 1);
   k_p2g_gather<T><<<nblk(nf), kT, 0, st>>>(G, (const T*)scr.slices, scr.occ, scr.spill, gu, gv, gw, wu, wv, ww,
