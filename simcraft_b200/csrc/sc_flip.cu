@@ -519,16 +519,16 @@ int flip_advect(const Context& ctx, int64_t n, double* pos, double* vel, int nx,
 }
 
 namespace {
-// Sorted copy of AoS particles plus cell buckets, for the stage functions.
+// Sorted copy of the particles as arrays plus cell buckets, for the stage functions.
 struct Sorted {
-  StageParticles a, b;
+  StageParticles b;
   int *key = nullptr, *cnt = nullptr, *start = nullptr, *cursor = nullptr, *bsum = nullptr;
   static size_t id_bytes(int64_t n) { return sizeof(int64_t) * (size_t)std::max<int64_t>(n, 1); }
   static size_t key_bytes(int64_t n) { return sizeof(int) * (size_t)std::max<int64_t>(n, 1); }
   static size_t cell_bytes(const Geo& G) { return sizeof(int) * (size_t)G.nx * G.ny * G.nz; }
   static size_t sum_bytes(const Geo& G) { return sizeof(int) * (((size_t)G.nx * G.ny * G.nz + 1023) / 1024 + 1); }
   static size_t bytes(int64_t n, const Geo& G) {
-    return 2 * (ScratchLease::padded(soa_bytes(n)) + ScratchLease::padded(id_bytes(n))) +
+    return ScratchLease::padded(soa_bytes(n)) + ScratchLease::padded(id_bytes(n)) +
            ScratchLease::padded(key_bytes(n)) + 3 * ScratchLease::padded(cell_bytes(G)) +
            ScratchLease::padded(sum_bytes(G));
   }
@@ -537,10 +537,8 @@ int make_sorted(Sorted& s, ScratchLease& lease, cudaStream_t st, int64_t n, cons
                 const Geo& G, double h) {
   const int64_t N = (int64_t)G.nx * G.ny * G.nz;
   if (!lease.ok()) return -3;
-  s.a.n = s.b.n = n;
-  lease.take(&s.a.buf, soa_bytes(n));
+  s.b.n = n;
   lease.take(&s.b.buf, soa_bytes(n));
-  lease.take(&s.a.id, Sorted::id_bytes(n));
   lease.take(&s.b.id, Sorted::id_bytes(n));
   lease.take(&s.key, Sorted::key_bytes(n));
   lease.take(&s.cnt, Sorted::cell_bytes(G));
@@ -552,9 +550,9 @@ int make_sorted(Sorted& s, ScratchLease& lease, cudaStream_t st, int64_t n, cons
     cudaMemsetAsync(s.start, 0, sizeof(int) * N, st);
     return 0;
   }
-  k_aos_to_soa<double><<<nblk(n), kT, 0, st>>>(n, pos, vel, s.a.P(), s.a.id);
   SortBufs sb{s.key, s.cnt, s.start, s.cursor, s.bsum};
-  sort_particles<double>(st, n, G, h, s.a.P(), s.a.id, s.b.P(), s.b.id, sb);
+  const PartsSrc<double> src{pos, pos + 1, pos + 2, vel, vel ? vel + 1 : nullptr, vel ? vel + 2 : nullptr, 3};
+  sort_particles<double>(st, n, G, h, src, nullptr, s.b.P(), s.b.id, sb);
   return 0;
 }
 }  // namespace
