@@ -905,7 +905,7 @@ def main():
     bytes_fwd = N * (6 * 8 + 1)
     achieved = bytes_fwde32 / (kms32[7] * 1e-3) / 1e9
     traffic = read_traffic("fwd_eisenstat_fp32", n)
-    roofline = {"bound": "hbm", "kernel": "fused Eisenstat forward sweep, FP32 (k_wave FwdEisenstatOp<float>), "
+    roofline = {"bound": "hbm", "kernel": "fused Eisenstat forward sweep, FP32 (k_sweep FwdEisenstatOp<float>), "
                                           "the top kernel of the mixed solve",
                 "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / pk["hbm_gbs"], "peak_source": pk_src + " (burst copy)",

@@ -187,7 +187,7 @@ int sc_pcg_time_kernels(sc_pcg* pcg, int reps, double* ms_out);
  * synchronisation is not acceptable.  As in sc_pcg_precond_device, entries the
  * reference never reads (couplings to inactive cells, inactive rows) may hold
  * any value, NaN included.  It allocates nothing: its scratch is one static device array
- * of about 4.4 MB that every GPU loading the library holds until exit, which
+ * of about 8.5 MB that every GPU loading the library holds until exit, which
  * limits the grid to 32768 tiled cells (ceil(nx/32)*32 * ceil(ny/8)*8 * nz,
  * e.g. 32^3) in at most 8 column tiles; larger grids return SC_ERR_INVALID with
  * a message.  The first call on each device performs a one-time set-up on that

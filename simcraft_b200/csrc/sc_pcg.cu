@@ -1946,7 +1946,7 @@ int PcgSolver::time_kernels(int reps, double* ms) {
 // counters) in the file-scope array below instead of allocating.  It launches
 // the same kernels as sc_pcg_precond_device.
 //
-// The array is kNoAllocBytes (about 7.6 MB) and lives on every GPU that loads
+// The array is kNoAllocBytes (about 8.5 MB) and lives on every GPU that loads
 // this library, until the process exits.  It bounds the problem size: at most
 // kNoAllocMaxTiled tiled elements (ceil(nx/32)*32 * ceil(ny/8)*8 * nz, e.g. a
 // 32^3 grid) in at most kNoAllocMaxTiles column tiles.  Every call shares the
