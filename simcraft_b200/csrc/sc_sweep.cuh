@@ -257,10 +257,13 @@ __device__ __forceinline__ void st_cluster64(uint32_t p, unsigned long long v) {
 __device__ __forceinline__ void add_cluster(uint32_t p, int v) {
   asm volatile("red.relaxed.cluster.shared::cluster.add.s32 [%0], %1;" ::"r"(p), "r"(v) : "memory");
 }
-// 16-byte copy global -> shared past L1, visible to this thread after cp_async_wait;
-// bytes 0: nothing is read, the destination becomes zero.
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+// 16-byte copy global -> shared past L1, visible to this thread after cp_async_wait.
+// Off, nothing is written either: copies in flight to one place are not ordered, so a
+// zero fill of a slot could land on the data that is copied there next.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool on) {
+  asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p cp.async.cg.shared.global [%0], [%1], 16;\n}\n" ::"r"(dst),
+               "l"(src), "r"((int)on)
+               : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
@@ -436,6 +439,26 @@ struct SweepSmem {
   static constexpr int bytes = sums + kSweepThreads / 32 * 8;
   static_assert(bytes <= room, "a sweep block's shared memory");
 };
+
+// What a compute warp copies while it sweeps group gi of a tile's NC chunks (groups of
+// four): the first `chunks` chunks of group `group` of this tile or the next one, DG
+// groups further on, into the slots that the group's own chunks leave.  ahead: groups of
+// the next tile already being copied; has_next: that tile is known and is swept.
+// One group of copies is committed per chunk, the empty ones too, and each chunk waits
+// for all but the last 4 * DG - 1, so a slot's last copy has landed before the next one
+// into it is issued.
+struct SweepAhead {
+  bool next;
+  int group, chunks;
+};
+__host__ __device__ __forceinline__ SweepAhead sweep_ahead(int gi, int NC, int DG, int ahead, bool has_next) {
+  const int NG = (NC + 3) >> 2, g = gi + DG;
+  const bool next = g >= NG;
+  const int group = next ? g - NG : g;
+  const bool on = group < NG && (!next || (has_next && ahead == group));
+  const int left = NC - 4 * group;
+  return {next, group, on ? (left < 4 ? left : 4) : 0};
+}
 
 struct SweepWait {
   PcgScalars* sc;
@@ -622,13 +645,13 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     const T* stage = reinterpret_cast<const T*>(dyn + SM::stage) + cw * D * NV * 128 + lane * kLane;
     const uint32_t stage_u32 = smem_u32(stage);
     // copies this lane's vectors of a chunk (at element v of a vector, f of the factor
-    // stream) into stage slot `slot`; bytes 16, or 0 for no chunk
-    auto copy = [&](int64_t v, int64_t f, int slot, int bytes) {
+    // stream) into stage slot `slot`; off: no chunk
+    auto copy = [&](int64_t v, int64_t f, int slot, bool on) {
 #pragma unroll
       for (int k = 0; k < NV; k++) {
         const T* p = k < NX ? op.src[k < NX ? k : 0] + v : op.fac + (f + (k - NX) * 128);
-        cp_async16(stage_u32 + (slot * NV + k) * SM::chunk, p, bytes);
-        if constexpr (sizeof(T) == 8) cp_async16(stage_u32 + (slot * NV + k) * SM::chunk + 512, p + 64, bytes);
+        cp_async16(stage_u32 + (slot * NV + k) * SM::chunk, p, on);
+        if constexpr (sizeof(T) == 8) cp_async16(stage_u32 + (slot * NV + k) * SM::chunk + 512, p + 64, on);
       }
     };
     constexpr int DG = D / 4;  // groups of four chunks in flight
@@ -675,7 +698,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           for (int i = 0; i < 4; i++) {
             const bool in = 4 * ahead + i < NC;
             const int64_t c = chunk_at(c0, in ? 4 * ahead + i : 0);
-            copy(c * 128 + lane * kLane, c * (Op::FS * 128) + lane * kLane, (4 * (group + ahead) + i) & (D - 1), in ? 16 : 0);
+            copy(c * 128 + lane * kLane, c * (Op::FS * 128) + lane * kLane, (4 * (group + ahead) + i) & (D - 1), in);
             if (n == 0) cp_async_commit();  // a group per chunk, as later
           }
         if (n == 0) {
@@ -754,30 +777,26 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         T* by = moy + (int64_t)d0 * 64;
         // the group DG further, of this tile or the next, is copied into the slots these
         // chunks leave, while their steps wait for one another
-        int tg = (d0 >> 2) + DG;
-        int64_t cf = c0;
-        if (tg >= NG) {
-          tg -= NG;
+        const int gi = d0 >> 2;
+        if (gi + DG >= NG && !next_known) {
           unsigned w;
-          if (!next_known && peek(n + 1, w)) {
+          if (peek(n + 1, w)) {
             next_known = true;
             Tile t1;
             if (w != kNoTile && tile_of(w, t1)) nc0 = (int64_t)((t1.Y * g.ntx + t1.X) * kSweepWarps + cw) * NC;
           }
-          cf = ahead == tg ? nc0 : -1;
-          if (cf >= 0 && tg < NG) ahead++;
         }
-        const int nf = cf >= 0 ? NC - 4 * tg : 0;  // its chunks (4, fewer at a tile's end)
-        cf = nf > 0 ? chunk_at(cf, 4 * tg) : c0;
+        const SweepAhead go = sweep_ahead(gi, NC, DG, ahead, nc0 >= 0);
+        if (go.next && go.chunks) ahead++;
+        const int64_t cf = go.chunks ? chunk_at(go.next ? nc0 : c0, 4 * go.group) : c0;
         const int64_t fv = cf * 128 + lane * kLane, ff = cf * (Op::FS * 128) + lane * kLane;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           const int d = d0 + i;
           const bool live = kMain || d < NC;
           const int slot = (sbase + i) & (D - 1);
-          const int bytes = i < nf ? 16 : 0;
-          const int64_t ahead_by = i < nf ? kDir * i : 0;
-          const int64_t av = fv + ahead_by * 128, af = ff + ahead_by * (Op::FS * 128);
+          const bool on = i < go.chunks;
+          const int64_t av = fv + kDir * i * 128, af = ff + kDir * i * (Op::FS * 128);
           if (live) {
             // the neighbours' boundary values, x entry d + 2 and y entry d + 1, and this
             // chunk's inputs.  (Fetching the next chunk's in the shadow of this one's
@@ -811,7 +830,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 #pragma unroll
               for (int k = 0; k < NO; k++) o[k][e] = ov[k];
               // into the slot this chunk's inputs came from
-              if (j == 0) copy(av, af, slot, bytes);
+              if (j == 0) copy(av, af, slot, on);
             }
             // hand the boundary on (entry d; x entry 0 is not needed)
             const bool ox = xlast & ((i > 0) | (d0 > 0));
@@ -822,7 +841,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
 #pragma unroll
             for (int k = 0; k < NO; k++) chunk_store(op.out[k] + (ato + kDir * i * (Op::OS * 128)), o[k]);
           } else {
-            copy(av, af, slot, bytes);
+            copy(av, af, slot, on);
           }
           cp_async_commit();
         }
