@@ -12,9 +12,14 @@
 // a step has no memory access and no barrier in its dependent chain.  Warps hand
 // their boundary values on every four steps (a chunk), through rings in shared
 // memory within a block, and through mailboxes in global memory between blocks;
-// in both a word that holds no value holds a sentinel, so a value is its own
-// flag and no fence or barrier is involved (an mbarrier per ring entry cost ~400
-// cycles of a chunk's ~1100; divergent branches around the hand-off another ~400).  A block of 4 such warps sweeps a 16 x 8 column tile.
+// in both a word that holds no value holds a sentinel.  A value is then its own flag,
+// and so is its absence: a warp stores a value only into words in which it has read
+// the sentinel, so the accesses to each word order one another and no fence or barrier
+// is involved.  (An mbarrier per ring entry cost ~400 cycles of a chunk's ~1100;
+// divergent branches around the hand-off another ~400.  Separate words in which a
+// consumer says how far it is need a fence before them, and a fence waits for the
+// stores of the outputs: 256^3 mixed solve 175 ms, with the look at the words 128.)
+// A block of 4 such warps sweeps a 16 x 8 column tile.
 // Four steps per hand-off: the lag it adds (a chunk per warp crossed) costs less
 // than a wait per step would, and it is the largest number for which both
 // boundary offsets (8 and 4 columns) fall on whole chunks.
@@ -246,11 +251,6 @@ __device__ __forceinline__ unsigned long long ld_shared64(uint32_t p) {
   return v;
 }
 // stores to cluster addresses
-__device__ __forceinline__ void st_cluster(uint32_t p, int v, bool on) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %2, 0;\n @p st.relaxed.cluster.shared::cluster.s32 [%0], %1;\n}\n" ::"r"(p),
-               "r"(v), "r"((int)on)
-               : "memory");
-}
 __device__ __forceinline__ void st_cluster64(uint32_t p, unsigned long long v) {
   asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(p), "l"(v) : "memory");
 }
@@ -274,7 +274,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // Hand-off words (mailboxes and rings).  Every access is a strong operation, and
 // an empty word holds the sentinel, a NaN payload that arithmetic never produces:
 // a consumer that reads anything else has the value; it then writes the sentinel
-// back, which makes the word free for its producer's next value.
+// back, which makes the word free for its producer's next value: that is stored only
+// where the sentinel has been read (a mailbox entry takes one value in a launch).
 template <class T>
 struct Sentinel;
 template <>
@@ -416,6 +417,32 @@ __device__ __forceinline__ void ring_give(uint32_t p, const Quad<double>& q, boo
       : "memory");
 }
 
+// The words of a ring entry of a block of the cluster, and whether any holds a value
+// (not zero).
+struct RingWords {
+  uint32_t w[4];  // FP64: the high words
+  __device__ __forceinline__ uint32_t held(uint32_t sentinel) const {
+    return (w[0] ^ sentinel) | (w[1] ^ sentinel) | (w[2] ^ sentinel) | (w[3] ^ sentinel);
+  }
+};
+template <class T>
+__device__ __forceinline__ RingWords ring_look(uint32_t p) {
+  RingWords r;
+  if constexpr (sizeof(T) == 4) {
+    asm volatile("ld.relaxed.cluster.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3])
+                 : "r"(p)
+                 : "memory");
+  } else {
+    unsigned long long q[4];
+    asm volatile("ld.relaxed.cluster.shared::cluster.v2.u64 {%0, %1}, [%2];" : "=l"(q[0]), "=l"(q[1]) : "r"(p) : "memory");
+    asm volatile("ld.relaxed.cluster.shared::cluster.v2.u64 {%0, %1}, [%2];" : "=l"(q[2]), "=l"(q[3]) : "r"(p + 16) : "memory");
+#pragma unroll
+    for (int i = 0; i < 4; i++) r.w[i] = (uint32_t)(q[i] >> 32);
+  }
+  return r;
+}
+
 // ---- shared memory of a sweep block -----------------------------------------------
 constexpr int kSweepWarps = SweepLayout::kWarps;       // compute warps, 2 (x) by 2 (y)
 constexpr int kSweepThreads = (kSweepWarps + 4) * 32;  // + 2 x and 2 y mailbox loaders
@@ -433,8 +460,7 @@ struct SweepSmem {
   static constexpr int ringy = ringx + kSweepWarps * kRing * 16 * (int)sizeof(T);  // [warp][entry][8 columns][4]
   static constexpr int tick = ringy + kSweepWarps * kRing * 32 * (int)sizeof(T);  // u64 [kTick]
   static constexpr int acks = tick + kTick * 8;   // int [kTick]
-  static constexpr int prog = acks + kTick * 4;   // int [warp][x, y]: the consumers' progress
-  static constexpr int misc = prog + kSweepWarps * 8;  // abort flag, last flag
+  static constexpr int misc = acks + kTick * 4;  // abort flag, last flag
   static constexpr int sums = misc + 16;
   static constexpr int bytes = sums + kSweepThreads / 32 * 8;
   static_assert(bytes <= room, "a sweep block's shared memory");
@@ -539,7 +565,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   int* s_misc = reinterpret_cast<int*>(dyn + SM::misc);  // abort flag, last flag
   constexpr int kVec = 4 * (int)sizeof(T);  // bytes of a lane's ring entry
   const uint32_t ringx = smem_u32(dyn + SM::ringx), ringy = smem_u32(dyn + SM::ringy), s_tick = smem_u32(dyn + SM::tick),
-                 s_acks = smem_u32(dyn + SM::acks), s_prog = smem_u32(dyn + SM::prog);
+                 s_acks = smem_u32(dyn + SM::acks);
   const int rank = cluster_rank(), nrank = a.cx * a.cy, rkx = rank % a.cx, rky = rank / a.cx;
   const int leader = FWD ? 0 : nrank - 1;  // the block whose first warp draws the cluster's tickets
   for (int i = threadIdx.x; i < kSweepWarps * kRing * 12; i += blockDim.x) ring_store(ringx + i * kVec, sentinel_quad<T>());
@@ -561,7 +587,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     return (unsigned)(e.x * a.cx + lane % a.cx) | (unsigned)(e.y * a.cy + lane / a.cx) << 12 | b << 24;
   };
   // gives ticket n to the cluster's blocks, once all their warps have read the one
-  // that held its place (one warp of the leader)
+  // that held its place (one warp of the leader; a warp counts itself when the word it
+  // read has come back, so a later store cannot change what it read)
   auto publish = [&](int n, unsigned w) {
     const int need = n / kTick * (nrank * (kSweepThreads / 32));
     int spins = 0;
@@ -635,12 +662,6 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     const int dx = FWD ? 1 : -1, dy = FWD ? a.cx : -a.cx;  // rank of the next block along x and y, from this one's
     const uint32_t orx = cluster_addr(ringx + (nwx * kRing * 4 + ty) * kVec, inner_x || !cout_x ? rank : rank + dx),
                    ory = cluster_addr(ringy + (nwy * kRing * 8 + tx) * kVec, inner_y || !cout_y ? rank : rank + dy);
-    // Progress of the consumers: groups of four chunks they are done with, stored by them
-    // into the producer's words; this warp's go to its own producers' (prog_x, prog_y).
-    const uint32_t x_prog = s_prog + cw * 8, y_prog = x_prog + 4;
-    const uint32_t prog_x = cluster_addr(s_prog + nwx * 8, !inner_x || !cin_x ? rank : rank - dx),
-                   prog_y = cluster_addr(s_prog + nwy * 8 + 4, !inner_y || !cin_y ? rank : rank - dy);
-    const bool tell_x = lane == 0 && (!inner_x || cin_x), tell_y = lane == 0 && (!inner_y || cin_y);
     constexpr uint32_t kSlotX = 4 * kVec, kSlotY = 8 * kVec;
     const T* stage = reinterpret_cast<const T*>(dyn + SM::stage) + cw * D * NV * 128 + lane * kLane;
     const uint32_t stage_u32 = smem_u32(stage);
@@ -671,20 +692,25 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     if (publisher) {
       for (pub = 0; pub < 3;) advance_ticket(-1);
     }
-    int ahead = 0;          // groups of the next tile already being copied
-    int group = 0;          // running number of groups of four chunks; ring entries 4 * group ...
+    int ahead = 0;  // groups of the next tile already being copied
+    int group = 0;  // running number of groups of four chunks; ring entries 4 * group ...
+    // The words of four entries there, which the lanes look at together: 4 x 4 rows, 4 x 8
+    // columns.  held: some of the next group's held a value then, or nobody looked.
+    const bool rings_x = inner_x || cout_x, rings_y = inner_y || cout_y;
+    const uint32_t look_x = orx + (lane >> 3) * kSlotX + ((lane & 3) - ty) * kVec,
+                   look_y = ory + (lane >> 3) * kSlotY + ((lane & 7) - tx) * kVec;
+    constexpr uint32_t kEmpty = sizeof(T) == 8 ? (uint32_t)((unsigned long long)Sentinel<T>::bits >> 32) : (uint32_t)Sentinel<T>::bits;
+    bool held = true;
     for (int n = 0;; n++) {
       const unsigned tw = acquire(n);
       if (tw == kNoTile) break;
       Tile tl;
       pub = 0;
-      // done with everything before this tile
-      st_cluster(prog_x, group, tell_x);
-      st_cluster(prog_y, group, tell_y);
       if (!tile_of(tw, tl)) {
         if (publisher)
           while (pub < 3) advance_ticket(n);
         group += NG;
+        held = true;
         ahead = 0;
         continue;
       }
@@ -760,16 +786,6 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         const uint32_t rxa = rx + half * kSlotX, rxb = rx + (half ^ 4) * kSlotX, rya = ry + half * kSlotY,
                        ryb = ry + (half ^ 4) * kSlotY, oxa = orx + half * kSlotX, oya = ory + half * kSlotY;
         const int sbase = D == 8 ? (int)half : 0;  // stage slots sbase .. sbase + 3, then the others
-        // until the consumers are done with the group before the last, whose words these
-        // chunks' boundary values go to
-        if (feeds_x | feeds_y) {
-          int spins = 0;
-          for (;;) {
-            const int px = ld_shared(x_prog), py = ld_shared(y_prog);
-            if (__all_sync(kFull, (!feeds_x | (px >= group - 1)) & (!feeds_y | (py >= group - 1)))) break;
-            if (!__all_sync(kFull, W.more(spins, lim))) break;
-          }
-        }
         constexpr int kDir = FWD ? 1 : -1;
         const int64_t cg = chunk_at(c0, d0);
         const int64_t ato = cg * (Op::OS * 128) + lane * kLane;
@@ -797,6 +813,13 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           const int slot = (sbase + i) & (D - 1);
           const bool on = i < go.chunks;
           const int64_t av = fv + kDir * i * 128, af = ff + kDir * i * (Op::FS * 128);
+          // in the last chunk, what the next group's entries hold: their consumers took the
+          // values about three chunks ago, unless they are late
+          RingWords nx{}, ny{};
+          if (i == 3) {
+            nx = ring_look<T>(look_x + (half ^ 4) * kSlotX);
+            ny = ring_look<T>(look_y + (half ^ 4) * kSlotY);
+          }
           if (live) {
             // the neighbours' boundary values, x entry d + 2 and y entry d + 1, and this
             // chunk's inputs.  (Fetching the next chunk's in the shadow of this one's
@@ -832,6 +855,16 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
               // into the slot this chunk's inputs came from
               if (j == 0) copy(av, af, slot, on);
             }
+            // until the words that this group's boundary values go to are empty
+            if (i == 0 && held) {
+              for (int spins = 0;;) {
+                const uint32_t hx = ring_look<T>(look_x + half * kSlotX).held(kEmpty),
+                               hy = ring_look<T>(look_y + half * kSlotY).held(kEmpty);
+                if (!__any_sync(kFull, (feeds_x & (hx != 0)) | (feeds_y & (hy != 0)))) break;
+                if (!__all_sync(kFull, W.more(spins, lim))) break;
+              }
+              __syncwarp();  // one lane looked, another one stores
+            }
             // hand the boundary on (entry d; x entry 0 is not needed)
             const bool ox = xlast & ((i > 0) | (d0 > 0));
             ring_give(oxa + i * kSlotX, val, ox & feeds_x);
@@ -843,13 +876,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           } else {
             copy(av, af, slot, on);
           }
+          if (i == 3) held = __any_sync(kFull, ((rings_x & (nx.held(kEmpty) != 0)) | (rings_y & (ny.held(kEmpty) != 0))));
           cp_async_commit();
         }
         group++;
         half ^= 4;
         __syncwarp();
-        st_cluster(prog_x, group, tell_x);
-        st_cluster(prog_y, group, tell_y);
       };
       for (int gi = 0; gi < NG; gi++) {
         if (4 * gi + 3 < NC - 2)
