@@ -1038,6 +1038,10 @@ PcgSolver::PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt
   sweep_set_attr<float, true, FwdEisenstatOp<float>>();
   nblocks_ = ctx->sm_count * 8;
   const int ntiles = sg_.ntiles();
+  if ((int64_t)sg_.ntx * sg_.nty > kMaxTiles) {
+    init_status_ = -3;
+    return;
+  }
   auto alloc = [&](size_t bytes) -> void* {
     void* p = nullptr;
     if (cudaMalloc(&p, bytes) != cudaSuccess) return nullptr;

@@ -221,6 +221,21 @@ struct SweepArgs {
 };
 constexpr int kMaxCluster = 16;  // blocks of a cluster (the stride of SweepArgs::bits)
 constexpr int kTileSwept = 16;
+
+// A block's ticket word: the number of its tile (Y * ntx + X) and the tile's bits above
+// it; kNoTile: no more tiles.  A grid has at most kMaxTiles tiles, so that their columns
+// have 32-bit numbers (a tile takes over 200 KB of a solver's arrays: these are
+// exhausted long before).
+constexpr int kTileBits = 27;
+constexpr int kMaxTiles = (1 << 24) - 1;
+constexpr unsigned kNoTile = 0xffffffffu;
+// the word of block `rank` of a cluster at `unit`
+__host__ __device__ __forceinline__ unsigned ticket_pack(const SweepLayout& g, int cx, int cy, int2 unit, int rank, unsigned bits) {
+  const int X = unit.x * cx + rank % cx, Y = unit.y * cy + rank / cx;
+  return (bits ? (unsigned)(Y * g.ntx + X) : 0u) | bits << kTileBits;  // a tile that is not swept may lie outside the grid
+}
+__host__ __device__ __forceinline__ int ticket_tile(unsigned w) { return (int)(w & ((1u << kTileBits) - 1)); }
+__host__ __device__ __forceinline__ int ticket_bits(unsigned w) { return (int)(w >> kTileBits); }
 inline int64_t sweep_mbx_elems(const SweepLayout& g) { return (int64_t)g.nc * SweepLayout::TY * 4; }  // per tile
 inline int64_t sweep_mby_elems(const SweepLayout& g) { return (int64_t)g.nc * SweepLayout::TX * 4; }
 
@@ -576,15 +591,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
   cluster_sync();
   const SweepWait W{a.sc, smem_u32(s_misc), spin_limit > 0 ? spin_limit : kSpinLimit};
   const int lim = W.limit > (1 << 28) ? (1 << 30) : 4 * W.limit;  // waits behind the mailbox loaders' own bound
-  // A block's ticket word: its tile X | Y << 12 | the tile's bits << 24, and the ticket's
-  // running number + 1 above; kNoTile: no more.
-  constexpr unsigned kNoTile = 0xffffffffu;
+  // (in shared memory the ticket's running number + 1 stands above the word)
   auto ticket_word = [&](int t) -> unsigned {  // lane r: the word of rank r
     if (t >= nticket || lane >= nrank) return kNoTile;
     const int at = FWD ? t : nticket - 1 - t;
     const int2 e = a.order[at];
-    const unsigned b = a.bits[at * kMaxCluster + lane];
-    return (unsigned)(e.x * a.cx + lane % a.cx) | (unsigned)(e.y * a.cy + lane / a.cx) << 12 | b << 24;
+    return ticket_pack(g, a.cx, a.cy, e, lane, a.bits[(int64_t)at * kMaxCluster + lane]);
   };
   // gives ticket n to the cluster's blocks, once all their warps have read the one
   // that held its place (one warp of the leader; a warp counts itself when the word it
@@ -615,13 +627,12 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
     return ok ? w : kNoTile;
   };
   struct Tile {
-    int X, Y, nb;
+    int id, nb;
   };
   // this block's tile: false if it is not swept
   auto tile_of = [&](unsigned w, Tile& t) -> bool {
-    t.X = (int)(w & 0xfff);
-    t.Y = (int)(w >> 12 & 0xfff);
-    t.nb = (int)(w >> 24);
+    t.id = ticket_tile(w);
+    t.nb = ticket_bits(w);
     return t.nb & kTileSwept;
   };
   const int first = FWD ? 0 : kSweepWarps - 1;  // the compute warp that starts a tile's wave
@@ -641,7 +652,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
       if (w == kNoTile) break;
       Tile tl;
       if (!tile_of(w, tl)) continue;
-      const int tid = tl.Y * g.ntx + tl.X;
+      const int tid = tl.id;
       if (isx) {
         if ((tl.nb & (FWD ? 1 : 2)) && !cin_x)  // entry 0 is not needed
           sweep_loader<T, 4>(W, (T*)a.mbx + (int64_t)tid * NC * 32 + l * 16, 32, 1, NC, ringx + cw * kRing * 4 * kVec, e0);
@@ -714,8 +725,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         ahead = 0;
         continue;
       }
-      const int nb = tl.nb, tid = tl.Y * g.ntx + tl.X;
-      const int64_t c0 = (int64_t)(tid * kSweepWarps + cw) * NC;
+      const int nb = tl.nb, tid = tl.id;
+      const int64_t c0 = ((int64_t)tid * kSweepWarps + cw) * NC;
       auto chunk_at = [&](int64_t first_chunk, int d) { return first_chunk + (FWD ? d : NC - 1 - d); };
       // the first groups, as far as they are not on their way
       const bool late = ahead < min(DG, NG);
@@ -799,7 +810,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           if (peek(n + 1, w)) {
             next_known = true;
             Tile t1;
-            if (w != kNoTile && tile_of(w, t1)) nc0 = (int64_t)((t1.Y * g.ntx + t1.X) * kSweepWarps + cw) * NC;
+            if (w != kNoTile && tile_of(w, t1)) nc0 = ((int64_t)t1.id * kSweepWarps + cw) * NC;
           }
         }
         const SweepAhead go = sweep_ahead(gi, NC, DG, ahead, nc0 >= 0);
@@ -902,8 +913,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           a.col_sums[(tid * kSweepWarps + cw) * 32 + lane] = acc;
           __threadfence();
           __syncwarp();
-          const int X2 = tl.X >> 1, t32 = tl.Y * ((g.ntx + 1) >> 1) + X2;
-          const bool other = nb & (tl.X & 1 ? 1 : 2);  // the other tile of the pair is swept
+          const int Y = tid / g.ntx, X = tid - Y * g.ntx, X2 = X >> 1, t32 = Y * ((g.ntx + 1) >> 1) + X2;
+          const bool other = nb & (X & 1 ? 1 : 2);  // the other tile of the pair is swept
           int done = 0;
           if (lane == 0) done = atomicAdd(&a.t32_count[t32], 1) + 1;
           if (__shfl_sync(kFull, done, 0) == (other ? 2 : 1) * kSweepWarps) {
@@ -912,7 +923,7 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
             const int Xl = X2 * 2 + (lane >> 4);
 #pragma unroll
             for (int r = 0; r < 8; r++)
-              c[r] = Xl < g.ntx ? __ldcg(&a.col_sums[((tl.Y * g.ntx + Xl) * kSweepWarps + (r >> 2) * 2 + ((lane >> 3) & 1)) * 32 +
+              c[r] = Xl < g.ntx ? __ldcg(&a.col_sums[((Y * g.ntx + Xl) * kSweepWarps + (r >> 2) * 2 + ((lane >> 3) & 1)) * 32 +
                                                      (r & 3) * 8 + (lane & 7)])
                                 : 0.0;
 #pragma unroll
