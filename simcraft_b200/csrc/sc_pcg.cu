@@ -909,11 +909,7 @@ void all_units_order(int ntx, int nyu, int2* o) {
   int n = 0;
   o[n++] = make_int2(ntx * nyu, 0);
   for (int d = 0; d <= ntx + nyu - 2; d++)
-    for (int X = 0; X < ntx; X++) {
-      const int Y = d - X;
-      if (Y < 0 || Y >= nyu) continue;
-      o[n++] = make_int2(X, Y);
-    }
+    for (int X = std::max(0, d - nyu + 1); X <= std::min(d, ntx - 1); X++) o[n++] = make_int2(X, d - X);
 }
 std::vector<int2> all_units_order(int ntx, int nyu) {
   std::vector<int2> o((size_t)ntx * nyu + 1);
