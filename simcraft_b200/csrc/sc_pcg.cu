@@ -1319,8 +1319,23 @@ int PcgSolver::download_pressure(double* pg, bool device) {
   return check_dev_error("download_pressure");
 }
 
+// The matrix in FP32, which only the FP32 SpMV reads (the inner PCG of the mixed solve,
+// not the Eisenstat iteration): made when it is first needed for a system, since the
+// inner method may change between two solves of the same one.
+void PcgSolver::ensure_matrix32() {
+  if (matrix32_valid_) return;
+  k_sweep_matrix32<<<grid_for(sg_.total / 4, ctx_->sm_count), kThreads, 0, ctx_->stream>>>(sg_, d64_.adiag, d64_.al, d64_.ad,
+                                                                                           d64_.ab, d32_);
+  launches_ += 1;
+  matrix32_valid_ = true;
+}
+
 int PcgSolver::ensure_pivots() {
-  if (pivots_valid_) return 0;
+  const bool wants_matrix32 = opt_.precision == PREC_MIXED && opt_.inner_method != INNER_EISENSTAT;
+  if (pivots_valid_) {
+    if (wants_matrix32) ensure_matrix32();
+    return 0;
+  }
   cudaStream_t st = ctx_->stream;
   const int grid = grid_for(g_.total, ctx_->sm_count), sgrid = grid_for(sg_.total / 4, ctx_->sm_count);
   // the pivot sweep reports a timeout through the status word: start it clean,
@@ -1375,11 +1390,9 @@ int PcgSolver::ensure_pivots() {
     }
     k_sweep_factor<float><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d32_);
     launches_ += 1;
-    if (opt_.inner_method != INNER_EISENSTAT) {
-      k_sweep_matrix32<<<sgrid, kThreads, 0, st>>>(sg_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, d32_);
-      launches_ += 1;
-    }
   }
+  matrix32_valid_ = false;
+  if (wants_matrix32) ensure_matrix32();
   select_active_tiles();
   int e = check_dev_error("pivots");
   if (e) return e;
@@ -1860,6 +1873,7 @@ int PcgSolver::time_kernels(int reps, double* ms) {
   // is FP64 in both).
   const bool f32 = opt_.precision == PREC_MIXED && have_f32_;
   if (f32) {
+    ensure_matrix32();
     k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d32_.r, d32_.p, partials_, sc_);
     cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
     k_copy<float><<<grid, kThreads, 0, s>>>(sg_, order_act_, d32_.r, d32_.s, sc_);

@@ -189,6 +189,7 @@ class PcgSolver {
 
  private:
   int ensure_pivots();
+  void ensure_matrix32();
   // eis: Eisenstat iteration (FP32 inner solve of the mixed path only)
   template <class T>
   int run_pcg(SysArrays<T>& A, double tol, int criterion, int max_iter, bool scale_rhs,
@@ -228,6 +229,7 @@ class PcgSolver {
   int init_status_ = 0;
   bool pivots_valid_ = false;
   bool have_f32_ = false;
+  bool matrix32_valid_ = false;  // the FP32 matrix is that of the pivots
   int nblocks_ = 0;     // elementwise grid
   SysArrays<double> d64_;
   SysArrays<float> d32_;

@@ -1,0 +1,36 @@
+"""A resident system under changing calls: the inner method of the mixed solve switched
+between two solves of the same system."""
+import numpy as np
+import pytest
+
+from test_sweep_rings_gpu import _system
+
+pytestmark = pytest.mark.gpu
+
+INNER_PCG, INNER_EISENSTAT = 0, 1
+
+
+@pytest.mark.parametrize("order", [(INNER_EISENSTAT, INNER_PCG), (INNER_PCG, INNER_EISENSTAT, INNER_PCG)])
+def test_the_inner_method_may_change_between_solves(gpu, order):
+    from simcraft_b200.solver import CRIT_REL_L2, PREC_MIXED, CgSolver3D
+
+    dims = (40, 24, 30)
+    solver = None
+    for seed in (11, 12):  # a second system in the same handle: nothing of the first may stay
+        adiag, an, act = _system(dims, False, seed)
+        b = np.random.default_rng(seed + 50).uniform(-1, 1, dims) * act
+        opts = dict(tol=1e-10, max_iter=400, criterion=CRIT_REL_L2, precision=PREC_MIXED)
+        if solver is None:
+            solver = CgSolver3D(*dims, inner_method=order[0], **opts)
+        solver.set_options(inner_method=order[0])
+        solver.upload(adiag, an, b, act)
+        for method in order:
+            solver.set_options(inner_method=method)
+            fresh = CgSolver3D(*dims, inner_method=method, **opts)
+            fresh.upload(adiag, an, b, act)
+            p = []
+            for s in (fresh, solver):
+                st = s.solve_resident()
+                assert st["status"] == 1 and st["true_rel_l2"] < 2e-10
+                p.append(s.download(np.zeros(dims)))
+            np.testing.assert_array_equal(p[1], p[0])
