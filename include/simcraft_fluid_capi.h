@@ -165,7 +165,7 @@ int sc_pcg_download(sc_pcg* pcg, double* pg, int device_pointer);
  * uploaded to `pcg`; r and z are device pointers in the reference layout. */
 int sc_pcg_precond_device(sc_pcg* pcg, const double* r, double* z);
 /* applyCompressedMatrix (project-solver.cc:16-39) on the uploaded system:
- * b = A x, device pointers. */
+ * b = A x, device pointers; x and b may overlap. */
 int sc_pcg_apply_device(sc_pcg* pcg, const double* x, double* b);
 
 /* Per-kernel device time of the solver's kernels on the uploaded system (each

@@ -1845,7 +1845,17 @@ int PcgSolver::precond_only(const double* r, double* z) {
 int PcgSolver::apply_only(const double* x, double* b) {
   cudaStream_t s = ctx_->stream;
   const int grid = grid_for(g_.total, ctx_->sm_count);
+  // A row reads its neighbours' x while other blocks write b, so overlapping x and b go
+  // through a copy, in an array whose values no call keeps (and whose padding is zero).
+  const size_t bytes = sizeof(double) * (size_t)g_.nx * g_.ny * g_.nz;
+  const uintptr_t xa = (uintptr_t)x, ba = (uintptr_t)b;
+  const bool overlap = xa < ba + bytes && ba < xa + bytes;
+  if (overlap) {
+    cudaMemcpyAsync(d64_.Az, x, bytes, cudaMemcpyDeviceToDevice, s);
+    x = d64_.Az;
+  }
   k_apply_checked<<<grid, kThreads, 0, s>>>(g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, x, b);
+  if (overlap) cudaMemsetAsync(d64_.Az, 0, bytes, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("apply");
   return check_dev_error("apply");
 }

@@ -1,5 +1,5 @@
 """A resident system under changing calls: the inner method of the mixed solve switched
-between two solves of the same system."""
+between two solves of the same system, and the matrix applied in place."""
 import numpy as np
 import pytest
 
@@ -34,3 +34,30 @@ def test_the_inner_method_may_change_between_solves(gpu, order):
                 assert st["status"] == 1 and st["true_rel_l2"] < 2e-10
                 p.append(s.download(np.zeros(dims)))
             np.testing.assert_array_equal(p[1], p[0])
+
+
+@pytest.mark.parametrize("dims", [(1, 1, 1), (33, 17, 9), (96, 64, 80)])
+@pytest.mark.parametrize("shift", [0, 1, 777, -1, -777])
+def test_apply_to_overlapping_vectors(gpu, dims, shift):
+    import torch
+    from simcraft_b200.solver import CRIT_REL_L2, CgSolver3D
+
+    adiag, an, act = _system(dims, False, 13)
+    n = int(np.prod(dims))
+    rhs = np.random.default_rng(14).uniform(-1, 1, dims) * act
+    s = CgSolver3D(*dims, tol=1e-10, max_iter=400, criterion=CRIT_REL_L2)
+    s.upload(adiag, an, rhs, act)
+    x = torch.from_numpy(np.random.default_rng(15).uniform(-1, 1, dims)).cuda()
+    ref = torch.empty_like(x)
+    s.apply(x, ref)
+    s.solve_resident()
+    before = s.download(np.zeros(dims))
+    buf = torch.zeros(n + 800, dtype=torch.float64, device="cuda")
+    at = max(0, -shift)
+    xv, bv = buf[at:at + n].view(dims), buf[at + shift:at + shift + n].view(dims)
+    for _ in range(5):
+        xv.copy_(x)
+        s.apply(xv, bv)
+        assert torch.equal(bv, ref)
+    s.solve_resident()  # the solver's own arrays are as they were
+    np.testing.assert_array_equal(s.download(np.zeros(dims)), before)
