@@ -1563,12 +1563,13 @@ int PcgSolver::solve_fp64(PcgStats* st) {
   int e = ensure_pivots();
   if (e) return e;
   e = run_pcg<double>(d64_, opt_.tol, opt_.criterion, opt_.max_iter, false, st);
-  if (e == 0 && (last_.err & DEV_ERR_NONFINITE))
-    return ctx_->set_error(-8, "pcg: NaN or Inf in the system or the right-hand side");
-  if (e) return e;
+  // the iterate is handed back whatever came of it: after an error the pressure is that
+  // of the failed solve, never an earlier one's
   k_sweep_to_tiled<double><<<grid_for(g_.total, ctx_->sm_count), kThreads, 0, ctx_->stream>>>(sg_, g_, d64_.p, press_);
   launches_ += 1;
-  return check_dev_error("pcg");
+  if (e == 0 && (last_.err & DEV_ERR_NONFINITE))
+    return ctx_->set_error(-8, "pcg: NaN or Inf in the system or the right-hand side");
+  return e ? e : check_dev_error("pcg");
 }
 
 // Mixed precision with reliable updates: FP32 CG on the split system

@@ -1,5 +1,6 @@
 """A resident system under changing calls: the inner method of the mixed solve switched
-between two solves of the same system, and the matrix applied in place."""
+between two solves of the same system, the matrix applied in place, and the pressure
+after a solve that failed."""
 import numpy as np
 import pytest
 
@@ -61,3 +62,28 @@ def test_apply_to_overlapping_vectors(gpu, dims, shift):
         assert torch.equal(bv, ref)
     s.solve_resident()  # the solver's own arrays are as they were
     np.testing.assert_array_equal(s.download(np.zeros(dims)), before)
+
+
+def test_after_a_failed_solve_the_pressure_is_not_the_previous_one(gpu):
+    """A right-hand side with an infinite value: the solve fails at its first residual with
+    p = 0, and that is what a download gives."""
+    from simcraft_b200._capi import CapiError
+    from simcraft_b200.solver import CRIT_REL_L2, CgSolver3D
+
+    dims = (24, 20, 18)
+    adiag, an, act = _system(dims, False, 16)
+    rhs = np.random.default_rng(17).uniform(-1, 1, dims) * act
+    s = CgSolver3D(*dims, tol=1e-10, max_iter=400, criterion=CRIT_REL_L2)
+    s.upload(adiag, an, rhs, act)
+    s.solve_resident()
+    good = s.download(np.zeros(dims))
+    assert np.abs(good).max() > 0.0
+    bad = rhs.copy()
+    bad[tuple(np.argwhere(act)[act.sum() // 2])] = np.inf
+    s.upload(adiag, an, bad, act)
+    with pytest.raises(CapiError):
+        s.solve_resident()
+    np.testing.assert_array_equal(s.download(np.full(dims, 7.0)), np.zeros(dims))
+    s.upload(adiag, an, rhs, act)
+    s.solve_resident()
+    np.testing.assert_array_equal(s.download(np.zeros(dims)), good)
