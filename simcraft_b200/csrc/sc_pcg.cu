@@ -590,33 +590,6 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// Entries that couple to an inactive cell, and whole inactive rows, are never
-// read by applyCompressedMatrix (it tests the neighbour's activity first).  The
-// PCG kernels multiply them by zeros instead of testing, so any non-finite
-// value there is replaced by 0 before the solve; finite values stay as given.
-__global__ void __launch_bounds__(kThreads)
-    k_mask_system(Tiled g, const uint8_t* __restrict__ act, double* __restrict__ adiag,
-                  double* __restrict__ al, double* __restrict__ ad, double* __restrict__ ab) {
-  auto fix = [](double* a, int64_t e) {
-    if (!isfinite(a[e])) a[e] = 0.0;
-  };
-  SC_ROWBLOCK_LOOP(g) {
-    Cell c;
-    c.init(g, rb, threadIdx.x);
-    const int64_t e = c.e;
-    if (!(c.inside && act[e])) {
-      fix(adiag, e);
-      fix(al, e);
-      fix(ad, e);
-      fix(ab, e);
-      continue;
-    }
-    if (c.x == 0 || !act[c.xm(g)]) fix(al, e);
-    if (c.y == 0 || !act[c.ym(g)]) fix(ad, e);
-    if (c.z == 0 || !act[c.zm(g)]) fix(ab, e);
-  }
-}
-
 // saxpy(pg, s, alpha); saxpy(r, z, -alpha); residual (:332-335, util.cc:394-402).
 // s and Az are zero on inactive cells, so the masked updates of the reference
 // are the plain updates here.
@@ -673,9 +646,26 @@ __global__ void __launch_bounds__(kThreads)
 // of the pivot recurrence (project-solver.cc:244-265).  For the Left term these are
 //   tau*A_L(p)*A_L(p-x+y) [if p-x+y active] + tau*A_L(p)*A_L(p-x+z) [if p-x+z active]
 // and likewise for Down and Back; they only depend on A.  PivotOp uses a
-// neighbour's terms only where that neighbour's pivot is not zero.  tile_act
-// (optional, zero on entry): 1 for the tiles holding an active cell.
-__global__ void __launch_bounds__(kThreads)
+// neighbour's terms only where that neighbour's pivot is not zero.  A coupling in
+// these products may itself lead to an inactive cell; a non-finite one then counts
+// as zero, a finite one as it is given.  tile_act (optional, zero on entry): 1 for
+// the tiles holding an active cell.
+// A thread has four cells of a column and reads them and the six columns around from
+// each column's own base, all loads before they are used: testing each cell's activity
+// first and looking up every element by its coordinates took 984 us at 256^3 (134 at
+// 128^3), and a pass over the Tiled arrays that cleared the non-finite entries before
+// that another 385 (57); now 530 (64) and none.
+struct TiledColumn {
+  int64_t base;
+  int skew, nz;  // slot of z: (z + skew) mod nz
+  __device__ __forceinline__ TiledColumn(const Tiled& g, int x, int y)
+      : base(g.tile_base(x >> 5, y / Tiled::TY) + (y % Tiled::TY) * 32 + (x & 31)), skew((x & 31) % g.nz), nz(g.nz) {}
+  __device__ __forceinline__ int64_t at(int z) const {  // z is moved into the grid
+    const int s = min(max(z, 0), nz - 1) + skew;
+    return base + (int64_t)(s >= nz ? s - nz : s) * (Tiled::TY * 32);
+  }
+};
+__global__ void __launch_bounds__(kThreads, 2)
     k_sweep_system(SweepLayout g, Tiled tg, const double* __restrict__ adiag, const double* __restrict__ al,
                    const double* __restrict__ ad, const double* __restrict__ ab, const uint8_t* __restrict__ act,
                    double tau, double* __restrict__ o_d, double* __restrict__ o_l, double* __restrict__ o_dn,
@@ -685,48 +675,53 @@ __global__ void __launch_bounds__(kThreads)
     const ChunkPos c = chunk_pos<double>(g, i);
     double v[7][4] = {};
     bool any = false;
+    if (c.inside && c.z0 + 3 >= 0 && c.z0 < g.nz) {
+      const int x = c.x, y = c.y, z0 = c.z0;
+      const bool hl = x > 0, hr = x < g.nx - 1, hd = y > 0, hu = y < g.ny - 1;
+      // the cell's column and those around (the cell's own where there is none)
+      const TiledColumn C(tg, x, y), L(tg, x - hl, y), R(tg, x + hr, y), D(tg, x, y - hd), U(tg, x, y + hu),
+          LU(tg, x - (hl && hu), y + (hl && hu)), RD(tg, x + (hr && hd), y - (hr && hd));
+      // bit j of a column: its cell at z0 - 1 + j is active
+      auto active = [&](const TiledColumn& t, bool there, int from, int to) {
+        unsigned bits = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int x = c.x, y = c.y, z = c.z0 + j;
-      if (!c.inside || z < 0 || z >= g.nz) continue;
-      const int64_t e = tg.off(x, y, z);
-      if (!act[e]) continue;
-      any = true;
-      v[0][j] = adiag[e];
-      if (x > 0 && act[tg.off(x - 1, y, z)]) {
-        const double a = al[e];
-        v[1][j] = a;
-        if (y < g.ny - 1) {
-          const int64_t o = tg.off(x - 1, y + 1, z);
-          if (act[o]) v[4][j] += tau * a * al[o];
+        for (int j = 0; j < 6; j++)
+          if (j >= from && j <= to) bits |= (unsigned)(act[t.at(z0 - 1 + j)] != 0) << j;
+        const unsigned in = 0x3fu & (z0 >= 1 ? ~0u : ~0u << (1 - z0)) & (z0 + 4 < g.nz ? ~0u : (1u << (g.nz - z0 + 1)) - 1u);
+        return there ? bits & in : 0u;
+      };
+      const unsigned aC = active(C, true, 0, 4), aL = active(L, hl, 1, 5), aLU = active(LU, hl && hu, 1, 4),
+                     aD = active(D, hd, 1, 5), aRD = active(RD, hr && hd, 1, 4), aR = active(R, hr, 0, 3),
+                     aU = active(U, hu, 0, 3);
+      any = (aC & 0x1eu) != 0;
+      // a coupling that leads to cell (xn, yn, zn)
+      auto to_cell = [&](double a, int xn, int yn, int zn) {
+        if (isfinite(a)) return a;
+        return xn >= 0 && yn >= 0 && zn >= 0 && act[tg.off(xn, yn, zn)] ? a : 0.0;
+      };
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int z = z0 + j;
+        const int64_t e = C.at(z), eLz = L.at(z + 1), eDz = D.at(z + 1);
+        const double d = adiag[e], l = al[e], dn = ad[e], b = ab[e];
+        const double l1 = al[LU.at(z)], l2 = al[eLz], d1 = ad[RD.at(z)], d2 = ad[eDz], b1 = ab[R.at(z - 1)], b2 = ab[U.at(z - 1)];
+        auto on = [&](unsigned bits, int at) { return (bits >> (j + 1 + at) & 1u) != 0; };
+        if (!on(aC, 0)) continue;
+        v[0][j] = d;
+        if (on(aL, 0)) {
+          v[1][j] = l;
+          if (on(aLU, 0)) v[4][j] += tau * l * to_cell(l1, x - 2, y + 1, z);
+          if (on(aL, 1)) v[4][j] += tau * l * to_cell(l2, x - 2, y, z + 1);
         }
-        if (z < g.nz - 1) {
-          const int64_t o = tg.off(x - 1, y, z + 1);
-          if (act[o]) v[4][j] += tau * a * al[o];
+        if (on(aD, 0)) {
+          v[2][j] = dn;
+          if (on(aRD, 0)) v[5][j] += tau * dn * to_cell(d1, x + 1, y - 2, z);
+          if (on(aD, 1)) v[5][j] += tau * dn * to_cell(d2, x, y - 2, z + 1);
         }
-      }
-      if (y > 0 && act[tg.off(x, y - 1, z)]) {
-        const double a = ad[e];
-        v[2][j] = a;
-        if (x < g.nx - 1) {
-          const int64_t o = tg.off(x + 1, y - 1, z);
-          if (act[o]) v[5][j] += tau * a * ad[o];
-        }
-        if (z < g.nz - 1) {
-          const int64_t o = tg.off(x, y - 1, z + 1);
-          if (act[o]) v[5][j] += tau * a * ad[o];
-        }
-      }
-      if (z > 0 && act[tg.off(x, y, z - 1)]) {
-        const double a = ab[e];
-        v[3][j] = a;
-        if (x < g.nx - 1) {
-          const int64_t o = tg.off(x + 1, y, z - 1);
-          if (act[o]) v[6][j] += tau * a * ab[o];
-        }
-        if (y < g.ny - 1) {
-          const int64_t o = tg.off(x, y + 1, z - 1);
-          if (act[o]) v[6][j] += tau * a * ab[o];
+        if (on(aC, -1)) {
+          v[3][j] = b;
+          if (on(aR, -1)) v[6][j] += tau * b * to_cell(b1, x + 1, y, z - 2);
+          if (on(aU, -1)) v[6][j] += tau * b * to_cell(b2, x, y + 1, z - 2);
         }
       }
     }
@@ -857,11 +852,25 @@ __host__ __device__ void tile_bits(int2 u, int cx, int cy, Swept swept, uint8_t*
 // order; a unit is cx by cy tiles) that hold an active tile, in the same order, and
 // their count in the header entry dst[-1].  Optional: per entry the bits of its tiles
 // (SweepArgs::bits), and zeros for the dot-product shares of tiles that are not swept
-// (nothing writes those meanwhile).  One block.
-__global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, int cx, int cy,
-                                                        const uint8_t* __restrict__ tile_act,
-                                                        const int2* __restrict__ all, int n, int2* __restrict__ dst,
-                                                        uint8_t* __restrict__ bits, double* __restrict__ tile_partials) {
+// (nothing writes those meanwhile).  A block per list.
+struct OrderList {
+  int cx, cy;
+  const int2* all;
+  int n;
+  int2* dst;
+  uint8_t* bits;
+  double* tile_partials;
+};
+struct OrderLists {
+  OrderList l[3];
+};
+__global__ void __launch_bounds__(1024) k_compact_order(int ntx, int nty, const uint8_t* __restrict__ tile_act, OrderLists lists) {
+  const OrderList& o = lists.l[blockIdx.x];
+  const int cx = o.cx, cy = o.cy, n = o.n;
+  const int2* const all = o.all;
+  int2* const dst = o.dst;
+  uint8_t* const bits = o.bits;
+  double* const tile_partials = o.tile_partials;
   __shared__ int wsum[32];
   __shared__ int carry;
   if (threadIdx.x == 0) carry = 0;
@@ -1337,20 +1346,19 @@ int PcgSolver::ensure_pivots() {
     return 0;
   }
   cudaStream_t st = ctx_->stream;
-  const int grid = grid_for(g_.total, ctx_->sm_count), sgrid = grid_for(sg_.total / 4, ctx_->sm_count);
+  const int sgrid = grid_for(sg_.total / 4, ctx_->sm_count);
   // the pivot sweep reports a timeout through the status word: start it clean,
   // with this context's wait bound
   cudaMemsetAsync(&sc_->err, 0, sizeof(unsigned), st);
   pivot_limit_ = spin_limit();
   cudaMemcpyAsync(&sc_->spin_limit, &pivot_limit_, sizeof(int), cudaMemcpyHostToDevice, st);
-  k_mask_system<<<grid, kThreads, 0, st>>>(g_, active_, t_adiag_, t_al_, t_ad_, t_ab_);
   // z, q and Az hold the pivots' neighbour products until select_active_tiles clears them
   cudaMemsetAsync(tile_act_, 0, (size_t)sg_.ntiles(), st);
   k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg_, g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, opt_.tau, d64_.adiag,
                                              d64_.al, d64_.ad, d64_.ab, d64_.z, d64_.q, d64_.Az, tile_act_);
   sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(d64_, opt_.sigma), st);
   k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d64_);
-  launches_ += 4;
+  launches_ += 3;
   {
     // the solve's scalars are set over the status word next: read it first
     unsigned* herr = reinterpret_cast<unsigned*>(sc_host_ + 1);
@@ -1410,14 +1418,12 @@ void PcgSolver::select_active_tiles() {
 #if !SC_SKIP_EMPTY_TILES
   cudaMemsetAsync(tile_act_, 1, (size_t)ntiles, st);  // every tile swept
 #endif
-  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 1, 1, tile_act_, order_all_, ntiles, order_act_, nullptr,
-                                      tile_partials_);
   const int ncx = (sg_.ntx + cl_x_ - 1) / cl_x_, ncy = (sg_.nty + cl_y_ - 1) / cl_y_;
-  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, cl_x_, cl_y_, tile_act_, order_cl_all_, ncx * ncy, order_cl_act_,
-                                      bits_act_, nullptr);
-  k_compact_order<<<1, 1024, 0, st>>>(sg_.ntx, sg_.nty, 2, 1, tile_act_, order_t32_all_, g_.ntiles(), order_t32_act_, nullptr,
-                                      nullptr);
-  launches_ += 3;
+  const OrderLists lists{{{1, 1, order_all_, ntiles, order_act_, nullptr, tile_partials_},
+                          {cl_x_, cl_y_, order_cl_all_, ncx * ncy, order_cl_act_, bits_act_, nullptr},
+                          {2, 1, order_t32_all_, g_.ntiles(), order_t32_act_, nullptr, nullptr}}};
+  k_compact_order<<<3, 1024, 0, st>>>(sg_.ntx, sg_.nty, tile_act_, lists);
+  launches_ += 1;
   // columns of tiles that are not swept add zeros
   cudaMemsetAsync(col_sums_, 0, sizeof(double) * (size_t)ntiles * kSweepWarps * 32, st);
   cudaMemsetAsync(t32_sums_, 0, sizeof(double) * (size_t)g_.ntiles(), st);
@@ -2099,16 +2105,15 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   const std::vector<uint8_t> hbits = all_tile_bits(sg, 1, 1, ord);
   if (failed(cudaMemcpyAsync(bits, hbits.data(), hbits.size(), cudaMemcpyHostToDevice, st), "uploading the tile bits"))
     return -2;
-  // system and right-hand side into the tiled layout, then the entries the
-  // reference never reads (couplings to inactive cells, inactive rows) cleared
-  // of non-finite values, as the allocating entry point does
+  // system into the tiled layout and from there into the sweeps', where the entries
+  // the reference never reads (couplings to inactive cells, inactive rows) are zero;
+  // right-hand side
   const int grid = grid_for(g.total, sm_count);
   k_to_tiled<uint8_t, uint8_t><<<grid, kThreads, 0, st>>>(g, active, act, nullptr);
   k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, adiag, tl[0], nullptr);
   k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[0], tl[1], nullptr);
   k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[3], tl[2], nullptr);
   k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[5], tl[3], nullptr);
-  k_mask_system<<<grid, kThreads, 0, st>>>(g, act, tl[0], tl[1], tl[2], tl[3]);
   const int sgrid = grid_for(sg.total / 4, sm_count);
   k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg, g, tl[0], tl[1], tl[2], tl[3], act, tau, A.adiag, A.al, A.ad, A.ab, A.z,
                                              A.q, A.Az, nullptr);
