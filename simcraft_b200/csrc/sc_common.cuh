@@ -33,15 +33,7 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// Global-memory accessors with explicit scope, used for cross-CTA hand-offs.
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_gpu(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
+// A word that other blocks write during this kernel.
 __device__ __forceinline__ unsigned ld_relaxed_gpu_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -51,29 +43,15 @@ __device__ __forceinline__ unsigned ld_relaxed_gpu_u32(const unsigned* p) {
 __device__ __forceinline__ double ld_cg(const double* p) { return __ldcg(p); }
 __device__ __forceinline__ float ld_cg(const float* p) { return __ldcg(p); }
 
-// Named barrier over a subset of the CTA.  The non-aligned `barrier.sync` form
-// is used on purpose: `bar.sync` is `barrier.sync.aligned`, which counts a whole
-// warp as arrived when its first lanes arrive.
-__device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
-  asm volatile("barrier.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-__device__ __forceinline__ int wrap_mod(int v, int n) {
-  // v in [-2n, 3n): returns v mod n in [0, n)
-  while (v < 0) v += n;
-  while (v >= n) v -= n;
-  return v;
-}
-
 // -------------------------------------------------------------------------------
 // Tiled, circularly skewed layout used by the pressure solver.
 //
 // The grid is cut into column tiles of 32 (x) by TY (y) cells spanning all of z.
 // Inside a tile, cell (x, y, z) with tx = x mod 32, ty = y mod TY is stored at
 //     ((slot * TY + ty) * 32 + tx),   slot = (z + tx) mod nz.
-// A warp that owns row ty of a tile walks the i+j+k wavefront with lane tx at
-// z = s - ty - tx, so at every step all 32 lanes touch one contiguous row of
-// 32 elements: the MIC(0) sweeps become coalesced streams.  Tiles are ordered
+// A warp whose lane tx is at z = s - tx touches one contiguous row of 32 elements at
+// every s: the system is produced in this layout, and the SpMV walks its slots.  (The
+// MIC(0) sweeps and the iteration's vectors use the SweepLayout below.)  Tiles are ordered
 // tile = Y * ntx + X.  Cells outside the grid (x >= nx or y >= ny) are padding
 // and hold zeros.
 struct Tiled {

@@ -1132,7 +1132,8 @@ int launch_iter_cells(cudaStream_t st, const Geo& G, int iters, double* const b[
 // most of that was the spline: with a thread per cell and a pass per window plane
 // a particle's factors were worked out anew in each of 4 passes, 36 a grid.  Now
 // a lane reads one coordinate (or the velocity), works out three factors, and the
-// cell's lanes trade them by shuffle: 12 a grid, one division per lane.  The sums
+// cell's lanes trade them by shuffle: 12 a grid, two divisions by h per lane (none
+// where 1/h is exact).  The sums
 // are the ones that the passes gave, bit for bit.  4.2M particles in FP64 1185 ->
 // 826 us, 33.5M in FP32 7.3 -> 5.3 ms.  Slower: the next particle's factors worked
 // out ahead (988 us, spills), the axis factors by stencil index and shifted by

@@ -185,7 +185,9 @@ SC_HD int info_find(uint32_t v, int e) {
 }
 
 // Writes the vertices and normals cube (i, j, k) with case word w creates,
-// numbered from vbase (arrays of 3 doubles per vertex).
+// numbered from vbase (arrays of 3 doubles per vertex).  This, emit_indices and
+// Grid::mask are the plain per-cube form, built on the host only; the kernels go by
+// mask_of, the case_info words and emit_entries.
 SC_HD void emit_vertices(const Grid& g, int i, int j, int k, uint64_t w, int64_t vbase, double* V,
                          double* N) {
   int seen = 0;
