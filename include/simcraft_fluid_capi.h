@@ -133,7 +133,12 @@ typedef struct {
 void sc_pcg_default_options(sc_pcg_options* opt);
 
 /* CgSolver3D(w, h, d) + setPreconditioner(ModifiedIncompleteCholesky)
- * (project-solver.h:100-121).  opt may be NULL for the defaults. */
+ * (project-solver.h:100-121).  opt may be NULL for the defaults.
+ * A solver holds about 49 + 114 p bytes of device memory per cell, p = (nz + 10
+ * rounded up to a multiple of 4) / nz: 165 at 512^3, 249 at 512 x 512 x 16, 1420
+ * for a domain one cell deep (x and y count rounded up to multiples of 32 and 8).
+ * The first mixed solve adds 8 + 65 p, the first with SC_INNER_PCG another 16, and
+ * the host-array entry points 9. */
 int sc_pcg_create(sc_context* ctx, int nx, int ny, int nz, const sc_pcg_options* opt,
                   sc_pcg** out);
 void sc_pcg_destroy(sc_pcg* pcg);

@@ -19,8 +19,8 @@
 //
 // Two layouts.  The system as its producers write it (matrix, right-hand side,
 // active flags, the pressure handed back, and the mixed solve's FP64 residual) is
-// in the Tiled layout; everything an iteration touches is in the SweepLayout, in
-// which the sweeps (sc_sweep.cuh) stream whole chunks.
+// in the Tiled layout; the factors and the vectors of an iteration are in the
+// SweepLayout, in which the sweeps (sc_sweep.cuh) stream whole chunks.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -234,6 +234,31 @@ __global__ void __launch_bounds__(kThreads) k_to_tiled(Tiled g, const Ts* __rest
     if (c.inside) {
       const int64_t r = lin(c.x, c.y, c.z, g.ny, g.nz);
       if (!mask_ref || mask_ref[r]) v = (Td)src[r];
+    }
+    dst[c.e] = v;
+  }
+}
+// An array of the system (axis 0, 1, 2: the couplings to the lower neighbour along x, y,
+// z; -1: the diagonal).  Whole inactive rows and couplings to inactive cells are never
+// read by applyCompressedMatrix (it tests the neighbour's activity first).  The SpMV and
+// the pivots' products multiply them by zeros or use them as they are, so a non-finite
+// value there becomes 0; finite values stay as given.
+__global__ void __launch_bounds__(kThreads) k_matrix_to_tiled(Tiled g, const double* __restrict__ src, double* __restrict__ dst,
+                                                              const uint8_t* __restrict__ act, int axis) {
+  SC_ROWBLOCK_LOOP(g) {
+    Cell c;
+    c.init(g, rb, threadIdx.x);
+    double v = 0.0;
+    if (c.inside) {
+      const int64_t r = lin(c.x, c.y, c.z, g.ny, g.nz);
+      v = src[r];
+      if (!isfinite(v)) {
+        bool read = act[r];
+        if (axis == 0) read = read && c.x > 0 && act[r - (int64_t)g.ny * g.nz];
+        if (axis == 1) read = read && c.y > 0 && act[r - g.nz];
+        if (axis == 2) read = read && c.z > 0 && act[r - 1];
+        if (!read) v = 0.0;
+      }
     }
     dst[c.e] = v;
   }
@@ -465,15 +490,18 @@ __device__ __forceinline__ double apply_row(const Tiled& g, const Cell& c, const
   return t;
 }
 
-// The PCG's SpMV.  The rows and couplings that touch an inactive cell are zero
-// (k_sweep_system) and the PCG vectors are zero there, so no activity is tested.
+// The PCG's SpMV: the matrix as its producer wrote it (Tiled), x and y in the
+// SweepLayout.  The vectors are zero on inactive cells, so only a row's own activity is
+// tested.
 // A block of 8 warps owns a 32 x 8 column tile (two sweep tiles) and walks a run of
 // its slots: warp ty is row ty, and lane tx has cell z = (slot - tx) mod nz of its
 // column, so that the z neighbours of a lane's cell are its own at the previous and
 // next slot and the x neighbours the adjacent lanes' there.  A three-slot register
 // window holds both (x by shuffle); the y neighbours are the adjacent rows at the
-// same z, and only the two edge lanes of a row reach into the next tiles.  Every load
-// is issued one slot ahead.  The upper couplings come from the neighbours' lower ones
+// same z, and only the two edge lanes of a row reach into the next tiles.  The matrix's
+// rows of a slot are whole lines: from a copy of it in the SweepLayout, of whose 16-byte
+// vectors a slot uses one element, FP64 took 1657 us at 512^3, now 1492 (4.41 TB/s).
+// Every load is issued one slot ahead.  The upper couplings come from the neighbours' lower ones
 // (A symmetric, checkSystemSymmetry, :41-57).
 // The order in which a thread adds its products, and the tree that adds the threads'
 // sums, decide the last bits of s.Az and with them the rounding of every later
@@ -482,9 +510,9 @@ __device__ __forceinline__ double apply_row(const Tiled& g, const Cell& c, const
 // result, whatever the layout underneath.
 template <class T>
 __global__ void __launch_bounds__(kThreads, 3)
-    k_spmv(SweepLayout g, const int2* __restrict__ tiles, const T* __restrict__ adiag, const T* __restrict__ al,
-           const T* __restrict__ ad, const T* __restrict__ ab, const T* __restrict__ x, T* __restrict__ y,
-           double* partials, PcgScalars* sc, int use_skip, int runs) {
+    k_spmv(SweepLayout g, Tiled tg, const int2* __restrict__ tiles, const T* __restrict__ adiag, const T* __restrict__ al,
+           const T* __restrict__ ad, const T* __restrict__ ab, const uint8_t* __restrict__ act, const T* __restrict__ x,
+           T* __restrict__ y, double* partials, PcgScalars* sc, int use_skip, int runs) {
   if (use_skip && sc->done != DONE_RUNNING) return;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int nz = g.nz;
@@ -513,32 +541,42 @@ __global__ void __launch_bounds__(kThreads, 3)
     column(xg < g.ntx * 16 ? xg : xg - 16, hy ? yg - 1 : yg, wym, lym, kym);
     column(xg < g.ntx * 16 ? xg : xg - 16, py ? yg + 1 : yg, wyp, lyp, kyp);
     column(ex0 ? xg - 1 : ex31 ? xg + 1 : (xg < g.ntx * 16 ? xg : xg - 16), yg, wxe, lxe, kxe);
+    // the matrix: this lane's own row, the one at y + 1 in the same slot, and for the last
+    // lane the first one of the next tile, whose slots are the z
+    constexpr int RS = Tiled::TY * 32;
+    const int64_t tb = tg.tile_base(tiles[li].x, tiles[li].y), row = tb + ty * 32 + tx,
+                  ryp = ty < Tiled::TY - 1 ? row + 32 : tb + (int64_t)tg.ntx * tg.tile_elems + tx,
+                  rxp = tb + tg.tile_elems + ty * 32;
     auto wrap = [nz](int v) { return v >= nz ? v - nz : v; };
+    int sp = wrap(s0 + 1);  // the next slot
     int z = s0 - tx % nz;
     if (z < 0) z += nz;
     const int zm = z == 0 ? nz - 1 : z - 1;
     int zp = wrap(z + 1);
     T x_m = __ldg(x + at(wc, zm + kc, lc)), x_c = __ldg(x + at(wc, z + kc, lc)), x_p = __ldg(x + at(wc, zp + kc, lc));
-    T al_c = __ldg(al + at(wc, z + kc, lc)), al_p = __ldg(al + at(wc, zp + kc, lc));
-    T ab_c = __ldg(ab + at(wc, z + kc, lc)), ab_p = __ldg(ab + at(wc, zp + kc, lc));
-    T d_n = __ldg(adiag + at(wc, z + kc, lc)), adc_n = __ldg(ad + at(wc, z + kc, lc));
+    T al_c = __ldg(al + row + (int64_t)s0 * RS), al_p = __ldg(al + row + (int64_t)sp * RS);
+    T ab_c = __ldg(ab + row + (int64_t)s0 * RS), ab_p = __ldg(ab + row + (int64_t)sp * RS);
+    T d_n = __ldg(adiag + row + (int64_t)s0 * RS), adc_n = __ldg(ad + row + (int64_t)s0 * RS);
+    uint8_t a_n = __ldg(act + row + (int64_t)s0 * RS);
     T ym_n = hy ? __ldg(x + at(wym, z + kym, lym)) : T(0), yp_n = py ? __ldg(x + at(wyp, z + kyp, lyp)) : T(0),
-      adp_n = py ? __ldg(ad + at(wyp, z + kyp, lyp)) : T(0);
-    T xe_n = ex0 || ex31 ? __ldg(x + at(wxe, z + kxe, lxe)) : T(0), ale_n = ex31 ? __ldg(al + at(wxe, z + kxe, lxe)) : T(0);
+      adp_n = py ? __ldg(ad + ryp + (int64_t)s0 * RS) : T(0);
+    T xe_n = ex0 || ex31 ? __ldg(x + at(wxe, z + kxe, lxe)) : T(0), ale_n = ex31 ? __ldg(al + rxp + (int64_t)z * RS) : T(0);
     for (int s = s0; s < s1; s++) {
-      const int z2 = wrap(zp + 1);
+      const int z2 = wrap(zp + 1), s2 = wrap(sp + 1);
       const T d = d_n, adc = adc_n, ymv = ym_n, ypv = yp_n, adp = adp_n, xe = xe_n, ale = ale_n;
+      const bool a = inside && a_n;
       // the next window entries and the next slot's loads first: their latency
       // overlaps this slot's work
-      const int64_t o2 = at(wc, z2 + kc, lc), o1 = at(wc, zp + kc, lc);
-      const T x_n = __ldg(x + o2), al_n = __ldg(al + o2), ab_n = __ldg(ab + o2);
-      d_n = __ldg(adiag + o1);
-      adc_n = __ldg(ad + o1);
+      const int64_t e1 = row + (int64_t)sp * RS, e2 = row + (int64_t)s2 * RS;
+      const T x_n = __ldg(x + at(wc, z2 + kc, lc)), al_n = __ldg(al + e2), ab_n = __ldg(ab + e2);
+      d_n = __ldg(adiag + e1);
+      adc_n = __ldg(ad + e1);
+      a_n = __ldg(act + e1);
       ym_n = hy ? __ldg(x + at(wym, zp + kym, lym)) : T(0);
       yp_n = py ? __ldg(x + at(wyp, zp + kyp, lyp)) : T(0);
-      adp_n = py ? __ldg(ad + at(wyp, zp + kyp, lyp)) : T(0);
+      adp_n = py ? __ldg(ad + ryp + (int64_t)sp * RS) : T(0);
       xe_n = ex0 || ex31 ? __ldg(x + at(wxe, zp + kxe, lxe)) : T(0);
-      ale_n = ex31 ? __ldg(al + at(wxe, zp + kxe, lxe)) : T(0);
+      ale_n = ex31 ? __ldg(al + rxp + (int64_t)zp * RS) : T(0);
       const bool hz = z > 0, pz = z < nz - 1;
       T xm = __shfl_up_sync(kFull, x_m, 1), xp = __shfl_down_sync(kFull, x_p, 1), alp = __shfl_down_sync(kFull, al_p, 1);
       if (tx == 0) xm = xe;
@@ -555,7 +593,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       t += cxp * xp;
       t += cyp * ypv;
       t += czp * x_p;
-      const T o = inside ? t : T(0);
+      const T o = a ? t : T(0);
       if (inside) y[at(wc, z + kc, lc)] = o;
       acc += (double)x_c * (double)o;
       x_m = x_c;
@@ -567,6 +605,7 @@ __global__ void __launch_bounds__(kThreads, 3)
       ab_p = ab_n;
       z = zp;
       zp = z2;
+      sp = s2;
     }
   }
   reduce_finalize(acc, 0.0, partials, sc, FIN_SPMV);
@@ -647,9 +686,8 @@ __global__ void __launch_bounds__(kThreads)
 //   tau*A_L(p)*A_L(p-x+y) [if p-x+y active] + tau*A_L(p)*A_L(p-x+z) [if p-x+z active]
 // and likewise for Down and Back; they only depend on A.  PivotOp uses a
 // neighbour's terms only where that neighbour's pivot is not zero.  A coupling in
-// these products may itself lead to an inactive cell; a non-finite one then counts
-// as zero, a finite one as it is given.  tile_act (optional, zero on entry): 1 for
-// the tiles holding an active cell.
+// these products may itself lead to an inactive cell and counts as it is given.
+// tile_act (optional, zero on entry): 1 for the tiles holding an active cell.
 // A thread has four cells of a column and reads them and the six columns around from
 // each column's own base, all loads before they are used: testing each cell's activity
 // first and looking up every element by its coordinates took 984 us at 256^3 (134 at
@@ -668,9 +706,7 @@ struct TiledColumn {
 __global__ void __launch_bounds__(kThreads, 2)
     k_sweep_system(SweepLayout g, Tiled tg, const double* __restrict__ adiag, const double* __restrict__ al,
                    const double* __restrict__ ad, const double* __restrict__ ab, const uint8_t* __restrict__ act,
-                   double tau, double* __restrict__ o_d, double* __restrict__ o_l, double* __restrict__ o_dn,
-                   double* __restrict__ o_b, double* __restrict__ dL, double* __restrict__ dD,
-                   double* __restrict__ dB, uint8_t* __restrict__ tile_act) {
+                   double tau, PcgSolver::PivotIn out, uint8_t* __restrict__ tile_act) {
   SC_CHUNK_LOOP(i, g) {
     const ChunkPos c = chunk_pos<double>(g, i);
     double v[7][4] = {};
@@ -694,11 +730,6 @@ __global__ void __launch_bounds__(kThreads, 2)
                      aD = active(D, hd, 1, 5), aRD = active(RD, hr && hd, 1, 4), aR = active(R, hr, 0, 3),
                      aU = active(U, hu, 0, 3);
       any = (aC & 0x1eu) != 0;
-      // a coupling that leads to cell (xn, yn, zn)
-      auto to_cell = [&](double a, int xn, int yn, int zn) {
-        if (isfinite(a)) return a;
-        return xn >= 0 && yn >= 0 && zn >= 0 && act[tg.off(xn, yn, zn)] ? a : 0.0;
-      };
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int z = z0 + j;
@@ -710,24 +741,23 @@ __global__ void __launch_bounds__(kThreads, 2)
         v[0][j] = d;
         if (on(aL, 0)) {
           v[1][j] = l;
-          if (on(aLU, 0)) v[4][j] += tau * l * to_cell(l1, x - 2, y + 1, z);
-          if (on(aL, 1)) v[4][j] += tau * l * to_cell(l2, x - 2, y, z + 1);
+          if (on(aLU, 0)) v[4][j] += tau * l * l1;
+          if (on(aL, 1)) v[4][j] += tau * l * l2;
         }
         if (on(aD, 0)) {
           v[2][j] = dn;
-          if (on(aRD, 0)) v[5][j] += tau * dn * to_cell(d1, x + 1, y - 2, z);
-          if (on(aD, 1)) v[5][j] += tau * dn * to_cell(d2, x, y - 2, z + 1);
+          if (on(aRD, 0)) v[5][j] += tau * dn * d1;
+          if (on(aD, 1)) v[5][j] += tau * dn * d2;
         }
         if (on(aC, -1)) {
           v[3][j] = b;
-          if (on(aR, -1)) v[6][j] += tau * b * to_cell(b1, x + 1, y, z - 2);
-          if (on(aU, -1)) v[6][j] += tau * b * to_cell(b2, x, y + 1, z - 2);
+          if (on(aR, -1)) v[6][j] += tau * b * b1;
+          if (on(aU, -1)) v[6][j] += tau * b * b2;
         }
       }
     }
-    double* const out[7] = {o_d, o_l, o_dn, o_b, dL, dD, dB};
 #pragma unroll
-    for (int k = 0; k < 7; k++) chunk_store(out[k] + c.e, v[k]);
+    for (int k = 0; k < 7; k++) chunk_store(out.a[k] + c.e, v[k]);
     // a warp holds one chunk
     if (tile_act && __any_sync(kFull, any) && c.lane == 0) tile_act[c.tile] = 1;
   }
@@ -774,20 +804,13 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 // The matrix in FP32 (the FP32 SpMV of the restarted defect correction).
-__global__ void __launch_bounds__(kThreads)
-    k_sweep_matrix32(SweepLayout g, const double* __restrict__ d, const double* __restrict__ l,
-                     const double* __restrict__ dn, const double* __restrict__ b, SysArrays<float> o) {
-  SC_CHUNK_LOOP(i, g) {
-    const int64_t c = i >> 5;
-    const int lane = (int)(i & 31);
-    const double* const in[4] = {d, l, dn, b};
-    float* const out[4] = {o.adiag, o.al, o.ad, o.ab};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const Quad<double> q = chunk_load(in[k] + c * 128 + lane * 2);
-      const float f[4] = {(float)q.e[0], (float)q.e[1], (float)q.e[2], (float)q.e[3]};
-      chunk_store(out[k] + c * 128 + lane * 4, f);
-    }
+__global__ void __launch_bounds__(kThreads) k_matrix32(int64_t n, SysArrays<double> a, SysArrays<float> o) {
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += stride) {
+    o.adiag[e] = (float)a.adiag[e];
+    o.al[e] = (float)a.al[e];
+    o.ad[e] = (float)a.ad[e];
+    o.ab[e] = (float)a.ab[e];
   }
 }
 
@@ -935,8 +958,11 @@ std::vector<uint8_t> all_tile_bits(const SweepLayout& g, int cx, int cy, const i
   return b;
 }
 // The sweeps of a solver's arrays.
-inline PivotOp pivot_op(const SysArrays<double>& A, double sigma) {
-  return {{A.adiag, A.al, A.ad, A.ab, A.z, A.q, A.Az}, nullptr, {A.fwd, A.fwd + 128, A.fwd + 256, A.fwd + 384}, sigma};
+inline PivotOp pivot_op(const PcgSolver::PivotIn& in, double* fwd, double sigma) {
+  return {{in.a[0], in.a[1], in.a[2], in.a[3], in.a[4], in.a[5], in.a[6]},
+          nullptr,
+          {fwd, fwd + 128, fwd + 256, fwd + 384},
+          sigma};
 }
 template <class T, bool SELFDOT = false>
 FwdOp<T, SELFDOT> fwd_op(const SysArrays<T>& A) {  // q = L^-1 r
@@ -1054,9 +1080,8 @@ PcgSolver::PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt
     return p;
   };
   const size_t nt = sizeof(double) * (size_t)g_.total, ns = sizeof(double) * (size_t)sg_.total;
-  double** tiled[] = {&t_adiag_, &t_al_, &t_ad_, &t_ab_, &rhs_, &press_};
-  double** swept[] = {&d64_.adiag, &d64_.al, &d64_.ad, &d64_.ab, &d64_.r,
-                      &d64_.p,     &d64_.z,  &d64_.s,  &d64_.q,  &d64_.Az};
+  double** tiled[] = {&d64_.adiag, &d64_.al, &d64_.ad, &d64_.ab, &rhs_, &press_};
+  double** swept[] = {&d64_.r, &d64_.p, &d64_.z, &d64_.s, &d64_.q, &d64_.Az};
   auto alloc_zero = [&](double** a, size_t bytes) {
     *a = (double*)alloc(bytes);
     if (*a) cudaMemsetAsync(*a, 0, bytes, ctx->stream);
@@ -1234,7 +1259,7 @@ int PcgSolver::upload(const double* adiag, const double* const an[6], const doub
   const int64_t N = (int64_t)g_.nx * g_.ny * g_.nz;
   const int grid = grid_for(g_.total, ctx_->sm_count);
   const double* src[5] = {adiag, an[0], an[3], an[5], rhs};
-  double* dst[5] = {t_adiag_, t_al_, t_ad_, t_ab_, rhs_};
+  double* dst[5] = {d64_.adiag, d64_.al, d64_.ad, d64_.ab, rhs_};
   // staging buffers for host input (one array at a time)
   double* stage = nullptr;
   uint8_t* stage_act = nullptr;
@@ -1254,7 +1279,10 @@ int PcgSolver::upload(const double* adiag, const double* const an[6], const doub
       s = stage;
     }
     // rhs is zeroed outside the active set (the reference never reads it there)
-    k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g_, s, dst[a], a == 4 ? act_ref : nullptr);
+    if (a == 4)
+      k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g_, s, dst[a], act_ref);
+    else
+      k_matrix_to_tiled<<<grid, kThreads, 0, st>>>(g_, s, dst[a], act_ref, a - 1);
   }
   int rc = 0;
   if (opt_.check_symmetry) {
@@ -1329,22 +1357,32 @@ int PcgSolver::download_pressure(double* pg, bool device) {
 }
 
 // The matrix in FP32, which only the FP32 SpMV reads (the inner PCG of the mixed solve,
-// not the Eisenstat iteration): made when it is first needed for a system, since the
-// inner method may change between two solves of the same one.
-void PcgSolver::ensure_matrix32() {
-  if (matrix32_valid_) return;
-  k_sweep_matrix32<<<grid_for(sg_.total / 4, ctx_->sm_count), kThreads, 0, ctx_->stream>>>(sg_, d64_.adiag, d64_.al, d64_.ad,
-                                                                                           d64_.ab, d32_);
+// not the Eisenstat iteration): allocated and made when it is first needed for a system,
+// since the inner method may change between two solves of the same one.
+int PcgSolver::ensure_matrix32() {
+  if (matrix32_valid_) return 0;
+  for (float** a : {&d32_.adiag, &d32_.al, &d32_.ad, &d32_.ab}) {
+    if (*a) continue;
+    void* p = nullptr;
+    if (cudaMalloc(&p, sizeof(float) * (size_t)g_.total) != cudaSuccess)
+      return ctx_->set_error(-3, "FP32 allocation failed");
+    allocs_.push_back(p);
+    *a = (float*)p;
+  }
+  k_matrix32<<<grid_for(g_.total, ctx_->sm_count), kThreads, 0, ctx_->stream>>>(g_.total, d64_, d32_);
   launches_ += 1;
   matrix32_valid_ = true;
+  return 0;
 }
+
+// The pivots' inputs (PivotOp) in arrays that hold nothing else until the first solve or
+// application: the diagonal and the lower couplings in r, p, s and the place of the
+// backward factors, the neighbour products in z, q and Az.
+PcgSolver::PivotIn PcgSolver::pivot_in() const { return {{d64_.r, d64_.p, d64_.s, d64_.bwd, d64_.z, d64_.q, d64_.Az}}; }
 
 int PcgSolver::ensure_pivots() {
   const bool wants_matrix32 = opt_.precision == PREC_MIXED && opt_.inner_method != INNER_EISENSTAT;
-  if (pivots_valid_) {
-    if (wants_matrix32) ensure_matrix32();
-    return 0;
-  }
+  if (pivots_valid_) return wants_matrix32 ? ensure_matrix32() : 0;
   cudaStream_t st = ctx_->stream;
   const int sgrid = grid_for(sg_.total / 4, ctx_->sm_count);
   // the pivot sweep reports a timeout through the status word: start it clean,
@@ -1352,12 +1390,12 @@ int PcgSolver::ensure_pivots() {
   cudaMemsetAsync(&sc_->err, 0, sizeof(unsigned), st);
   pivot_limit_ = spin_limit();
   cudaMemcpyAsync(&sc_->spin_limit, &pivot_limit_, sizeof(int), cudaMemcpyHostToDevice, st);
-  // z, q and Az hold the pivots' neighbour products until select_active_tiles clears them
+  // select_active_tiles clears the vectors that hold the pivots' inputs
+  const PivotIn in = pivot_in();
   cudaMemsetAsync(tile_act_, 0, (size_t)sg_.ntiles(), st);
-  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg_, g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, opt_.tau, d64_.adiag,
-                                             d64_.al, d64_.ad, d64_.ab, d64_.z, d64_.q, d64_.Az, tile_act_);
-  sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(d64_, opt_.sigma), st);
-  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d64_);
+  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg_, g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, opt_.tau, in, tile_act_);
+  sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(in, d64_.fwd, opt_.sigma), st);
+  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, in.a[0], d64_);
   launches_ += 3;
   {
     // the solve's scalars are set over the status word next: read it first
@@ -1369,8 +1407,7 @@ int PcgSolver::ensure_pivots() {
   if (opt_.precision == PREC_MIXED) {
     if (!have_f32_) {
       const size_t n32 = sizeof(float) * (size_t)sg_.total;
-      float** arr32[] = {&d32_.adiag, &d32_.al, &d32_.ad, &d32_.ab, &d32_.fwd, &d32_.bwd,
-                         &d32_.r,     &d32_.p,  &d32_.z,  &d32_.s,  &d32_.q,   &d32_.Az};
+      float** arr32[] = {&d32_.fwd, &d32_.bwd, &d32_.r, &d32_.p, &d32_.z, &d32_.s, &d32_.q, &d32_.Az};
       for (float** a : arr32) {
         void* p = nullptr;
         const size_t bytes = n32 * (a == &d32_.fwd ? kFwdStream<float> : a == &d32_.bwd ? kBwdStream : 1);
@@ -1396,11 +1433,12 @@ int PcgSolver::ensure_pivots() {
       reset_mailboxes(true);
       have_f32_ = true;
     }
-    k_sweep_factor<float><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, d64_.adiag, d32_);
+    k_sweep_factor<float><<<sgrid, kThreads, 0, st>>>(sg_, d64_.fwd, in.a[0], d32_);
     launches_ += 1;
   }
   matrix32_valid_ = false;
-  if (wants_matrix32) ensure_matrix32();
+  if (wants_matrix32)
+    if (int e = ensure_matrix32()) return e;
   select_active_tiles();
   int e = check_dev_error("pivots");
   if (e) return e;
@@ -1441,8 +1479,8 @@ void PcgSolver::launch_spmv(SysArrays<T>& A, cudaStream_t st, int use_skip) {
   const int want = 12 * ctx_->sm_count;
   const int runs = std::max(1, std::min((want + ntiles - 1) / ntiles, g_.nz / 16));
   const int grid = std::min(3 * ctx_->sm_count, ntiles * runs);
-  k_spmv<T><<<grid, kThreads, 0, st>>>(sg_, order_t32_act_, A.adiag, A.al, A.ad, A.ab, A.s, A.Az, partials_, sc_, use_skip,
-                                       runs);
+  k_spmv<T><<<grid, kThreads, 0, st>>>(sg_, g_, order_t32_act_, A.adiag, A.al, A.ad, A.ab, active_, A.s, A.Az, partials_, sc_,
+                                       use_skip, runs);
 }
 
 template <class T>
@@ -1659,7 +1697,7 @@ int PcgSolver::solve_mixed_reliable(PcgStats* st) {
     // residual replacement after the chunks in flight
     if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed chunk");
     seen = launched;
-    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, t_adiag_, t_al_, t_ad_, t_ab_, active_, A.p, scale, press_,
+    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, A.p, scale, press_,
                                                  rres_, partials_, sc_);
     k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rres_, 1.0 / scale, active_, A.r, A.p, partials_, sc_,
                                                 FIN_NONE);
@@ -1755,7 +1793,7 @@ int PcgSolver::solve_mixed(PcgStats* st) {
     outer++;
     // x += rnorm d ; r -= rnorm A d   (FP64)
     launches_ += 1;
-    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, t_adiag_, t_al_, t_ad_, t_ab_, active_, d32_.p, rnorm,
+    k_mixed_update<<<nblocks_, kThreads, 0, s>>>(g_, sg_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, d32_.p, rnorm,
                                                  press_, rres_, partials_, sc_);
     cudaMemcpyAsync(sc_host_, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("mixed update");
@@ -1776,7 +1814,7 @@ int PcgSolver::solve_mixed(PcgStats* st) {
 int PcgSolver::true_residual(PcgStats* st) {
   cudaStream_t s = ctx_->stream;
   launches_ += 2;
-  k_true_residual<<<nblocks_, kThreads, 0, s>>>(g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, press_, rhs_, partials_, sc_);
+  k_true_residual<<<nblocks_, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, press_, rhs_, partials_, sc_);
   PcgScalars* h = sc_host_ + 1;
   cudaMemcpyAsync(h, sc_, sizeof(PcgScalars), cudaMemcpyDeviceToHost, s);
   // ||b||
@@ -1861,7 +1899,7 @@ int PcgSolver::apply_only(const double* x, double* b) {
     cudaMemcpyAsync(d64_.Az, x, bytes, cudaMemcpyDeviceToDevice, s);
     x = d64_.Az;
   }
-  k_apply_checked<<<grid, kThreads, 0, s>>>(g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, x, b);
+  k_apply_checked<<<grid, kThreads, 0, s>>>(g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, x, b);
   if (overlap) cudaMemsetAsync(d64_.Az, 0, bytes, s);
   if (cudaStreamSynchronize(s) != cudaSuccess) return check_dev_error("apply");
   return check_dev_error("apply");
@@ -1882,19 +1920,9 @@ int PcgSolver::time_kernels(int reps, double* ms) {
   init.alpha = 0.0;
   init.beta = 0.0;
   init.sigma = 1.0;
-  cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_, sc_);
-  cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-  k_copy<double><<<grid, kThreads, 0, s>>>(sg_, order_act_, d64_.r, d64_.s, sc_);
   // The mixed solver iterates in FP32: time its FP32 kernels (the pivot sweep
   // is FP64 in both).
   const bool f32 = opt_.precision == PREC_MIXED && have_f32_;
-  if (f32) {
-    ensure_matrix32();
-    k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d32_.r, d32_.p, partials_, sc_);
-    cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
-    k_copy<float><<<grid, kThreads, 0, s>>>(sg_, order_act_, d32_.r, d32_.s, sc_);
-  }
   auto kernel = [&](auto& A, int which) {
     using T = std::remove_reference_t<decltype(*A.r)>;
     const SweepPlan plan = sweep(sizeof(T) == 4, 0, FIN_NONE);
@@ -1924,6 +1952,19 @@ int PcgSolver::time_kernels(int reps, double* ms) {
         break;
     }
   };
+  auto benign_state = [&]() -> int {
+    cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
+    k_init<double><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d64_.r, d64_.p, partials_, sc_);
+    cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
+    k_copy<double><<<grid, kThreads, 0, s>>>(sg_, order_act_, d64_.r, d64_.s, sc_);
+    if (f32) {
+      if ((e = ensure_matrix32())) return e;
+      k_init<float><<<nblocks_, kThreads, 0, s>>>(g_, sg_, rhs_, 1.0, active_, d32_.r, d32_.p, partials_, sc_);
+      cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
+      k_copy<float><<<grid, kThreads, 0, s>>>(sg_, order_act_, d32_.r, d32_.s, sc_);
+    }
+    return 0;
+  };
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);
@@ -1932,11 +1973,11 @@ int PcgSolver::time_kernels(int reps, double* ms) {
     for (int i = 0; i < reps; i++) {
       switch (which) {
         case 0: {
-          // the neighbour products live in z, q and Az only until the sweeps use those; rebuild them
-          k_sweep_system<<<grid, kThreads, 0, s>>>(sg_, g_, t_adiag_, t_al_, t_ad_, t_ab_, active_, opt_.tau, d64_.adiag,
-                                                   d64_.al, d64_.ad, d64_.ab, d64_.z, d64_.q, d64_.Az, nullptr);
-          sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(d64_, opt_.sigma), s);
-          k_sweep_factor<double><<<grid, kThreads, 0, s>>>(sg_, d64_.fwd, d64_.adiag, d64_);
+          // the pivots' inputs live in the solve's arrays only until that starts; rebuild them
+          const PivotIn in = pivot_in();
+          k_sweep_system<<<grid, kThreads, 0, s>>>(sg_, g_, d64_.adiag, d64_.al, d64_.ad, d64_.ab, active_, opt_.tau, in, nullptr);
+          sweep(false, 0, FIN_NONE, true).run<double, true>(pivot_op(in, d64_.fwd, opt_.sigma), s);
+          k_sweep_factor<double><<<grid, kThreads, 0, s>>>(sg_, d64_.fwd, in.a[0], d64_);
           break;
         }
         default:
@@ -1953,14 +1994,14 @@ int PcgSolver::time_kernels(int reps, double* ms) {
     cudaEventElapsedTime(&t, a, b);
     return (double)t / reps;
   };
-  for (int k = 0; k < 8; k++) {
+  for (int k = 0; k < 8 && !e; k++) {
     cudaMemcpyAsync(sc_, &init, sizeof(PcgScalars), cudaMemcpyHostToDevice, s);
     ms[k] = (k < 6 || f32) ? timed(k) : 0.0;
+    if (k == 0) e = benign_state();
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  pivots_valid_ = true;
-  return check_dev_error("time_kernels");
+  return e ? e : check_dev_error("time_kernels");
 }
 
 }  // namespace sc
@@ -2076,7 +2117,7 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   uint8_t* bits = (uint8_t*)(order + kNaSweepTiles + 1);
   PcgScalars* scal = (PcgScalars*)(q + kNaSmallBytes - na_align(sizeof(PcgScalars)));
   SysArrays<double> A;
-  A.adiag = arr[0], A.al = arr[1], A.ad = arr[2], A.ab = arr[3], A.r = arr[12], A.q = arr[13], A.z = arr[14], A.Az = arr[15];
+  A.r = arr[12], A.q = arr[13], A.z = arr[14], A.Az = arr[15];
   A.fwd = arr[4], A.bwd = arr[8];  // four arrays each
   // The array keeps the previous call's contents: reset what must start at
   // zero (scheduling counters, scalars) and the mailbox sentinels.
@@ -2105,18 +2146,16 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   const std::vector<uint8_t> hbits = all_tile_bits(sg, 1, 1, ord);
   if (failed(cudaMemcpyAsync(bits, hbits.data(), hbits.size(), cudaMemcpyHostToDevice, st), "uploading the tile bits"))
     return -2;
-  // system into the tiled layout and from there into the sweeps', where the entries
-  // the reference never reads (couplings to inactive cells, inactive rows) are zero;
-  // right-hand side
+  // system into the tiled layout and from there into the sweeps'; right-hand side
   const int grid = grid_for(g.total, sm_count);
   k_to_tiled<uint8_t, uint8_t><<<grid, kThreads, 0, st>>>(g, active, act, nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, adiag, tl[0], nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[0], tl[1], nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[3], tl[2], nullptr);
-  k_to_tiled<double, double><<<grid, kThreads, 0, st>>>(g, an[5], tl[3], nullptr);
+  k_matrix_to_tiled<<<grid, kThreads, 0, st>>>(g, adiag, tl[0], active, -1);
+  k_matrix_to_tiled<<<grid, kThreads, 0, st>>>(g, an[0], tl[1], active, 0);
+  k_matrix_to_tiled<<<grid, kThreads, 0, st>>>(g, an[3], tl[2], active, 1);
+  k_matrix_to_tiled<<<grid, kThreads, 0, st>>>(g, an[5], tl[3], active, 2);
   const int sgrid = grid_for(sg.total / 4, sm_count);
-  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg, g, tl[0], tl[1], tl[2], tl[3], act, tau, A.adiag, A.al, A.ad, A.ab, A.z,
-                                             A.q, A.Az, nullptr);
+  const PcgSolver::PivotIn in{{arr[0], arr[1], arr[2], arr[3], A.z, A.q, A.Az}};
+  k_sweep_system<<<sgrid, kThreads, 0, st>>>(sg, g, tl[0], tl[1], tl[2], tl[3], act, tau, in, nullptr);
   k_ref_to_sweep<double><<<sgrid, kThreads, 0, st>>>(sg, r, A.r);
   if (failed(cudaGetLastError(), "converting the system to the solver's layouts")) return -2;
   // pivots, couplings, forward and backward sweeps
@@ -2135,8 +2174,8 @@ int mic_precond_noalloc(cudaStream_t st, int device, int sm_count, int nx, int n
   wa.use_skip = 0;
   wa.fin_kind = FIN_NONE;
   const int wgrid = std::min(ntiles, 2 * sm_count);
-  launch_sweep<double, true>(wa, pivot_op(A, sigma), st, wgrid);
-  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg, A.fwd, A.adiag, A);
+  launch_sweep<double, true>(wa, pivot_op(in, A.fwd, sigma), st, wgrid);
+  k_sweep_factor<double><<<sgrid, kThreads, 0, st>>>(sg, A.fwd, in.a[0], A);
   launch_sweep<double, true>(wa, fwd_op<double>(A), st, wgrid);
   launch_sweep<double, false>(wa, bwd_op<double>(A), st, wgrid);
   k_sweep_to_ref<double><<<sgrid, kThreads, 0, st>>>(sg, A.z, z);

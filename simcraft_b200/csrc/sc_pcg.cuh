@@ -148,14 +148,18 @@ struct PcgScalars {
 };
 
 template <class T>
-struct SysArrays {  // one precision's copy of everything the PCG iterates on (SweepLayout)
-  T *adiag = nullptr, *al = nullptr, *ad = nullptr, *ab = nullptr;
+struct SysArrays {  // one precision's copy of everything the PCG iterates on
+  T *adiag = nullptr, *al = nullptr, *ad = nullptr, *ab = nullptr;  // the matrix (Tiled); the rest in the SweepLayout
   T *fwd = nullptr, *bwd = nullptr;  // the sweeps' factor streams (sc_sweep.cuh)
   T *r = nullptr, *p = nullptr, *z = nullptr, *s = nullptr, *q = nullptr, *Az = nullptr;
 };
 
 class PcgSolver {
  public:
+  // PivotOp's inputs (SweepLayout): diagonal, lower couplings, neighbour products
+  struct PivotIn {
+    double* a[7];
+  };
   PcgSolver(Context* ctx, int nx, int ny, int nz, const PcgOptions& opt);
   ~PcgSolver();
   int status() const { return init_status_; }
@@ -178,10 +182,10 @@ class PcgSolver {
   const Tiled& geom() const { return g_; }
   uint64_t launches() const { return launches_; }
   // Direct access for in-device producers (FLIP buildSystem writes these).
-  double* adiag64() { return t_adiag_; }
-  double* al64() { return t_al_; }
-  double* ad64() { return t_ad_; }
-  double* ab64() { return t_ab_; }
+  double* adiag64() { return d64_.adiag; }
+  double* al64() { return d64_.al; }
+  double* ad64() { return d64_.ad; }
+  double* ab64() { return d64_.ab; }
   double* rhs64() { return rhs_; }
   uint8_t* active() { return active_; }
   double* pressure64() { return press_; }
@@ -192,7 +196,8 @@ class PcgSolver {
 
  private:
   int ensure_pivots();
-  void ensure_matrix32();
+  int ensure_matrix32();
+  PivotIn pivot_in() const;
   // eis: Eisenstat iteration (FP32 inner solve of the mixed path only)
   template <class T>
   int run_pcg(SysArrays<T>& A, double tol, int criterion, int max_iter, bool scale_rhs,
@@ -236,9 +241,8 @@ class PcgSolver {
   int nblocks_ = 0;     // elementwise grid
   SysArrays<double> d64_;
   SysArrays<float> d32_;
-  // FP64, Tiled layout: the system, the solution, and the mixed solve's residual
-  double *t_adiag_ = nullptr, *t_al_ = nullptr, *t_ad_ = nullptr, *t_ab_ = nullptr, *rhs_ = nullptr;
-  double *press_ = nullptr, *rres_ = nullptr;
+  // FP64, Tiled layout: the right-hand side, the solution, and the mixed solve's residual
+  double *rhs_ = nullptr, *press_ = nullptr, *rres_ = nullptr;
   uint8_t* active_ = nullptr;
   double* partials_ = nullptr;  // 2 per block
   double* tile_partials_ = nullptr;
