@@ -166,9 +166,11 @@ struct FwdEisenstatOp {
 // dL/dD/dB hold the tau-weighted products with the diagonal neighbours'
 // couplings (k_sweep_system), so the sweep only streams its own column.
 // A step is three divisions, a square root and another division one after another.
-// They are evaluated without branches, and with operands 1 where a term is absent:
-// a division 0 / x leaves the fast path of the division for the whole warp.  One
-// 16 x 8 x 8192 column tile 1005 -> 642 ns a step, 128^3 697 -> 631 us.
+// Only inactive cells branch around them; a term that is absent divides 1 by 1, since
+// 0 / x leaves the fast path of the division for the whole warp.  A 16 x 8 x 8192 column
+// tile 1007 -> 546 ns a step; 32^3 150 -> 94 us, 128^3 688 -> 583 us, 256^3 2420 -> 1900
+// us, half of the cells fluid, with k_sweep_system and k_sweep_factor.  (Without the
+// branch for inactive cells 118, 701 and 2340 us.)
 struct PivotOp {
   static constexpr int NX = 7, NF = 0, FS = 1, NO = 4, OS = kFwdStream<double>;
   const double* src[NX];  // adm, al, ad, ab, dL, dD, dB
@@ -177,18 +179,21 @@ struct PivotOp {
   double sigma;
   __device__ __forceinline__ double step(const double* v, double EL, double ED, double EB, double* o, double&) const {
     const double adiag = v[0], al = v[1], ad = v[2], ab = v[3];
-    const bool on = adiag != 0.0, qL = EL != 0.0 && v[4] != 0.0, qD = ED != 0.0 && v[5] != 0.0, qB = EB != 0.0 && v[6] != 0.0;
-    const double tL = (qL ? v[4] : 1.0) / (qL ? EL * EL : 1.0), tD = (qD ? v[5] : 1.0) / (qD ? ED * ED : 1.0),
-                 tB = (qB ? v[6] : 1.0) / (qB ? EB * EB : 1.0);
-    double ee = adiag;
-    ee -= (al * EL) * (al * EL);
-    ee = qL ? ee - tL : ee;
-    ee -= (ad * ED) * (ad * ED);
-    ee = qD ? ee - tD : ee;
-    ee -= (ab * EB) * (ab * EB);
-    ee = qB ? ee - tB : ee;
-    if (ee < sigma * adiag) ee = adiag;
-    const double rE = 1.0 / sqrt(on ? ee : 1.0), E = on ? rE : 0.0;
+    double E = 0.0;
+    if (adiag != 0.0) {
+      const bool qL = EL != 0.0 && v[4] != 0.0, qD = ED != 0.0 && v[5] != 0.0, qB = EB != 0.0 && v[6] != 0.0;
+      const double tL = (qL ? v[4] : 1.0) / (qL ? EL * EL : 1.0), tD = (qD ? v[5] : 1.0) / (qD ? ED * ED : 1.0),
+                   tB = (qB ? v[6] : 1.0) / (qB ? EB * EB : 1.0);
+      double ee = adiag;
+      ee -= (al * EL) * (al * EL);
+      ee = qL ? ee - tL : ee;
+      ee -= (ad * ED) * (ad * ED);
+      ee = qD ? ee - tD : ee;
+      ee -= (ab * EB) * (ab * EB);
+      ee = qB ? ee - tB : ee;
+      if (ee < sigma * adiag) ee = adiag;
+      E = 1.0 / sqrt(ee);
+    }
     o[0] = al * EL;
     o[1] = ad * ED;
     o[2] = ab * EB;
