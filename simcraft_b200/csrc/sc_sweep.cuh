@@ -18,7 +18,10 @@
 // is involved.  (An mbarrier per ring entry cost ~400 cycles of a chunk's ~1100;
 // divergent branches around the hand-off another ~400.  Separate words in which a
 // consumer says how far it is need a fence before them, and a fence waits for the
-// stores of the outputs: 256^3 mixed solve 175 ms, with the look at the words 128.)
+// stores of the outputs: 256^3 mixed solve 175 ms.  The look at the words instead is
+// asked for three chunks before its answer is needed, in rings long enough for that:
+// 127 ms; with the answer awaited in the same chunk, from rings of half the length,
+// 136, and the FP32 sweeps of 512^3 took 908 and 956 us instead of 728 and 766.)
 // A block of 4 such warps sweeps a 16 x 8 column tile.
 // Four steps per hand-off: the lag it adds (a chunk per warp crossed) costs less
 // than a wait per step would, and it is the largest number for which both
@@ -464,7 +467,7 @@ __device__ __forceinline__ RingWords ring_look(uint32_t p) {
 // ---- shared memory of a sweep block -----------------------------------------------
 constexpr int kSweepWarps = SweepLayout::kWarps;       // compute warps, 2 (x) by 2 (y)
 constexpr int kSweepThreads = (kSweepWarps + 4) * 32;  // + 2 x and 2 y mailbox loaders
-constexpr int kRing = 8;                               // entries of a boundary ring
+constexpr int kRing = 16;                              // entries of a boundary ring: four groups
 constexpr int kTick = 8;                               // tickets a block can hold
 template <class T, int NV>
 struct SweepSmem {
@@ -788,18 +791,19 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
       };
       double acc = 0.0;
       T prev = T(0);
-      // ring addresses of the current group's half and the other one
-      uint32_t half = (group & 1) * 4;
+      // ring entries of the current group
+      uint32_t cur = (group * 4) % kRing;
       // the last value of the entries before the first chunk's: x entry 1, y entry 0
       Quad<T> x0, y0;
-      take(has_x, rx + (half + 1) * kSlotX, has_y, ry + half * kSlotY, x0, y0, [] {});
+      take(has_x, rx + (cur + 1) * kSlotX, has_y, ry + cur * kSlotY, x0, y0, [] {});
       T xc = x0.e[3], yc = y0.e[3];
       // four chunks from d0 on; main part: none of what they take from the rings has ended
       auto four_chunks = [&](auto main_part, int d0) {
         constexpr bool kMain = decltype(main_part)::value;
-        const uint32_t rxa = rx + half * kSlotX, rxb = rx + (half ^ 4) * kSlotX, rya = ry + half * kSlotY,
-                       ryb = ry + (half ^ 4) * kSlotY, oxa = orx + half * kSlotX, oya = ory + half * kSlotY;
-        const int sbase = D == 8 ? (int)half : 0;  // stage slots sbase .. sbase + 3, then the others
+        const uint32_t nxt = (cur + 4) % kRing;
+        const uint32_t rxa = rx + cur * kSlotX, rxb = rx + nxt * kSlotX, rya = ry + cur * kSlotY, ryb = ry + nxt * kSlotY,
+                       oxa = orx + cur * kSlotX, oya = ory + cur * kSlotY;
+        const int sbase = D == 8 ? (int)(cur & 4) : 0;  // stage slots sbase .. sbase + 3, then the others
         constexpr int kDir = FWD ? 1 : -1;
         const int64_t cg = chunk_at(c0, d0);
         const int64_t ato = cg * (Op::OS * 128) + lane * kLane;
@@ -820,6 +824,10 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
         if (go.next && go.chunks) ahead++;
         const int64_t cf = go.chunks ? chunk_at(go.next ? nc0 : c0, 4 * go.group) : c0;
         const int64_t fv = cf * 128 + lane * kLane, ff = cf * (Op::FS * 128) + lane * kLane;
+        // What the next group's entries hold: asked for in the first chunk, looked at after the
+        // last, since the answer comes from another block.  Their consumers took the last values
+        // there two groups ago, unless they are late.
+        RingWords look_nx, look_ny;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           const int d = d0 + i;
@@ -827,12 +835,9 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           const int slot = (sbase + i) & (D - 1);
           const bool on = i < go.chunks;
           const int64_t av = fv + kDir * i * 128, af = ff + kDir * i * (Op::FS * 128);
-          // in the last chunk, what the next group's entries hold: their consumers took the
-          // values about three chunks ago, unless they are late
-          RingWords nx{}, ny{};
-          if (i == 3) {
-            nx = ring_look<T>(look_x + (half ^ 4) * kSlotX);
-            ny = ring_look<T>(look_y + (half ^ 4) * kSlotY);
+          if (i == 0) {
+            look_nx = ring_look<T>(look_x + nxt * kSlotX);
+            look_ny = ring_look<T>(look_y + nxt * kSlotY);
           }
           if (live) {
             // the neighbours' boundary values, x entry d + 2 and y entry d + 1, and this
@@ -872,8 +877,8 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
             // until the words that this group's boundary values go to are empty
             if (i == 0 && held) {
               for (int spins = 0;;) {
-                const uint32_t hx = ring_look<T>(look_x + half * kSlotX).held(kEmpty),
-                               hy = ring_look<T>(look_y + half * kSlotY).held(kEmpty);
+                const uint32_t hx = ring_look<T>(look_x + cur * kSlotX).held(kEmpty),
+                               hy = ring_look<T>(look_y + cur * kSlotY).held(kEmpty);
                 if (!__any_sync(kFull, (feeds_x & (hx != 0)) | (feeds_y & (hy != 0)))) break;
                 if (!__all_sync(kFull, W.more(spins, lim))) break;
               }
@@ -890,11 +895,11 @@ __global__ void __launch_bounds__(kSweepThreads, 1)
           } else {
             copy(av, af, slot, on);
           }
-          if (i == 3) held = __any_sync(kFull, ((rings_x & (nx.held(kEmpty) != 0)) | (rings_y & (ny.held(kEmpty) != 0))));
+          if (i == 3) held = __any_sync(kFull, (rings_x & (look_nx.held(kEmpty) != 0)) | (rings_y & (look_ny.held(kEmpty) != 0)));
           cp_async_commit();
         }
         group++;
-        half ^= 4;
+        cur = nxt;
         __syncwarp();
       };
       for (int gi = 0; gi < NG; gi++) {
