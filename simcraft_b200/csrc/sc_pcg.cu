@@ -692,7 +692,7 @@ __global__ void __launch_bounds__(kThreads)
 // each column's own base, all loads before they are used: testing each cell's activity
 // first and looking up every element by its coordinates took 984 us at 256^3 (134 at
 // 128^3), and a pass over the Tiled arrays that cleared the non-finite entries before
-// that another 385 (57); now 530 (64) and none.
+// that another 385 (57); now 480 (68) and none.
 struct TiledColumn {
   int64_t base;
   int skew, nz;  // slot of z: (z + skew) mod nz
